@@ -1001,36 +1001,47 @@ __device__ __forceinline__ uint32_t ld4u(const uint8_t *p)
 }
 
 // Position offset of the t-th probe of a search, relative to its start: the step is
-// 1 for probes 0..64 and grows by one every 64 probes after that.
-__device__ __forceinline__ int64_t probe_offset(int64_t t)
+// 1 for probes 0..64 and grows by one every 64 probes after that.  (Below 2^32 for every
+// stream: a search stops at the first probe past the stream, less than 2^31 bytes long.)
+__device__ __forceinline__ uint32_t probe_offset(uint32_t t)
 {
-    if (t <= 0) return 0;
-    const int64_t m = 62 + t, q = m >> 6, r = m - (q << 6);
-    return 1 + 64 * (q * (q - 1) / 2) + q * (r + 1);
+    if (t == 0) return 0;
+    const uint32_t m = 62 + t, q = m >> 6, r = m - (q << 6);
+    return 1 + 32 * (q * (q - 1)) + q * (r + 1);
 }
 
 // Shared-memory window over one stream for the encoder: positions [lo, hi) sit at
-// r[x & (ERING - 1)], the first 16 ring bytes mirrored past its end so that 4-byte reads
-// never wrap.  The window follows the parse position; reads outside it (far search
+// r[x & (cap - 1)], the first EMIRROR ring bytes mirrored past its end so that reads of up to
+// 32 bytes never wrap.  The window follows the parse position; reads outside it (far search
 // probes, old match candidates) go to global memory.  Without it the candidate reads of
 // low-entropy streams, spread over the last few KiB, mostly miss L1.
-constexpr int ERING = 4096, ESEG = 1024, ELOOK = 512;
+#ifndef XRING_
+#define XRING_ 4096
+#endif
+// The liblz4-identical encoder's warps (one per CTA) hold 16 KiB of table each; with a 2 KiB
+// window eleven of them fit an SM (f32 blocks of 125 x 150, 5000 x 6000 product: 0.98 ms; ten
+// with 4 KiB windows 1.26 ms, twelve with 1 KiB 0.91 ms there but 1.02x the time on 64 KiB
+// streams, whose candidates then come from global memory).
+constexpr int XCTAS = 11, XRING = 2048;
+constexpr int ERING = 4096, ESEG = 512, ELOOK = 256, EMIRROR = 32;
+constexpr int EPEER = 128 + 64;                    // words of the lanes-by-hash masks of warp_lz4_compress
 
 struct EncSrc {
     const uint8_t *g;   // the stream in global memory
-    uint8_t *r;         // ERING + 16 bytes, 16-byte aligned
+    uint8_t *r;         // cap + EMIRROR bytes, 16-byte aligned
+    int cap;            // ring size, a power of two
     int lo, hi, n;
 };
 
 __device__ __forceinline__ uint32_t es_byte(const EncSrc &s, int x)
 {
-    return (x >= s.lo && x < s.hi) ? (uint32_t)s.r[x & (ERING - 1)] : (uint32_t)__ldg(s.g + x);
+    return (x >= s.lo && x < s.hi) ? (uint32_t)s.r[x & (s.cap - 1)] : (uint32_t)__ldg(s.g + x);
 }
 
 __device__ __forceinline__ uint32_t es_rd32(const EncSrc &s, int x)
 {
     if (x >= s.lo && x + 4 <= s.hi) {
-        const int o = x & (ERING - 1);
+        const int o = x & (s.cap - 1);
         const uint32_t *w = reinterpret_cast<const uint32_t *>(s.r) + (o >> 2);
         return __funnelshift_r(w[0], w[1], (uint32_t)(o & 3) * 8);
     }
@@ -1045,57 +1056,46 @@ __device__ __forceinline__ uint32_t es_hash(const EncSrc &s, int p, bool small)
     return (uint32_t)(((v << 24) * 889523592379ull) >> (64 - 12));
 }
 
-// Extends the window up to position `want` (warp-uniform) in ESEG pieces.
+// Extends the window up to position `want` (warp-uniform) in ESEG pieces; a piece's loads are
+// all issued before its stores.
 __device__ __forceinline__ void es_fill(EncSrc &s, int want)
 {
     const int lane = threadIdx.x & 31;
     while (s.hi < s.n && s.hi < want) {
         const int base = s.hi, cnt = min(ESEG, s.n - base);
-        __syncwarp();                                    // reads of the slots being replaced are done
-        for (int x = lane * 4; x < cnt; x += 128) {
-            uint32_t v = 0;
+        uint32_t v[ESEG / 128];
+#pragma unroll
+        for (int i = 0; i < ESEG / 128; i++) {
+            const int x = lane * 4 + i * 128;
+            v[i] = 0;
             if (base + x + 8 <= s.n) {
-                v = ld4u(s.g + base + x);
+                v[i] = ld4u(s.g + base + x);
             } else {
                 for (int k = 0; k < 4; k++)
-                    if (base + x + k < s.n) v |= (uint32_t)__ldg(s.g + base + x + k) << (8 * k);
+                    if (base + x + k < s.n) v[i] |= (uint32_t)__ldg(s.g + base + x + k) << (8 * k);
             }
-            const int o = (base + x) & (ERING - 1);
-            *reinterpret_cast<uint32_t *>(s.r + o) = v;
-            if (o < 16) *reinterpret_cast<uint32_t *>(s.r + ERING + o) = v;
+        }
+        __syncwarp();                                    // reads of the slots being replaced are done
+#pragma unroll
+        for (int i = 0; i < ESEG / 128; i++) {
+            const int x = lane * 4 + i * 128, o = (base + x) & (s.cap - 1);
+            if (x >= cnt) continue;
+            *reinterpret_cast<uint32_t *>(s.r + o) = v[i];
+            if (o < EMIRROR) *reinterpret_cast<uint32_t *>(s.r + s.cap + o) = v[i];
         }
         s.hi = base + cnt;
-        s.lo = max(s.lo, base + ESEG - ERING);
+        s.lo = max(s.lo, base + ESEG - s.cap);
         __syncwarp();
     }
 }
 
-// Shared-memory accesses through 32-bit shared-window addresses (volatile: they keep
-// their order relative to each other, which the table updates rely on).
+// Shared-memory word through a 32-bit shared-window address.
 __device__ __forceinline__ uint32_t lds32(uint32_t a)
 {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ uint32_t lds_tab(uint32_t a, bool small)
-{
-    uint32_t v;
-    if (small) {
-        uint16_t h;
-        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(a) : "memory");
-        v = h;
-    } else {
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    }
-    return v;
-}
-__device__ __forceinline__ void sts_tab(uint32_t a, uint32_t v, bool small)
-{
-    if (small) asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
-    else asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-
 // liblz4's hash of the 4 bytes v4 at a position (byU16 tables) or of those and the fifth
 // byte b4 (byU32 tables).
 template <bool SMALL>
@@ -1113,211 +1113,353 @@ __device__ __forceinline__ uint32_t lz_hash_v(uint32_t v4, uint32_t b4)
 // byU16 table (inputs below 64 KiB + 11 bytes: 13-bit hash of 4 bytes) over its byU32
 // table (12-bit hash of 5 bytes, 65535-byte distance limit).
 //
-// Two regimes.  Searching (no match at the parse position): one step evaluates 32
-// consecutive probes of liblz4's search (its step schedule), resolving probes that share
-// a hash bucket in probe order with __match_any_sync.  Right after a match liblz4
-// inserts ip - 2 and tests ip itself; on low-entropy data that test nearly always
-// succeeds, so it runs as a short scalar path that every lane executes identically (the
-// window bytes around ip and around the candidate come from a few aligned shared-memory
-// words, the match length from one 64-bit compare, table updates written by all lanes
-// with the same value), leaving the warp-wide machinery for long matches and searches.
+// liblz4's parse is one serial chain (what a position finds depends on which earlier positions
+// were inserted), and its latency bounds the kernel: a launch has far fewer compressible streams
+// than the SMs have warp slots.  So 32 consecutive positions, one per lane, are handled at once:
+// the bytes, the hash, the table's candidate as of the window's start, whether it matches, how
+// far forwards (to 16 bytes) and backwards (to 4), and from that the chain of matches from every
+// lane by pointer doubling over the lanes.  This chain is liblz4's as long as no tested lane has
+// an inserted lane of the same hash before it in the window (that lane would be its candidate):
+// one ballot finds the first step where it has.  The steps before it are written together, the
+// step itself is walked exactly (its candidates are the inserted lanes, a bit mask, else the
+// table's), and the chain goes on from its end.  Steps with long matches or literal runs and
+// long backward extensions are walked too, with warp-wide loops.  Inserted lanes enter the table
+// at the window's end.  Searches past their 64th probe, whose step grows, take 32 probes per step
+// at the probes' own positions.
+// Measured against one scalar step per sequence (650 cycles each; a window of 32 positions now
+// takes about 2,100): 64 KiB sign/exponent planes 5.1 -> 2.2 ms a stream; k_lz4_encode on the
+// 5000 x 6000 float32 product 4.75 -> 0.98 ms, on the 4056 x 3712 float64 one 2.30 -> 0.93 ms
+// (of which 0.4 ms from handing out the compressible planes first).
 template <bool SMALL>
 __device__ __forceinline__ int warp_lz4_compress(const uint8_t *__restrict__ src, int n, uint8_t *__restrict__ dst,
-                                                 int cap, uint32_t *tab, uint8_t *ring, int *need_out)
+                                                 int cap, uint32_t *tab, uint32_t *bm, uint8_t *ring, int rcap,
+                                                 int *need_out)
 {
     const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
     uint16_t *tab16 = reinterpret_cast<uint16_t *>(tab);
-    for (int i = lane; i < 4096; i += 32) tab[i] = 0u;
+    for (int i = lane; i < 1024; i += 32) reinterpret_cast<uint4 *>(tab)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = lane; i < EPEER; i += 32) bm[i] = 0u;
     EncSrc s;
-    s.g = src; s.r = ring; s.lo = 0; s.hi = 0; s.n = n;
-    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring), tab_s = (uint32_t)__cvta_generic_to_shared(tab);
-    constexpr uint32_t TSH = SMALL ? 1 : 2;             // table entry size: 2 or 4 bytes
+    s.g = src; s.r = ring; s.cap = rcap; s.lo = 0; s.hi = 0; s.n = n;
+    const uint32_t *rw = reinterpret_cast<const uint32_t *>(ring);
+    const int wmask = (rcap >> 2) - 1;
     __syncwarp();
-    int need = 0, op = 0, anchor = 0, ip = 1, mt = 0;
-    int token_pos = 0, token_val = 0;
+    int need = 0, op = 0, anchor = 0;
     const int mfl1 = n - 12 + 1, mlimit = n - 5;
 #define TGET(h) (SMALL ? (uint32_t)tab16[h] : tab[h])
 #define TPUT(h, v) do { if (SMALL) tab16[h] = (uint16_t)(v); else tab[h] = (uint32_t)(v); } while (0)
-#define NEED(x) do { const int nx_ = (x); need = max(need, nx_); if (nx_ > cap) { *need_out = need; return 0; } } while (0)
-    if (n < 13) goto last_literals;
-    es_fill(s, ELOOK);
-    if (lane == 0) TPUT(es_hash(s, 0, SMALL), 0);
-    __syncwarp();
-    for (;;) {
-        // ---- search from ip: probes p0 + probe_offset(t), t = 0, 1, ...
-        {
-            const int p0 = ip;
-            int64_t t0 = 0;
+    // The sequence that ends with the match of position pr at distance d: L bytes are known to
+    // match (`longer`: perhaps more), `back` bytes before pr match too (`more_back`: perhaps
+    // more).  Sets anchor to its end; false when the output does not fit.
+    auto sequence = [&](int pr, int d, int L, bool longer, int back, bool more_back) -> bool {
+        const int lits = pr - anchor, lim = mlimit - pr;
+        back = min(back, lits);
+        if (L >= lim) { L = lim; longer = false; }
+        if (more_back) {
             for (;;) {
-                es_fill(s, p0 + (int)(probe_offset(t0) < n ? probe_offset(t0) : (int64_t)n) + ELOOK);
-                const int64_t t = t0 + lane;
-                // the step is 1 for the first 66 probes: positions are p0 + t there
-                const bool dense = t0 + 32 <= 65;
-                const int64_t p = dense ? p0 + t : p0 + probe_offset(t);
-                const int64_t pn = dense ? p + 1 : p0 + probe_offset(t + 1);
-                const bool valid = pn <= mfl1;
-                const uint32_t h = valid ? es_hash(s, (int)p, SMALL) : (0x80000000u | (uint32_t)lane);
-                const uint32_t ctab = valid ? TGET(h) : 0u;
-                const unsigned peers = __match_any_sync(FULLMASK, h);
-                const unsigned lower = peers & ((1u << lane) - 1u);
-                const int srcl = lower ? 31 - __clz(lower) : lane;
-                const int pl = __shfl_sync(FULLMASK, (int)p, srcl);
-                const uint32_t cand = lower ? (uint32_t)pl : ctab;
-                const bool m = valid && (SMALL || cand + 65535u >= (uint32_t)p) &&
-                               es_rd32(s, (int)cand) == es_rd32(s, (int)p);
-                const unsigned mm = __ballot_sync(FULLMASK, m), em = __ballot_sync(FULLMASK, !valid);
-                const int W = mm ? __ffs(mm) - 1 : 32, E = em ? __ffs(em) - 1 : 32;
-                const int lastw = min(W, E - 1);
-                __syncwarp();
-                if (lane <= lastw) {
-                    const unsigned upto = (lastw >= 31) ? FULLMASK : ((2u << lastw) - 1u);
-                    const unsigned higher = peers & ~((2u << lane) - 1u) & upto;
-                    if (!higher) TPUT(h, (uint32_t)p);
-                }
-                __syncwarp();
-                if (W < E) {
-                    ip = __shfl_sync(FULLMASK, (int)p, W);
-                    mt = (int)__shfl_sync(FULLMASK, cand, W);
-                    break;
-                }
-                if (E < 32) goto last_literals;
-                t0 += 32;
+                const int k = back + lane + 1;
+                const bool ok = k <= lits && pr - d - k >= 0 && es_byte(s, pr - k) == es_byte(s, pr - d - k);
+                const unsigned badm = __ballot_sync(FULLMASK, !ok);
+                const int ext = badm ? __ffs((int)badm) - 1 : 32;
+                back += ext;
+                if (ext < 32) break;
             }
         }
-        for (;;) {   // extend the match backwards
-            const int k = lane + 1;
-            const bool ok = (ip - k >= anchor) && (mt - k >= 0) && es_byte(s, ip - k) == es_byte(s, mt - k);
-            const unsigned badm = __ballot_sync(FULLMASK, !ok);
-            const int ext = badm ? __ffs(badm) - 1 : 32;
-            ip -= ext;
-            mt -= ext;
-            if (ext < 32) break;
-        }
-        {   // literals
-            const int lit = ip - anchor;
-            token_pos = op;
-            op += 1;
-            NEED(op + lit + 8 + lit / 255);
-            if (lit >= 15) {
-                token_val = 15 << 4;
-                const int rem = lit - 15, nff = rem / 255;
-                for (int x = lane; x < nff; x += 32) dst[op + x] = 255;
-                if (lane == 0) dst[op + nff] = (uint8_t)(rem % 255);
-                op += nff + 1;
-            } else {
-                token_val = lit << 4;
-            }
-            for (int x = lane; x < lit; x += 32) dst[op + x] = (uint8_t)es_byte(s, anchor + x);
-            op += lit;
-        }
-        {   // the match found by the search: offset, length (warp-wide compare), token
-            const int mo = ip - mt;
-            if (lane == 0) { dst[op] = (uint8_t)mo; dst[op + 1] = (uint8_t)(mo >> 8); }
-            op += 2;
-            int mc = 0;
-            for (int a = ip + 4, bpos = mt + 4;; a += 32, bpos += 32) {
-                es_fill(s, a + 32 + ELOOK);
-                const int pa = a + lane;
-                const bool eq = pa < mlimit && es_byte(s, pa) == es_byte(s, bpos + lane);
+        if (longer) {
+            for (;;) {
+                const int a = pr + L + lane;
+                if (pr + L + 64 > s.hi) es_fill(s, pr + L + ELOOK);
+                const bool eq = a < mlimit && es_byte(s, a) == es_byte(s, a - d);
                 const unsigned ne = __ballot_sync(FULLMASK, !eq);
-                const int cnum = ne ? __ffs(ne) - 1 : 32;
-                mc += cnum;
+                const int cnum = ne ? __ffs((int)ne) - 1 : 32;
+                L += cnum;
                 if (cnum < 32) break;
             }
-            ip += mc + 4;
-            NEED(op + 6 + (mc + 240) / 255);
-            if (mc >= 15) {
-                token_val += 15;
-                const int rem = mc - 15, nff = rem / 255;
-                for (int x = lane; x < nff; x += 32) dst[op + x] = 255;
-                if (lane == 0) dst[op + nff] = (uint8_t)(rem % 255);
-                op += nff + 1;
-            } else {
-                token_val += mc;
-            }
-            if (lane == 0) dst[token_pos] = (uint8_t)token_val;
         }
-        // ---- after each match: insert ip - 2, look ip up, insert it; a hit is a match with
-        // no literals (scalar path, identical on every lane)
+        const int lit = lits - back, mc = L + back - 4;
+        anchor = pr + L;
+        if (lit < 15 && mc < 15) {
+            need = max(need, op + lit + 9);
+            if (need > cap) return false;
+            if (lane < lit + 3)
+                dst[op + lane] = (uint8_t)(lane == 0 ? (uint32_t)((lit << 4) | mc)
+                                                     : lane <= lit ? es_byte(s, pr - lits + lane - 1)
+                                                                   : (uint32_t)d >> (8 * (lane - lit - 1)));
+            op += lit + 3;
+            return true;
+        }
+        const int eb = (lit >= 15 ? (lit - 15) / 255 + 1 : 0), mb = (mc >= 15 ? (mc - 15) / 255 + 1 : 0);
+        const int o = op + 1 + eb;                              // the literals' offset
+        need = max(need, max(op + lit + 9 + lit / 255, o + lit + 8 + (mc + 240) / 255));
+        if (need > cap) return false;
+        if (lane == 0) dst[op] = (uint8_t)((min(lit, 15) << 4) | min(mc, 15));
+        for (int x = lane; x < eb; x += 32) dst[op + 1 + x] = (uint8_t)(x < eb - 1 ? 255 : (lit - 15) % 255);
+        for (int x = lane; x < lit; x += 32) dst[o + x] = (uint8_t)es_byte(s, pr - lits + x);
+        if (lane < 2) dst[o + lit + lane] = (uint8_t)(d >> (8 * lane));
+        for (int x = lane; x < mb; x += 32) dst[o + lit + 2 + x] = (uint8_t)(x < mb - 1 ? 255 : (mc - 15) % 255);
+        op = o + lit + 2 + mb;
+        return true;
+    };
+    if (n >= 13) {
+        es_fill(s, ELOOK);
+        if (lane == 0) TPUT(es_hash(s, 0, SMALL), 0);
+        __syncwarp();
+        // `hot`: ip follows a match (liblz4 inserts ip - 2, then tests ip itself); else a search
+        // is under way whose t-th probe is p0 + probe_offset(t), t0 probes done.
+        bool hot = false;
+        int ip = 0, p0 = 1, t0 = 0;
+        const uint32_t head = ld4u(src);                        // the bytes an empty bucket's candidate 0 has
         for (;;) {
-            anchor = ip;
-            if (ip >= mfl1) goto last_literals;
-            if (ip + 64 > s.hi) es_fill(s, ip + ELOOK);
-            uint32_t a0, a1, a2, a3;                         // bytes ip-2 .. ip+13
+            if (hot && ip >= mfl1) break;
+            if (!hot && t0 > 33) {
+                // ---- probes with a growing step (the step is 1 for the first 66 probes)
+                bool end = false;
+                int pr = 0, c = 0;
+                for (;;) {
+                    es_fill(s, (int)min((uint32_t)p0 + probe_offset((uint32_t)t0), (uint32_t)n) + ELOOK);
+                    const uint32_t p = (uint32_t)p0 + probe_offset((uint32_t)(t0 + lane)),
+                                   pn = (uint32_t)p0 + probe_offset((uint32_t)(t0 + lane + 1));
+                    const bool valid = pn <= (uint32_t)mfl1;
+                    const uint32_t v = valid ? es_rd32(s, (int)p) : 0u;
+                    const uint32_t h = !valid ? 0x80000000u | (uint32_t)lane
+                                              : lz_hash_v<SMALL>(v, SMALL ? 0u : es_byte(s, (int)p + 4));
+                    const uint32_t ctab = valid ? TGET(h) : 0u;
+                    bool m = valid && (SMALL || ctab + 65535u >= p) && (ctab ? es_rd32(s, (int)ctab) : head) == v;
+                    const unsigned em = __ballot_sync(FULLMASK, !valid);
+                    const int E = em ? __ffs((int)em) - 1 : 32;
+                    unsigned mm = __ballot_sync(FULLMASK, m);
+                    int W = mm ? __ffs((int)mm) - 1 : 32;
+                    // The probes up to the first match enter the table.  Two of them with one hash
+                    // (seen when a lane reads back another's position) change what the later
+                    // one finds: then the step is taken again with the lanes' candidates among
+                    // the probes themselves.
+                    const bool put = lane <= min(W, E - 1);
+                    __syncwarp();
+                    if (put) TPUT(h, p);
+                    __syncwarp();
+                    const bool clash = put && TGET(h) != (SMALL ? p & 0xffffu : p);
+                    uint32_t cand = ctab;
+                    if (__any_sync(FULLMASK, clash)) {
+                        const unsigned peers = __match_any_sync(FULLMASK, h), lower = peers & lt;
+                        const int cl = lower ? 31 - __clz((int)lower) : lane;
+                        const uint32_t pl = __shfl_sync(FULLMASK, p, cl), vl = __shfl_sync(FULLMASK, v, cl);
+                        if (lower) {
+                            cand = pl;
+                            m = valid && (SMALL || cand + 65535u >= p) && vl == v;
+                        }
+                        mm = __ballot_sync(FULLMASK, m);
+                        W = mm ? __ffs((int)mm) - 1 : 32;
+                        const int lastw = min(W, E - 1);
+                        if (put) TPUT(h, ctab);
+                        __syncwarp();
+                        const unsigned upto = (lastw >= 31) ? FULLMASK : ((2u << lastw) - 1u);
+                        if (lane <= lastw && !(peers & ~lt & ~(1u << lane) & upto)) TPUT(h, p);
+                        __syncwarp();
+                    }
+                    if (W < E) {
+                        pr = (int)__shfl_sync(FULLMASK, p, W);
+                        c = (int)__shfl_sync(FULLMASK, cand, W);
+                        break;
+                    }
+                    if (E < 32) { end = true; break; }
+                    t0 += 32;
+                }
+                if (end) break;
+                if (!sequence(pr, pr - c, 4, true, 0, true)) { *need_out = need; return 0; }
+                ip = anchor;
+                hot = true;
+                continue;
+            }
+            // ---- window of 32 consecutive positions
+            const int w0 = hot ? ip - 2 : p0 + t0;
+            if (w0 + 64 > s.hi) es_fill(s, w0 + ELOOK);
+            const int p = w0 + lane;
+            const bool valid = p < mfl1;
+            uint32_t prev, v, n0, n1, n2;                       // bytes p-4 .., p .., p+4 .., p+8 .., p+12 ..
             {
-                const uint32_t o = (uint32_t)(ip - 2) & (ERING - 1);
-                const uint32_t wa = ring_s + (o & ~3u);
-                const uint32_t sh = (o & 3) * 8;
-                const uint32_t w0 = lds32(wa), w1 = lds32(wa + 4), w2 = lds32(wa + 8), w3 = lds32(wa + 12),
-                               w4 = lds32(wa + 16);
-                a0 = __funnelshift_r(w0, w1, sh);
-                a1 = __funnelshift_r(w1, w2, sh);
-                a2 = __funnelshift_r(w2, w3, sh);
-                a3 = __funnelshift_r(w3, w4, sh);
+                const uint32_t *w = rw + (((p >> 2) - 1) & wmask);
+                const uint32_t sh = (uint32_t)(p & 3) * 8;
+                prev = __funnelshift_r(w[0], w[1], sh);
+                v = __funnelshift_r(w[1], w[2], sh);
+                n0 = __funnelshift_r(w[2], w[3], sh);
+                n1 = __funnelshift_r(w[3], w[4], sh);
+                n2 = __funnelshift_r(w[4], w[5], sh);
             }
-            const uint32_t v0 = __funnelshift_r(a0, a1, 16);   // bytes ip .. ip+3
-            const uint32_t h2 = lz_hash_v<SMALL>(a0, a1 & 0xffu), h0 = lz_hash_v<SMALL>(v0, (a1 >> 16) & 0xffu);
-            const uint32_t c = (h0 == h2) ? (uint32_t)(ip - 2) : lds_tab(tab_s + (h0 << TSH), SMALL);
-            sts_tab(tab_s + (h2 << TSH), (uint32_t)(ip - 2), SMALL);
-            sts_tab(tab_s + (h0 << TSH), (uint32_t)ip, SMALL);
-            uint32_t cv, cn0, cn1;                            // bytes c .. c+11
-            if ((int)c >= s.lo) {
-                const uint32_t o = c & (ERING - 1);
-                const uint32_t wa = ring_s + (o & ~3u);
-                const uint32_t sh = (o & 3) * 8;
-                const uint32_t w0 = lds32(wa), w1 = lds32(wa + 4), w2 = lds32(wa + 8), w3 = lds32(wa + 12);
-                cv = __funnelshift_r(w0, w1, sh);
-                cn0 = __funnelshift_r(w1, w2, sh);
-                cn1 = __funnelshift_r(w2, w3, sh);
-            } else {
-                cv = ld4u(src + c);
-                cn0 = ld4u(src + c + 4);
-                cn1 = ld4u(src + c + 8);
+            const uint32_t h = lz_hash_v<SMALL>(v, n0 & 0xffu);
+            const int c = valid ? (int)TGET(h) : 0;
+            // lanes of the same hash: those that share its low 7 bits and those that share the
+            // rest, collected in shared memory (__match_any_sync takes about 11 cycles for every
+            // distinct value, 350 here; this 80)
+            if (valid) {
+                atomicOr(bm + (h & 127u), 1u << lane);
+                atomicOr(bm + 128 + (h >> 7), 1u << lane);
             }
-            if (!((SMALL || c + 65535u >= (uint32_t)ip) && cv == v0)) {
-                ip += 1;
-                __syncwarp();
-                break;                                        // back to searching from ip + 1
+            __syncwarp();
+            // the candidate's bytes: from the window when it (and the 4 bytes before it) are still
+            // there, else from global memory; the first 4 positions only as far as the match
+            bool hit_t;
+            uint32_t info;                                      // match length, backward length, distance
+            {
+                const bool inring = c - 4 >= s.lo || s.lo == 0;
+                const uintptr_t ca = reinterpret_cast<uintptr_t>(src) + (uintptr_t)(max(c, 4) - 4);
+                const uint32_t *w = inring ? rw + (((c >> 2) - 1) & wmask)
+                                           : reinterpret_cast<const uint32_t *>(ca & ~uintptr_t(3));
+                const uint32_t sh = (inring ? (uint32_t)c & 3u : (uint32_t)(ca & 3)) * 8;
+                const uint32_t w0_ = w[0], w1_ = w[1], w2_ = w[2], w3_ = w[3], w4_ = w[4], w5_ = w[5];
+                const uint32_t cp = __funnelshift_r(w0_, w1_, sh), c0 = __funnelshift_r(w2_, w3_, sh),
+                               c1 = __funnelshift_r(w3_, w4_, sh), c2 = __funnelshift_r(w4_, w5_, sh);
+                uint32_t cv = __funnelshift_r(w1_, w2_, sh);
+                const bool low = !inring && c < 4;
+                if (low) cv = __funnelshift_r(cp, cv, 8 * c);
+                hit_t = valid && cv == v && (SMALL || c + 65535 >= p);
+                const uint32_t x0 = n0 ^ c0, x1 = n1 ^ c1, x2 = n2 ^ c2;
+                const uint32_t x = x0 ? x0 : x1 ? x1 : x2;
+                int len = (x0 ? 4 : x1 ? 8 : 12) + (x ? (__ffs((int)x) - 1) >> 3 : 4);
+                int bk = min(__clz((int)(prev ^ cp)) >> 3, c);
+                uint32_t more = (len == 16 ? 1u : 0u) | (bk == 4 ? 2u : 0u);
+                if (low) { len = 4; bk = 0; more = 3u; }
+                info = (uint32_t)len | (more << 5) | ((uint32_t)bk << 8) | ((uint32_t)(p - c) << 16);
             }
-            const uint64_t nx = ((uint64_t)__funnelshift_r(a2, a3, 16) << 32) | __funnelshift_r(a1, a2, 16);
-            const uint64_t x = nx ^ (((uint64_t)cn1 << 32) | cn0);
-            const int lim = mlimit - (ip + 4);
-            int mc = x ? (__ffsll((long long)x) - 1) >> 3 : 8;
-            if (mc >= lim) {
-                mc = lim;
-            } else if (mc == 8) {                            // long match: warp-wide compare from ip + 12
-                for (int a = ip + 12, bpos = (int)c + 12;; a += 32, bpos += 32) {
-                    es_fill(s, a + 32 + ELOOK);
-                    const int pa = a + lane;
-                    const bool eq = pa < mlimit && es_byte(s, pa) == es_byte(s, bpos + lane);
-                    const unsigned ne = __ballot_sync(FULLMASK, !eq);
-                    const int cnum = ne ? __ffs(ne) - 1 : 32;
-                    mc += cnum;
-                    if (cnum < 32) break;
+            const unsigned peers = valid ? bm[h & 127u] & bm[128 + (h >> 7)] : 0u;
+            __syncwarp();
+            if (valid) { bm[h & 127u] = 0u; bm[128 + (h >> 7)] = 0u; }
+            const unsigned vmask = __ballot_sync(FULLMASK, valid), H = __ballot_sync(FULLMASK, hit_t);
+            // The step from this lane by the table's candidates alone: match at lane rq (32: none
+            // left), the next step at lane jq, lit literals and a match of mc + 4 bytes.  `odd`
+            // steps are walked below.
+            const unsigned hq = H & (FULLMASK << lane), reach = H ? FULLMASK >> __clz((int)H) : 0u;
+            const int rq = hq ? __ffs((int)hq) - 1 : 32;
+            const uint32_t iq = __shfl_sync(FULLMASK, info, rq & 31);
+            const int Lq = (int)(iq & 31u), bq = (int)((iq >> 8) & 7u);
+            const int jq = rq < 32 ? rq + Lq : 32;
+            auto odd_step = [&](int lits, int lit, int mc) {
+                return (iq & 32u) || ((iq & 64u) && lits > bq) || lit >= 15 || mc >= 15 || w0 + jq > mlimit;
+            };
+            int lit = rq - lane - min(bq, rq - lane), mc = Lq + min(bq, rq - lane) - 4;
+            bool odd = odd_step(rq - lane, lit, mc);
+            // Along the chain from this lane (at most 8 steps fit in a window): the lanes where a
+            // step starts (m), the lanes tested (tq), the bytes written (sq)
+            const int sz = rq < 32 ? 3 + lit : 0;
+            unsigned m = 1u << lane, tq = (FULLMASK << lane) & (rq < 32 ? FULLMASK >> (31 - rq) : FULLMASK);
+            int sq = sz;
+            {
+                int j = jq;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const unsigned mj = __shfl_sync(FULLMASK, m, j & 31), tj = __shfl_sync(FULLMASK, tq, j & 31);
+                    const int js = __shfl_sync(FULLMASK, j | (sq << 8), j & 31);
+                    if (j < 32) { m |= mj; tq |= tj; sq += js >> 8; j = js & 255; }
                 }
             }
-            const int mo = ip - (int)c;
-            NEED(op + 9 + (mc >= 15 ? (mc + 240) / 255 : 0));
-            if (lane == 0) {
-                uint8_t *dp = dst + op;
-                dp[0] = (uint8_t)(mc >= 15 ? 15 : mc);
-                dp[1] = (uint8_t)mo;
-                dp[2] = (uint8_t)(mo >> 8);
+            const unsigned plt = peers & lt;                    // earlier lanes of this lane's hash
+            unsigned ins = 0;                                   // inserted lanes
+            int q = hot ? 2 : 0;                                // the lane tested next
+            bool end = false;
+            for (;;) {
+                const unsigned vis = __shfl_sync(FULLMASK, m, q), tm = __shfl_sync(FULLMASK, tq, q);
+                const int s0 = __shfl_sync(FULLMASK, sq, q);
+                const unsigned hv = (hot ? vis : vis & ~(1u << q)) >> 2;
+                const int extra = w0 + q - anchor;              // literals before the first step's lane
+                int grow = 0;
+                if (extra > 0) {
+                    const int lits = rq - lane + extra, bk = min(bq, lits), l0 = lit;
+                    if (lane == q) {
+                        lit = lits - bk;
+                        mc = Lq + bk - 4;
+                        odd = odd_step(lits, lit, mc);
+                    }
+                    grow = __shfl_sync(FULLMASK, lit - l0, q);
+                }
+                const unsigned bit = 1u << lane, steps = vis & reach;
+                const unsigned viol = __ballot_sync(FULLMASK, ((steps & bit) && odd) || ((tm & bit) && (plt & (ins | tm | hv))));
+                // the steps before the first one to be walked
+                unsigned below = FULLMASK;
+                if (viol) below = (1u << (31 - __clz((int)(vis & (viol ^ (viol - 1)))))) - 1u;
+                const unsigned ems = steps & below;
+                ins |= (tm & below) | (hv & (below >> 2));
+                if (ems) {
+                    const int last = 31 - __clz((int)ems);
+                    const int ev = __shfl_sync(FULLMASK, jq | ((sq - sz) << 8), last);
+                    const int total = s0 - (ev >> 8) + grow;
+                    need = max(need, op + total + 6);           // op + lit + 9 of the last one
+                    if (need > cap) { *need_out = need; return 0; }
+                    const int off = s0 - sq + (lane == q ? 0 : grow);
+                    if (ems & bit) {
+                        uint8_t *o = dst + op + off;
+                        o[0] = (uint8_t)((lit << 4) | mc);
+                        o[1 + lit] = (uint8_t)(iq >> 16);
+                        o[2 + lit] = (uint8_t)(iq >> 24);
+                    }
+                    // literals: one lane each, those before the window's lanes first
+                    const unsigned vle = ems & (lt | bit);
+                    const int qv = 31 - __clz((int)vle);
+                    const int ov = __shfl_sync(FULLMASK, off | (lit << 16), qv & 31);
+                    const int x = lane - qv + (qv == q ? extra : 0);
+                    if (vle && x < (ov >> 16)) dst[op + (ov & 0xffff) + 1 + x] = (uint8_t)v;
+                    if (extra > 0) {
+                        const int lq = __shfl_sync(FULLMASK, lit, q);
+                        if (lane < min(extra, lq)) dst[op + 1 + lane] = (uint8_t)es_byte(s, anchor + lane);
+                    }
+                    op += total;
+                    hot = true;
+                    ip = anchor = w0 + (ev & 255);
+                    q = ip - w0;
+                    if (q > 31) break;
+                }
+                // ---- the step at q, walked: a lane past q is probed when all of q .. lane - 1
+                // were, which inserted them
+                const unsigned from = FULLMASK << q, hb = hot ? 1u << (q - 2) : 0u;
+                const unsigned pm = plt & (ins | hb | from);
+                const int cl0 = 31 - __clz((int)pm);
+                const uint32_t vc = __shfl_sync(FULLMASK, v, cl0 & 31);
+                const bool hit = pm ? vc == v : hit_t;
+                const unsigned b = __ballot_sync(FULLMASK, hit) & from & vmask;
+                if (!b) {
+                    ins |= hb | from;
+                    end = vmask != FULLMASK;
+                    if (hot) p0 = w0 + q + 1;
+                    hot = false;
+                    t0 = w0 + 32 - p0;
+                    break;
+                }
+                const int r = __ffs((int)b) - 1, pr = w0 + r;
+                ins |= hb | (from & (FULLMASK >> (31 - r)));
+                const uint32_t inf = __shfl_sync(FULLMASK, info, r);
+                const unsigned pmr = __shfl_sync(FULLMASK, pm, r);
+                int L, back, d;
+                bool longer, more_back;
+                if (pmr) {                                      // a match with lane cl of this window
+                    const int cl = 31 - __clz((int)pmr);
+                    d = r - cl;
+                    const uint32_t ob = __shfl_sync(FULLMASK, v, (lane - d) & 31);
+                    const unsigned eq = __ballot_sync(FULLMASK, lane >= d && ((v ^ ob) & 0xffu) == 0);
+                    L = __ffs((int)~(eq >> r)) - 1;             // r >= 1: the shifted-in bits end the run
+                    longer = r + L == 32;
+                    back = __clz((int)~(eq << (32 - r)));       // at most cl: lanes below d are not equal
+                    more_back = back == cl;
+                } else {
+                    L = (int)(inf & 31u);
+                    back = (int)((inf >> 8) & 7u);
+                    d = (int)(inf >> 16);
+                    longer = (inf & 32u) != 0;
+                    more_back = (inf & 64u) != 0;
+                }
+                if (!sequence(pr, d, L, longer, back, more_back && pr - anchor > back)) { *need_out = need; return 0; }
+                hot = true;
+                ip = anchor;
+                q = ip - w0;
+                if (q > 31) break;
             }
-            op += 3;
-            if (mc >= 15) {
-                const int rem = mc - 15, nff = rem / 255;
-                for (int xx = lane; xx < nff; xx += 32) dst[op + xx] = 255;
-                if (lane == 0) dst[op + nff] = (uint8_t)(rem % 255);
-                op += nff + 1;
-            }
-            ip += mc + 4;
+            if (((ins >> lane) & 1u) && !(peers & ins & ~lt & ~(1u << lane))) TPUT(h, p);
+            __syncwarp();
+            if (end) break;
         }
     }
-last_literals:
     {
         const int last = n - anchor;
-        NEED(op + last + 1 + (last + 255 - 15) / 255);
+        need = max(need, op + last + 1 + (last + 255 - 15) / 255);
+        if (need > cap) { *need_out = need; return 0; }
         if (last >= 15) {
             const int rem = last - 15, nff = rem / 255;
             if (lane == 0) dst[op] = 15 << 4;
@@ -1333,10 +1475,20 @@ last_literals:
     }
 #undef TGET
 #undef TPUT
-#undef NEED
     __syncwarp();
     *need_out = need;
     return op;
+}
+
+// The k-th stream to be handed out of `total` streams, `per` per block: the last stream of every
+// block first, then the one before it.  In little-endian shuffled floats the last byte planes
+// (sign, exponent) compress and cost up to a hundred times what an incompressible plane costs; in
+// block order the last ones would start when the other streams are done and run on alone.
+__device__ __forceinline__ int64_t stream_at(int64_t k, int64_t total, int per)
+{
+    int64_t j, b;
+    divmod(k, total / per, j, b);
+    return b * per + (per - 1 - j);
 }
 
 // E2: one warp per stream: run check, then LZ4 into the stream's slot (capacity =
@@ -1344,19 +1496,21 @@ last_literals:
 // Streams are handed out dynamically (one atomic per stream): compressible streams cost
 // far more than incompressible ones, and in shuffled float data they recur at a fixed
 // stride, which a static round-robin assignment would pile onto the same warps.
-__global__ void __launch_bounds__(32, 10) k_lz4_encode(const uint8_t *__restrict__ img, int64_t nstreams_total,
-                                                    int neblock, uint8_t *slots, EncStream *es,
+__global__ void __launch_bounds__(32, XCTAS) k_lz4_encode(const uint8_t *__restrict__ img, int64_t nstreams_total,
+                                                    int per, int neblock, uint8_t *slots, EncStream *es,
                                                     unsigned long long *next)
 {
     extern __shared__ __align__(16) uint32_t sm_tab[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t *tab = sm_tab + warp * (4096 + (ERING + 16) / 4);
-    uint8_t *ring = reinterpret_cast<uint8_t *>(tab + 4096);
+    uint32_t *tab = sm_tab + warp * (4096 + EPEER + (XRING + EMIRROR) / 4);
+    uint32_t *bm = tab + 4096;
+    uint8_t *ring = reinterpret_cast<uint8_t *>(bm + EPEER);
     for (;;) {
         unsigned long long got = 0;
         if (lane == 0) got = atomicAdd(next, 1ull);
-        const int64_t sid = (int64_t)__shfl_sync(FULLMASK, got, 0);
-        if (sid >= nstreams_total) break;
+        const int64_t k = (int64_t)__shfl_sync(FULLMASK, got, 0);
+        if (k >= nstreams_total) break;
+        const int64_t sid = stream_at(k, nstreams_total, per);
         const uint8_t *src = img + sid * neblock;
         const uint8_t first = __ldg(src);
         bool run = true;
@@ -1375,8 +1529,8 @@ __global__ void __launch_bounds__(32, 10) k_lz4_encode(const uint8_t *__restrict
         } else {
             int need = 0;
             const int cs = neblock < 65536 + 12 - 1
-                               ? warp_lz4_compress<true>(src, neblock, slots + sid * neblock, neblock, tab, ring, &need)
-                               : warp_lz4_compress<false>(src, neblock, slots + sid * neblock, neblock, tab, ring, &need);
+                               ? warp_lz4_compress<true>(src, neblock, slots + sid * neblock, neblock, tab, bm, ring, XRING, &need)
+                               : warp_lz4_compress<false>(src, neblock, slots + sid * neblock, neblock, tab, bm, ring, XRING, &need);
             if (cs > 0 && cs < neblock) { e.kind = SK_LZ4; e.csize = cs; e.need = need; }
             else { e.kind = SK_RAW; e.csize = neblock; e.need = need; }
         }
@@ -1415,7 +1569,7 @@ struct ParSmem {              // per CTA
         uint16_t tab16[8192]; // liblz4 search (byU16); probe: four tables of 2048
         uint32_t tab32[4096]; // parallel parse: position + 1 of each bucket (0: empty); liblz4 byU32
     };
-    uint8_t ring[ERING + 16];
+    uint8_t ring[ERING + EMIRROR];
     union {
         struct {
             uint16_t cw[PW];  // match distance of each window position
@@ -1424,6 +1578,7 @@ struct ParSmem {              // per CTA
             uint16_t path[PW / 4 + 2];
         } w;
         uint8_t stage[4][PSTAGE];
+        uint32_t peer[EPEER]; // liblz4 search: lanes-by-hash masks
     };
     uint32_t bits[32];        // match flags, one word per 32 positions
     int32_t nchain;           // matches on the window's chain
@@ -1493,7 +1648,7 @@ __device__ __forceinline__ void cta_fill(EncSrc &s, int want)
             }
             const int o = (base + x) & (ERING - 1);
             *reinterpret_cast<uint32_t *>(s.r + o) = v;
-            if (o < 16) *reinterpret_cast<uint32_t *>(s.r + ERING + o) = v;
+            if (o < EMIRROR) *reinterpret_cast<uint32_t *>(s.r + ERING + o) = v;
         }
         s.hi = base + cnt;
         s.lo = max(s.lo, base + ESEG - ERING);
@@ -1530,7 +1685,7 @@ __device__ __forceinline__ int cta_lz4_compress_par(const uint8_t *__restrict__ 
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(S.ring);
     for (int i = tid; i < 4096 / 4; i += PT) reinterpret_cast<uint4 *>(S.tab32)[i] = make_uint4(0u, 0u, 0u, 0u);
     EncSrc s;
-    s.g = src; s.r = S.ring; s.lo = 0; s.hi = 0; s.n = n;
+    s.g = src; s.r = S.ring; s.cap = ERING; s.lo = 0; s.hi = 0; s.n = n;
     __syncthreads();
     int op = 0, anchor = 0, pos = 0;
     const int mfl1 = n - 11, mlimit = n - 5;
@@ -1806,7 +1961,7 @@ __device__ __forceinline__ int cta_probe(const uint8_t *__restrict__ src, int n,
 // byte planes): stored raw; few matches: the liblz4 search (one warp), whose accelerating
 // skip makes them cheap; the rest: the parallel parse.
 __global__ void __launch_bounds__(PT, 8) k_lz4_encode_par(const uint8_t *__restrict__ img, int64_t nstreams_total,
-                                                       int neblock, uint8_t *slots, EncStream *es,
+                                                       int per, int neblock, uint8_t *slots, EncStream *es,
                                                        unsigned long long *next)
 {
     extern __shared__ __align__(16) uint8_t sm_par[];
@@ -1815,9 +1970,10 @@ __global__ void __launch_bounds__(PT, 8) k_lz4_encode_par(const uint8_t *__restr
     for (;;) {
         if (tid == 0) S.sid = (long long)atomicAdd(next, 1ull);
         __syncthreads();
-        const int64_t sid = S.sid;
+        const int64_t k = S.sid;
         __syncthreads();
-        if (sid >= nstreams_total) break;
+        if (k >= nstreams_total) break;
+        const int64_t sid = stream_at(k, nstreams_total, per);
         const uint8_t *src = img + sid * neblock;
         const uint8_t first = __ldg(src);
         bool run = true;
@@ -1841,8 +1997,8 @@ __global__ void __launch_bounds__(PT, 8) k_lz4_encode_par(const uint8_t *__restr
                 if (warp == 0) {
                     int need = 0;
                     const int cs = neblock < 65536 + 12 - 1
-                                       ? warp_lz4_compress<true>(src, neblock, slots + sid * neblock, neblock, S.tab32, S.ring, &need)
-                                       : warp_lz4_compress<false>(src, neblock, slots + sid * neblock, neblock, S.tab32, S.ring, &need);
+                                       ? warp_lz4_compress<true>(src, neblock, slots + sid * neblock, neblock, S.tab32, S.peer, S.ring, ERING, &need)
+                                       : warp_lz4_compress<false>(src, neblock, slots + sid * neblock, neblock, S.tab32, S.peer, S.ring, ERING, &need);
                     if (cs > 0 && cs < neblock) { e.kind = SK_LZ4; e.csize = cs; e.need = need; }
                     else { e.kind = SK_RAW; e.csize = neblock; e.need = need; }
                 }
@@ -2299,21 +2455,21 @@ int encode_gather(const Geom &g, const void *in, int64_t ld, bool shuffle, int s
     return 0;
 }
 
-void encode_streams(const uint8_t *img, int64_t ns, int neblock, uint8_t *slots, EncStream *es,
+void encode_streams(const uint8_t *img, int64_t ns, int per, int neblock, uint8_t *slots, EncStream *es,
                     unsigned long long *cursor, bool exact_lz4, cudaStream_t st)
 {
     const int sms = sm_count();
     if (exact_lz4) {
         static bool attr = false;
-        // per warp: 16 KiB hash table + the source window; 1 warp per CTA, 10 CTAs per SM
-        const int wpb = 1, smem = wpb * (4096 * 4 + ERING + 16);
+        // per warp: 16 KiB hash table, lane masks, the source window; 1 warp per CTA, XCTAS per SM
+        const int wpb = 1, smem = wpb * (4096 * 4 + EPEER * 4 + XRING + EMIRROR);
         if (!attr) {
             cudaFuncSetAttribute(k_lz4_encode, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             attr = true;
         }
-        const int64_t blocks = std::min<int64_t>((ns + wpb - 1) / wpb, (int64_t)sms * 10);
+        const int64_t blocks = std::min<int64_t>((ns + wpb - 1) / wpb, (int64_t)sms * XCTAS);
         IAB_TIMED("k_lz4_encode", st, k_lz4_encode<<<(unsigned)std::max<int64_t>(blocks, 1), wpb * 32, smem, st>>>(
-            img, ns, neblock, slots, es, cursor));
+            img, ns, per, neblock, slots, es, cursor));
     } else {
         static bool attr = false;
         const int smem = (int)sizeof(ParSmem);                 // one stream per CTA of PT threads, 8 CTAs per SM
@@ -2323,7 +2479,7 @@ void encode_streams(const uint8_t *img, int64_t ns, int neblock, uint8_t *slots,
         }
         const int64_t blocks = std::min<int64_t>(ns, (int64_t)sms * 8);
         IAB_TIMED("k_lz4_encode_par", st, k_lz4_encode_par<<<(unsigned)std::max<int64_t>(blocks, 1), PT, smem, st>>>(
-            img, ns, neblock, slots, es, cursor));
+            img, ns, per, neblock, slots, es, cursor));
     }
 }
 
@@ -2361,7 +2517,7 @@ int encode_launch(const Geom &g, const void *in, int64_t ld, bool shuffle, int s
     if (r) return r;
     const int nstreams = encode_nstreams(g, shuffle, splitmode);
     if (!w->memcpy_only)
-        encode_streams(w->img.as<uint8_t>(), g.nchunks * g.nblocks * nstreams, (int)(g.blocksize / nstreams),
+        encode_streams(w->img.as<uint8_t>(), g.nchunks * g.nblocks * nstreams, nstreams, (int)(g.blocksize / nstreams),
                        w->slots.as<uint8_t>(), w->es.as<EncStream>(),
                        reinterpret_cast<unsigned long long *>(w->tot.as<int64_t>() + 1), w->exact_lz4, st);
     return encode_emit(g, shuffle, splitmode, d_out, w, st);
@@ -3020,7 +3176,7 @@ int encode_group_launch(CodecGroup *grp, bool exact_lz4, bool memcpy_only, cudaS
                                                                            grp->shuffle));
     }
     if (!memcpy_only)
-        encode_streams(grp->img.as<uint8_t>(), grp->nbl * grp->nstreams, grp->neblock, grp->slots.as<uint8_t>(),
+        encode_streams(grp->img.as<uint8_t>(), grp->nbl * grp->nstreams, grp->nstreams, grp->neblock, grp->slots.as<uint8_t>(),
                        grp->es.as<EncStream>(), reinterpret_cast<unsigned long long *>(grp->counters.as<uint8_t>() + 64),
                        exact_lz4, st);
     IAB_TIMED("k_layout", st, k_layout_g<<<(unsigned)std::max<int64_t>(grp->nch, 1), LAYOUT_T, 0, st>>>(

@@ -249,12 +249,12 @@ int encode_image_finish(const Geom &g, bool shuffle, int splitmode, DevBuf *d_ou
 
 // encode_launch in stages, so that several containers can share one LZ4 launch:
 // encode_gather (dense -> byte-plane image), encode_streams (LZ4 over ns streams of neblock
-// bytes each; the streams of several containers when their images, slots and results lie
+// bytes each, `per` streams per block; the streams of several containers when their images, slots and results lie
 // back to back), encode_emit (chunk layout, offsets, payloads into *d_out).  The stream
 // cursor `cursor` must be zero before encode_streams.
 int encode_nstreams(const Geom &g, bool shuffle, int splitmode);
 int encode_gather(const Geom &g, const void *in, int64_t ld, bool shuffle, int splitmode, EncodeWork *w, cudaStream_t st);
-void encode_streams(const uint8_t *img, int64_t ns, int neblock, uint8_t *slots, EncStream *es,
+void encode_streams(const uint8_t *img, int64_t ns, int per, int neblock, uint8_t *slots, EncStream *es,
                     unsigned long long *cursor, bool exact_lz4, cudaStream_t st);
 int encode_emit(const Geom &g, bool shuffle, int splitmode, DevBuf *d_out, EncodeWork *w, cudaStream_t st);
 int encode_finish(EncodeWork *w, std::vector<int64_t> *h_off, std::vector<int32_t> *h_len, cudaStream_t st);
