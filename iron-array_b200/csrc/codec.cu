@@ -1990,7 +1990,8 @@ __global__ void __launch_bounds__(PT, 8) k_lz4_encode_par(const uint8_t *__restr
         if (run) {
             e.kind = SK_RUN; e.csize = first; e.need = 0;
         } else {
-            const int hits = cta_probe(src, neblock, S);
+            // (LZ4 compresses no block below 13 bytes, and the probe's windows need 11)
+            const int hits = neblock < 13 ? 0 : cta_probe(src, neblock, S);
             if (hits < 16) {                     // no matches to speak of: store the stream raw
                 e.kind = SK_RAW; e.csize = neblock; e.need = neblock + 1;
             } else if (hits < 256) {

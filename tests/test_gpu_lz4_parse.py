@@ -42,3 +42,17 @@ def test_streams_equal_the_oracles(ctx, ia, n):
         _, want = O.encode_array(x, (n,), (n,))
         assert c.chunks() == want, (n, i)
         c.free()
+
+
+@pytest.mark.parametrize("n", range(1, 15))
+def test_parallel_encoder_streams_below_its_probe(ia, n):
+    """Streams of a few bytes: shorter than the 13 bytes LZ4 compresses and the 11 the probe of
+    the parallel encoder reads at a time; they are stored raw."""
+    ctx = ia.Context(encoder=ia.ENCODER_PARALLEL)
+    x = np.random.default_rng(n).integers(0, 256, 7 * n).astype(np.uint8)
+    c = ia.Container.from_numpy(ctx, x, (7 * n,), (n,))
+    _, want = O.encode_array(x, (7 * n,), (n,))
+    assert c.chunks() == want
+    assert np.array_equal(c.to_numpy(), x)
+    c.free()
+    ctx.close()
