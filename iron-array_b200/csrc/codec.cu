@@ -158,50 +158,71 @@ __global__ void k_parse(Geom g, const uint8_t *__restrict__ ch, const int64_t *_
 
 // D1: LZ4 stream decode, one CTA (256 threads) per stream, streams handed out
 // dynamically from a job queue (which may hold the streams of several containers: each job
-// carries its source, destination and status word).  The stream is consumed in windows of up to DW compressed bytes staged in
-// shared memory, and each window is decoded without any serial walk:
-//  1. for every byte q of the window, next[q] = where the following token would start if
-//     a sequence began at q (STOP when that sequence does not end inside the window,
-//     ENDS when it is the stream's last, literal-only sequence);
-//  2. the chain of token positions from the window start is built by pointer doubling
-//     (next, next^2, next^4, ... composed in two ping-pong tables, the chain doubled
-//     alongside), so the window's sequences are all located in O(log) parallel steps;
-//  3. their literal and match lengths are read in parallel and an exclusive scan gives
-//     each sequence's output offset;
-//  4. the output is resolved in groups of at most DCAP bytes in shared memory: a literal
+// carries its source, destination and status word).  The stream is consumed in windows of up
+// to DW compressed bytes staged in shared memory (the next window's loads are issued as soon
+// as its start is known).  With many streams in flight the SM's issue rate bounds the kernel,
+// so each step is chosen for few instructions per byte:
+//  1. the chain of token positions from the window start: every thread walks the tokens of one
+//     32-byte segment from one of its first four bytes, four tracks per segment.  A walk from
+//     a wrong byte need not meet the true chain soon (sequences of 3 bytes keep their phase),
+//     but the true chain soon runs on one of the four tracks: so a track's exit is linked to
+//     the track it enters (after a few more tokens, where it is on none), and the tracks on
+//     the path from the window start are marked by pointer doubling over the 256 tracks.  The
+//     result is a bit per window byte.  (Doubling over every byte of the window took 24,000 of
+//     a window's 51,000 cycles, with the SM full; this takes 8,700 of 27,000);
+//  2. each thread reads the lengths of the tokens of its 8 bytes, and an exclusive scan over
+//     token counts and output lengths numbers the sequences and places their output;
+//  3. the output is resolved in groups of at most DCAP bytes in shared memory: a literal
 //     byte takes its value from the window, a match byte points at its source (a source
-//     inside the same match is folded back below the match start modulo the offset), and
-//     pointer jumping settles every byte in O(log depth) rounds; sources before the group
-//     are read from the already written output;
+//     inside the same match is folded back below the match start modulo the offset); sources
+//     before the group are read from the already written output (a ring of its latest bytes,
+//     else global memory).  Sequences are filled by one, eight or all threads, by length;
+//  4. every byte follows its sources (at most HOPS of them per sweep; a byte left open keeps
+//     its place on the chain, so that the chains through it shorten) and is written;
 //  5. a sequence with more than DCAP output bytes is copied straight in global memory
 //     (all its sources lie before its own match start), and a sequence too long for a
 //     window is decoded alone with its header read from global memory.
+// Measured against the doubled chain, matches copied byte by byte from global memory where the
+// ring did not reach, and separate resolving and writing sweeps: a 512 MiB float64 operand pair
+// of 64 KiB planes 2.06 -> 1.25 ms, 250 KB planes of a smooth 1.6 GB float32 matrix 9.85 -> 6.1 ms.
 namespace dcta {
 constexpr int THREADS = 256;
 constexpr int DW = 2048;                   // compressed bytes per window
+constexpr int SEG = 32, NSEG = DW / SEG;   // segments of the chain walk
+constexpr int TRACKS = THREADS / NSEG;
+constexpr int SPAN = DW / THREADS;         // per thread of the field step (at most 3 tokens)
 constexpr int MAXS = DW / 3 + 2;           // sequences per window (a non-final one takes >= 3 bytes)
-constexpr int PATH = 1024;                 // >= 2 * the largest power of two below MAXS + 1
-constexpr int HB = 4096;                   // output history kept in shared memory for match sources
-constexpr int LONGSEQ = 64;                // longer sequences are filled by the whole CTA
-constexpr int DCAP = 4096;                 // output bytes resolved in shared memory at once
-constexpr int WALK_MAX = 24;               // chains of at most this many sequences are walked
+constexpr int HB = 8192;                   // output history kept in shared memory for match sources
+constexpr int LONGSEQ = 16, GROUP = 8;     // longer sequences are filled by GROUP threads
+constexpr int VLONG = 256;                 // and longer ones by the whole CTA
+constexpr int DCAP = 3584;                 // output bytes resolved in shared memory at once
+constexpr int HOPS = 12;
+constexpr int WALK_MAX = 32;               // chains of at most this many sequences are walked by one thread
 constexpr uint16_t STOP = 0xFFFF, ENDS = 0xFFFE;
 constexpr uint32_t RES = 0x80000000u;      // resolved output byte (value in the low 8 bits)
+constexpr uint32_t BIAS = 65536;           // else the source's place relative to the group, plus BIAS
 struct Smem {
     union {
-        uint32_t st[DCAP];                 // per output byte: RES | value, or the source's index
-        uint16_t J[2][DW];                 // next-token tables (dead once the window's chain is known)
+        uint32_t st[DCAP];                 // per output byte
+        struct {                           // the chain walk (before the output is resolved)
+            uint32_t m[THREADS];           // a track's tokens, track-major
+            uint32_t any[NSEG];            // the tokens of a segment's tracks
+            uint16_t link[2][THREADS + 1]; // the track after it, then the 2nd, 4th, ... (THREADS: none)
+            uint16_t entry[THREADS];       // where the path enters a track
+            uint8_t on[THREADS];           // on the path
+        } c;
     };
     int32_t ostart[MAXS + 1];              // output offset of each sequence in the window
-    int32_t llen[MAXS];
+    uint16_t llen[MAXS];
     int32_t mlen[MAXS];
     uint16_t lpos[MAXS];
     uint16_t off[MAXS];
-    uint16_t path[PATH];
-    uint8_t win[DW + 16];
+    uint32_t mask[DW / 32];                // token positions
+    uint4 raw[DW / 16 + 1];                // the window from its 16-byte boundary
     uint8_t hist[HB];                      // the last HB output bytes (ring, by absolute position)
-    int32_t longs[DCAP / (LONGSEQ + 1) + 1];  // sequences of a group longer than LONGSEQ bytes
-    int32_t nlong;
+    uint16_t longs[DCAP / (LONGSEQ + 1) + 1];  // sequences of a group longer than LONGSEQ bytes
+    uint16_t vlongs[DCAP / (VLONG + 1) + 1];   // longer than VLONG bytes
+    int32_t nlong, nvlong;
     int32_t wsum[THREADS / 32];
     int32_t scal[9];
 };
@@ -211,9 +232,10 @@ struct Smem {
 // the stream from the window start).
 __device__ __forceinline__ uint16_t dcta_next(const uint8_t *win, int q, int n, int rem)
 {
-    int r = q + 1;
     const int tok = win[q];
-    int lit = tok >> 4;
+    int lit = tok >> 4, r = q + 3 + lit;
+    if (lit != 15 && (tok & 15) != 15 && r <= n) return (uint16_t)r;
+    r = q + 1;
     if (lit == 15) {
         int b = 255;
         while (b == 255) {
@@ -246,7 +268,13 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
     Smem &S = *reinterpret_cast<Smem *>(sm_dcta);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int njobs = (int)min((int64_t)*njobs_p, jcap);
-    if (tid == 0) S.nlong = 0;                     // first use follows the barriers below
+    if (tid == 0) S.nlong = S.nvlong = 0;          // first use follows the barriers below
+    // 16 bytes of the window at p from its 16-byte boundary; every block read holds a byte of the stream
+    auto fetch = [&](const uint8_t *in, int p, int isz) -> uint4 {
+        const int y = tid * 16 - (int)(reinterpret_cast<uintptr_t>(in + p) & 15);
+        return tid <= DW / 16 && p + y < isz && y < DW ? __ldg(reinterpret_cast<const uint4 *>(in + p + y))
+                                                       : make_uint4(0u, 0u, 0u, 0u);
+    };
     for (;;) {
         __syncthreads();
         if (tid == 0) S.scal[0] = (int)atomicAdd(next_job, 1u);
@@ -261,120 +289,131 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
         int p = 0, op = 0;                 // window start in the input, output written so far
         int hist_from = 0;                 // S.hist holds output bytes [hist_from, written)
         bool bad = false, done = false;    // block-uniform
-        bool walk = true;                  // block-uniform: walk this window's chain (sparse windows)
+        bool walk = false;                 // block-uniform: one thread walks this window's chain (after a sparse window)
+        uint4 pre = fetch(in, 0, isz);
         while (!done && !bad) {
             const int rem = isz - p, n = min(DW, rem);
+            const uint8_t *win = reinterpret_cast<const uint8_t *>(S.raw) + (reinterpret_cast<uintptr_t>(in + p) & 15);
             __syncthreads();
-            {                                          // every load issued before any store
-                uint8_t v[DW / THREADS];
-#pragma unroll
-                for (int k = 0; k < DW / THREADS; k++) {
-                    const int x = tid + k * THREADS;
-                    v[k] = x < n ? __ldg(in + p + x) : (uint8_t)0;
-                }
-#pragma unroll
-                for (int k = 0; k < DW / THREADS; k++) S.win[tid + k * THREADS] = v[k];
-            }
+            if (tid <= DW / 16) S.raw[tid] = pre;
+            if (tid < DW / 32) S.mask[tid] = 0;
             __syncthreads();
-            // Windows of few sequences (long literal runs, long matches): one thread walks the
+            if (n <= 0) { bad = true; break; }
+            // After a window of few sequences (long literal runs, long matches) one thread walks the
             // chain of token positions, at most WALK_MAX steps; when the chain does not leave the
-            // window by then, and for the windows that follow a dense one, the chain is built by
-            // doubling.  Both leave path[0 .. cnt) = token positions, path[cnt] >= n.
-            int cnt = -1;
+            // window by then, and in the other windows, all threads walk tracks.  Both leave the tokens in mask, why the chain ended (n, ENDS or STOP) in
+            // scal[1], the last token in scal[3].
+            bool found = false;
             if (walk) {
                 if (tid == 0) {
-                    int q = 0, k = 0, res = -1;
-                    S.path[0] = 0;
+                    int q = 0, k = 0, res = 0;
                     for (;;) {
-                        const uint16_t v = dcta_next(S.win, q, n, rem);
-                        S.path[++k] = v;
-                        if (v >= n) { res = k; break; }
-                        if (k >= WALK_MAX) break;
+                        const uint16_t v = dcta_next(win, q, n, rem);
+                        S.mask[q >> 5] |= 1u << (q & 31);
+                        if (v >= n) { res = 1; S.scal[1] = v; S.scal[3] = q; break; }
+                        if (++k >= WALK_MAX) break;
                         q = v;
                     }
                     S.scal[8] = res;
                 }
                 __syncthreads();
-                cnt = S.scal[8];
+                found = S.scal[8] != 0;
             }
-            if (cnt < 0) {
+            if (!found) {
+                const int seg = tid % NSEG, lo = seg * SEG, hi = min(lo + SEG, n);
+                uint32_t m = 0;
+                int x = lo + tid / NSEG;
+                while (x < hi) {                            // positions grow: at most SEG / 3 + 1 steps
+                    m |= 1u << (x - lo);
+                    x = dcta_next(win, x, n, rem);
+                }
+                S.c.m[tid] = m;
+                if (tid < DW / 32) S.mask[tid] = 0;         // (the one-thread walk's, when it gave up)
+                __syncthreads();
+                if (tid < NSEG) {
+                    uint32_t any = 0;
 #pragma unroll
-            for (int k = 0; k < DW / THREADS; k++) {      // eight independent table entries per thread
-                const int q = tid + k * THREADS;
-                if (q < n) S.J[0][q] = dcta_next(S.win, q, n, rem);
-            }
-            if (tid == 0) { S.path[0] = 0; S.scal[1] = PATH; }
-            __syncthreads();
-            // chain of token positions by doubling: after level k, path[0 .. 2^(k+1)) known
-            int len = 1, cur = 0;
-            for (;;) {
-                for (int j = tid; j < len; j += THREADS) {
-                    const uint16_t pj = S.path[j];
-                    const uint16_t v = pj < n ? S.J[cur][pj] : pj;
-                    S.path[len + j] = v;
-                    if (v >= n) atomicMin(&S.scal[1], len + j);
+                    for (int t = 0; t < TRACKS; t++) any |= S.c.m[t * NSEG + tid];
+                    S.c.any[tid] = any;
                 }
                 __syncthreads();
-                const int t = S.scal[1];
-                if (t < 2 * len) { cnt = t; break; }
-                // J_{k+1} = J_k o J_k (a thread's loads issued together, then its stores)
-                {
-                    uint16_t v[DW / THREADS], w[DW / THREADS];
+                int e = x, link = THREADS;
+                while (e < n && !((S.c.any[e / SEG] >> (e % SEG)) & 1u)) e = dcta_next(win, e, n, rem);
+                if (e < n) {
 #pragma unroll
-                    for (int k = 0; k < DW / THREADS; k++) {
-                        const int q = tid + k * THREADS;
-                        v[k] = q < n ? S.J[cur][q] : (uint16_t)0xFFFF;
-                    }
-#pragma unroll
-                    for (int k = 0; k < DW / THREADS; k++) w[k] = v[k] < n ? S.J[cur][v[k]] : v[k];
-#pragma unroll
-                    for (int k = 0; k < DW / THREADS; k++) {
-                        const int q = tid + k * THREADS;
-                        if (q < n) S.J[cur ^ 1][q] = w[k];
-                    }
+                    for (int t = 0; t < TRACKS; t++)
+                        if ((S.c.m[t * NSEG + e / SEG] >> (e % SEG)) & 1u) link = t * NSEG + e / SEG;
                 }
-                cur ^= 1;
-                len *= 2;
+                S.c.link[0][tid] = (uint16_t)link;
+                S.c.on[tid] = tid == 0;                     // the window starts on track 0 of segment 0
+                if (tid == 0) S.c.link[0][THREADS] = S.c.link[1][THREADS] = (uint16_t)THREADS;
+                __syncthreads();
+                int j = link;
+#pragma unroll
+                for (int k = 0; (1 << k) < NSEG; k++) {     // tracks fewer than 2^k links away are on
+                    if (S.c.on[tid] && j < THREADS) S.c.on[j] = 1;
+                    j = S.c.link[k & 1][j];
+                    S.c.link[(k & 1) ^ 1][tid] = (uint16_t)j;
+                    __syncthreads();
+                }
+                const bool on = S.c.on[tid];
+                if (on) {
+                    int last = lo + 31 - __clz((int)m);
+                    for (int t = x; t != e; t = dcta_next(win, t, n, rem)) {   // tokens on no track
+                        atomicOr(&S.mask[t >> 5], 1u << (t & 31));
+                        last = t;
+                    }
+                    if (link < THREADS) S.c.entry[link] = (uint16_t)e;
+                    else { S.scal[1] = e; S.scal[3] = last; }
+                }
+                __syncthreads();
+                if (on) atomicOr(&S.mask[seg], m & (FULLMASK << (tid ? S.c.entry[tid] % SEG : 0)));
                 __syncthreads();
             }
-            }
-            walk = cnt <= WALK_MAX;
-            const uint16_t term = S.path[cnt];          // n, ENDS or STOP
-            const int nseq = term == STOP ? cnt - 1 : cnt;
-            if (nseq > 0) {
-                // sequence fields and validity
+            const int term = S.scal[1], lastq = S.scal[3];  // term: n, ENDS or STOP
+            const int pnext = p + (term == STOP ? lastq : n);
+            if (term != STOP || lastq > 0) {                // at least one whole sequence
+                if (term != ENDS) pre = fetch(in, pnext, isz);
+                // sequence fields and validity: the tokens of this thread's SPAN bytes
                 if (tid == 0) S.scal[2] = 0;
-                int part = 0;
-                constexpr int PER = (MAXS + THREADS - 1) / THREADS;
-                const int i0 = tid * PER;
-                for (int i = i0; i < min(i0 + PER, nseq); i++) {
-                    const int q = S.path[i];
-                    const int tok = S.win[q];
-                    int r = q + 1, lit = tok >> 4;
-                    if (lit == 15) {
-                        int b = 255;
-                        while (b == 255) { b = S.win[r++]; lit += b; }
-                    }
-                    S.lpos[i] = (uint16_t)r;
-                    S.llen[i] = lit;
-                    r += lit;
-                    int ml = 0, mo = 0;
-                    if (!(i == nseq - 1 && term == ENDS)) {
-                        mo = S.win[r] | (S.win[r + 1] << 8);
-                        r += 2;
-                        ml = tok & 15;
-                        if (ml == 15) {
+                int part = 0, num = 0;                      // output bytes, sequences
+                int f_lit[3], f_ml[3], f_lp[3], f_off[3];
+                uint32_t mt = (S.mask[tid * SPAN >> 5] >> (tid * SPAN & 31)) & ((1u << SPAN) - 1u);
+                if (term == STOP && lastq / SPAN == tid) mt &= ~(1u << (lastq % SPAN));   // not whole
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    f_lit[k] = f_ml[k] = f_lp[k] = f_off[k] = 0;
+                    if (mt) {
+                        const int q = tid * SPAN + __ffs((int)mt) - 1;
+                        mt &= mt - 1;
+                        const int tok = win[q];
+                        int r = q + 1, lit = tok >> 4;
+                        if (lit == 15) {
                             int b = 255;
-                            while (b == 255) { b = S.win[r++]; ml += b; }
+                            while (b == 255) { b = win[r++]; lit += b; }
                         }
-                        ml += 4;
+                        f_lp[k] = r;
+                        f_lit[k] = lit;
+                        r += lit;
+                        int ml = 0;
+                        if (!(q == lastq && term == ENDS)) {
+                            f_off[k] = win[r] | (win[r + 1] << 8);
+                            r += 2;
+                            ml = tok & 15;
+                            if (ml == 15) {
+                                int b = 255;
+                                while (b == 255) { b = win[r++]; ml += b; }
+                            }
+                            ml += 4;
+                        }
+                        f_ml[k] = ml;
+                        part += lit + ml;
+                        num++;
                     }
-                    S.off[i] = (uint16_t)mo;
-                    S.mlen[i] = ml;
-                    part += lit + ml;
                 }
-                // exclusive scan of the output lengths
-                int incl = part;
+                // exclusive scan of counts (10 bits) and output lengths (below 255 DW < 2^20)
+                static_assert(MAXS < 1024 && 255 * DW < (1 << 20), "packed scan");
+                int incl = part | (num << 20);
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const int v = __shfl_up_sync(FULLMASK, incl, o);
@@ -383,17 +422,31 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
                 if (lane == 31) S.wsum[warp] = incl;
                 __syncthreads();
                 int wbase = 0;
-                for (int w = 0; w < warp; w++) wbase += S.wsum[w];
-                int acc = wbase + incl - part;
-                for (int i = i0; i < min(i0 + PER, nseq); i++) {
-                    S.ostart[i] = acc;
-                    const int ms = op + acc + S.llen[i];             // absolute match start
-                    if (S.mlen[i] > 0 && (S.off[i] == 0 || S.off[i] > ms)) S.scal[2] = 1;
-                    acc += S.llen[i] + S.mlen[i];
+#pragma unroll
+                for (int w = 0; w < THREADS / 32; w++) wbase += w < warp ? S.wsum[w] : 0;
+                const int excl = wbase + incl - (part | (num << 20));
+                int acc = excl & 0xFFFFF, i = excl >> 20;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    if (k < num) {
+                        S.ostart[i] = acc;
+                        S.llen[i] = (uint16_t)f_lit[k];
+                        S.mlen[i] = f_ml[k];
+                        S.lpos[i] = (uint16_t)f_lp[k];
+                        S.off[i] = (uint16_t)f_off[k];
+                        const int ms = op + acc + f_lit[k];             // absolute match start
+                        if (f_ml[k] > 0 && (f_off[k] == 0 || f_off[k] > ms)) S.scal[2] = 1;
+                        acc += f_lit[k] + f_ml[k];
+                        i++;
+                    }
                 }
-                if (tid == THREADS - 1) S.ostart[nseq] = acc;      // nseq <= MAXS: the last thread holds the total
+                if (tid == THREADS - 1) {                          // the last thread holds the totals
+                    S.ostart[i] = acc;
+                    S.scal[7] = i;
+                }
                 __syncthreads();
-                const int total = S.ostart[nseq];
+                const int nseq = S.scal[7], total = S.ostart[nseq];
+                walk = nseq <= WALK_MAX;
                 if (S.scal[2] || total > osz - op) { bad = true; break; }
                 // output in groups of at most DCAP bytes
                 int a = 0;
@@ -407,66 +460,68 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
                     const int b = lo;
                     if (S.ostart[b] - base <= DCAP) {
                         const int span = S.ostart[b] - base;
-                        // a match byte's source, relative to the group (>= 0: a pointer into st),
-                        // or its value when it precedes the group (the ring, else global memory)
-                        auto src_entry = [&](int src) -> uint32_t {
-                            if (src >= 0) return (uint32_t)src;
-                            const int abs = op + base + src;
-                            return RES | (abs >= hist_from ? (uint32_t)S.hist[abs & (HB - 1)] : (uint32_t)__ldcg(out + abs));
+                        // Bytes first, first + step, ... of sequence i: literal bytes as values,
+                        // match bytes as their sources' places (match byte k's at m0 - d + (k mod d):
+                        // below the match start even when the match overlaps itself).
+                        auto fill = [&](int i, int first, int step) {
+                            const int s0 = S.ostart[i] - base, lit = S.llen[i], ml = S.mlen[i];
+                            const uint8_t *lp = win + S.lpos[i];
+                            for (int x = first; x < lit; x += step) S.st[s0 + x] = RES | lp[x];
+                            const int d = S.off[i];
+                            uint32_t *st = S.st + s0 + lit;
+                            const uint32_t src = BIAS + (uint32_t)(s0 + lit - d);
+                            if (ml <= d) {
+                                for (int k = first; k < ml; k += step) st[k] = src + k;
+                            } else {
+                                const int inc = step < d ? step : step % d;
+                                for (int k = first, km = first < d ? first : first % d; k < ml; k += step) {
+                                    st[k] = src + km;
+                                    km += inc;
+                                    if (km >= d) km -= d;
+                                }
+                            }
                         };
-                        // Sequence-parallel fill: a thread writes whole sequences (match byte k at
-                        // m0 + k takes its source at m0 - d + (k mod d): below the match start even
-                        // when the match overlaps itself); sequences longer than LONGSEQ bytes are
-                        // listed and filled by the whole CTA after.
                         for (int i = a + tid; i < b; i += THREADS) {
-                            const int s0 = S.ostart[i] - base, lit = S.llen[i], ml = S.mlen[i];
-                            if (lit + ml > LONGSEQ) {
-                                S.longs[atomicAdd(&S.nlong, 1)] = i;
-                                continue;
-                            }
-                            const int lp = S.lpos[i], d = S.off[i], m0 = s0 + lit;
-                            for (int r = 0; r < lit; r++) S.st[s0 + r] = RES | S.win[lp + r];
-                            int km = 0;                                  // k mod d
-                            for (int k = 0; k < ml; k++) {
-                                S.st[m0 + k] = src_entry(m0 - d + km);
-                                if (++km == d) km = 0;
-                            }
+                            const int len = S.llen[i] + S.mlen[i];
+                            if (len <= LONGSEQ) fill(i, 0, 1);
+                            else if (len <= VLONG) S.longs[atomicAdd(&S.nlong, 1)] = (uint16_t)i;
+                            else S.vlongs[atomicAdd(&S.nvlong, 1)] = (uint16_t)i;
                         }
                         __syncthreads();
-                        const int nlong = S.nlong;
-                        for (int j = 0; j < nlong; j++) {
-                            const int i = S.longs[j];
-                            const int s0 = S.ostart[i] - base, lit = S.llen[i], ml = S.mlen[i];
-                            const int lp = S.lpos[i], d = S.off[i], m0 = s0 + lit;
-                            for (int x = tid; x < lit + ml; x += THREADS)
-                                S.st[s0 + x] = x < lit ? RES | S.win[lp + x] : src_entry(m0 - d + (x - lit) % d);
-                        }
+                        const int nlong = S.nlong, nvlong = S.nvlong;
+                        for (int j = tid / GROUP; j < nlong; j += THREADS / GROUP) fill(S.longs[j], tid % GROUP, GROUP);
+                        for (int j = 0; j < nvlong; j++) fill(S.vlongs[j], tid, THREADS);
                         __syncthreads();
-                        if (tid == 0) S.nlong = 0;                     // read above, before the barrier
-                        for (;;) {                                 // pointer jumping
+                        if (tid == 0) S.nlong = S.nvlong = 0;          // read above, before the barrier
+                        uint8_t *o = out + op + base;
+                        // sources before the group: the ring, as far as this group's bytes do not
+                        // replace it, else the written output
+                        const int hist_lo = max(hist_from, op + base + span - HB);
+                        for (;;) {                                 // follow the sources, write
                             int open = 0;
                             for (int x = tid; x < span; x += THREADS) {
-                                const uint32_t v = S.st[x];
-                                if (!(v & RES)) {
-                                    const uint32_t t = S.st[v];
-                                    S.st[x] = t;
-                                    open |= !(t & RES);
+                                uint32_t v = S.st[x];
+                                for (int h = 0; h < HOPS && v - BIAS < (uint32_t)DCAP; h++) v = S.st[v - BIAS];
+                                if (v < BIAS) {
+                                    const int abs = op + base + (int)v - (int)BIAS;
+                                    v = RES | (abs >= hist_lo ? (uint32_t)S.hist[abs & (HB - 1)] : (uint32_t)__ldcg(out + abs));
+                                }
+                                S.st[x] = v;
+                                if (v & RES) {
+                                    o[x] = (uint8_t)v;
+                                    S.hist[(op + base + x) & (HB - 1)] = (uint8_t)v;
+                                } else {
+                                    open = 1;
                                 }
                             }
                             if (!__syncthreads_or(open)) break;
-                        }
-                        uint8_t *o = out + op + base;
-                        for (int x = tid; x < span; x += THREADS) {
-                            const uint8_t byte = (uint8_t)S.st[x];
-                            o[x] = byte;
-                            S.hist[(op + base + x) & (HB - 1)] = byte;
                         }
                         hist_from = max(hist_from, op + base + span - HB);
                         a = b;
                     } else {
                         // one sequence larger than DCAP: literals, then the match from global memory
                         const int abs0 = op + base, lit = S.llen[a], ml = S.mlen[a], d = S.off[a];
-                        for (int x = tid; x < lit; x += THREADS) out[abs0 + x] = S.win[S.lpos[a] + x];
+                        for (int x = tid; x < lit; x += THREADS) out[abs0 + x] = win[S.lpos[a] + x];
                         __syncthreads();
                         const int m0 = abs0 + lit;
                         for (int x = tid; x < ml; x += THREADS) out[m0 + x] = __ldcg(out + m0 - d + (d > x ? x : x % d));
@@ -477,7 +532,7 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
                 }
                 op += total;
                 if (term == ENDS) { done = true; break; }
-                p += term == STOP ? S.path[cnt - 1] : n;
+                p = pnext;
                 continue;
             }
             // the sequence at p does not fit in a window: decode it alone, header from global
@@ -531,6 +586,7 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
                 op += lit + ml;
                 hist_from = op;                            // the ring missed this sequence
                 if (nr < 0) done = true; else p = nr;
+                if (!done) pre = fetch(in, p, isz);
             }
         }
         if (!bad && op != osz) bad = true;
