@@ -638,12 +638,10 @@ __device__ __forceinline__ bool item_pos(const Geom &g, int64_t c, int64_t b, in
     return row < g.shape[0] && col < g.shape[1];
 }
 
-// Partitions whose block rows hold whole groups of 4 items of 4 or 8 bytes take the
-// word-level fast paths below, edge blocks included.
-__device__ __forceinline__ bool geom_fast(const Geom &g)
-{
-    return !(g.block[1] & 3) && (g.itemsize == 4 || g.itemsize == 8);
-}
+// Partitions with items of 4 or 8 bytes take the fast paths below, edge blocks included:
+// where block rows hold whole groups of 4 items, 4 items and a word of each plane at a time,
+// else item by item.
+__device__ __forceinline__ bool geom_quads(const Geom &g) { return !(g.block[1] & 3); }
 
 // Block b of chunk c: its first logical row and column, and how many of its rows (nr) and
 // columns (nc) hold logical items (the rest is chunk or array padding; 0 when none do).
@@ -678,14 +676,16 @@ __device__ __forceinline__ BlockSpan block_span(const Geom &g, int64_t c, int64_
     return s;
 }
 
-// D2 fast path: shuffled, split blocks of partitions whose block rows hold whole groups of 4
-// items, in slices of SC_ITEMS items (one CTA per slice at a time).  One thread stages the
-// slice's bytes of every byte plane (read in place from raw streams or the LZ4 scratch) into
-// shared memory with bulk asynchronous copies completing on an mbarrier; then each thread
-// rebuilds 4 consecutive items from one 4-byte word per plane and writes the logical ones to
-// the dense row (edge blocks: the items in chunk or array padding are not written; slices of
-// padding only are skipped).  Every other block is appended to the list `rest` for the
-// general path.
+// D2 fast path: shuffled, split blocks of 4- and 8-byte items, in slices of SC_ITEMS items
+// (one CTA per slice at a time).  One thread stages the slice's bytes of every byte plane (read
+// in place from raw streams or the LZ4 scratch) into shared memory with bulk asynchronous
+// copies completing on an mbarrier; then each thread rebuilds items and writes the logical ones
+// to the dense row (edge blocks: the items in chunk or array padding are not written; slices of
+// padding only are skipped): 4 consecutive items from one 4-byte word per plane where block rows
+// hold whole groups of 4, else one item from a byte per plane, consecutive lanes taking
+// consecutive items (4000 x 6000 float64 in blocks of 100 x 150: 0.12 ms, 0.79 by the general
+// path's bytewise tiles).  Every other block is
+// appended to the list `rest` for the general path.
 constexpr int SC_ITEMS = 4096;
 constexpr int SC_PLANE = SC_ITEMS + 32;            // a slice of a plane from its 16-byte boundary
 constexpr uint32_t SC_WAIT_POLLS = 1u << 22;
@@ -714,17 +714,17 @@ __device__ __forceinline__ bool scatter_fast_unit(const Geom &g, const uint8_t *
                                                   uint64_t *bar, uint32_t &parity, int *abort_all)
 {
     const int tid = threadIdx.x;
-    const int qpr = (int)(g.block[1] / 4);
+    const int rowlen = (int)g.block[1];
     int64_t c, b;
     divmod(t, g.nblocks, c, b);
     const BlockDesc d = bd[t];
-    if (d.mode != BM_SHUFFLED || d.nstreams != TS || !geom_fast(g)) {
+    if (d.mode != BM_SHUFFLED || d.nstreams != TS) {
         if (tid == 0 && sl == 0) rest[atomicAdd(nrest, 1)] = rest_id;   // left to k_scatter
         return true;
     }
     const BlockSpan sp = block_span(g, c, b);
     const int i0s = sl * SC_ITEMS, cnt = (int)min((int64_t)SC_ITEMS, g.blockn - i0s);
-    if (sp.nc == 0 || i0s / (qpr * 4) >= sp.nr) return true;          // the slice holds only padding
+    if (sp.nc == 0 || i0s / rowlen >= sp.nr) return true;             // the slice holds only padding
     // per plane: its slice starts at src, 16-byte word a16 = src - shift; the bulk copy
     // takes the whole words of [a16, a16 + want) before the buffer end lim, threads copy
     // the bytes that the buffer end cuts off (zeros past it)
@@ -785,9 +785,32 @@ __device__ __forceinline__ bool scatter_fast_unit(const Geom &g, const uint8_t *
     }
     uint8_t *const obase = out + (sp.row0 * ld + sp.col0) * TS;
     const int nr = sp.nr, nc = sp.nc;
+    if (!geom_quads(g)) {
+        const int step = (int)blockDim.x, step_r = step / rowlen, step_c = step - step_r * rowlen;
+        int r = (i0s + tid) / rowlen, cc = i0s + tid - r * rowlen;
+        for (int i = tid; i < cnt; i += step, r += step_r, cc += step_c) {
+            if (cc >= rowlen) { cc -= rowlen; r++; }
+            if (r >= nr || cc >= nc) continue;                            // padding items
+            uint32_t v[TS / 4];
+#pragma unroll
+            for (int w = 0; w < TS / 4; w++) {
+                v[w] = 0;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int k = w * 4 + j;
+                    v[w] |= (code[k] >= 256 ? (uint32_t)(code[k] - 256) : (uint32_t)stage[k][code[k] + i]) << (8 * j);
+                }
+            }
+            uint8_t *o = obase + ((int64_t)r * ld + cc) * TS;
+            if constexpr (TS == 8) *reinterpret_cast<uint2 *>(o) = make_uint2(v[0], v[1]);
+            else *reinterpret_cast<uint32_t *>(o) = v[0];
+        }
+        __syncthreads();                           // stage is read before the next slice's copies
+        return true;
+    }
     // (row, column) of each thread's quad, advanced by a fixed step per iteration (one
     // division per slice instead of one per quad)
-    const int rowlen = qpr * 4, step = (int)blockDim.x * 4;
+    const int step = (int)blockDim.x * 4;
     const int step_r = step / rowlen, step_c = step - step_r * rowlen;
     int r = (i0s + tid * 4) / rowlen, cc = i0s + tid * 4 - r * rowlen;
     for (int qd = tid; qd < cnt / 4; qd += blockDim.x, r += step_r, cc += step_c) {
@@ -944,23 +967,41 @@ __global__ void __launch_bounds__(256) k_scatter(Geom g, const int *__restrict__
 }
 
 // ============================================================================ encode
-// E1 fast path: shuffle on, block rows of whole groups of 4 items; each thread reads 4
-// consecutive items of a block row (zero for the items in chunk or array padding) and
-// writes one 4-byte word into each byte plane of the image.
+// E1 fast path: shuffle on, items of 4 or 8 bytes (zero for the items in chunk or array
+// padding).  Block rows of whole groups of 4 items: each thread reads 4 consecutive items of a
+// row and writes one 4-byte word into each byte plane of the image.  Other blocks, whose planes
+// may start at any byte: one item per thread, a byte into each plane, the bytes of a warp
+// next to each other (5000 x 6000 float32 in blocks of 125 x 150: 0.13 ms, 0.29 by the
+// general path).  In slices of SC_ITEMS items, so that a few large blocks spread over the SMs.
 template <int TS>
 __device__ __forceinline__ void gather_fast_block(const Geom &g, const uint8_t *__restrict__ in, int64_t ld,
-                                                  uint8_t *__restrict__ img, int64_t t)
+                                                  uint8_t *__restrict__ img, int64_t t, int sl)
 {
-    if (!geom_fast(g)) return;
-    const int qpr = (int)(g.block[1] / 4), nq = (int)(g.blockn / 4);
+    const int i0s = sl * SC_ITEMS, cnt = (int)min((int64_t)SC_ITEMS, g.blockn - i0s);
     int64_t c, b;
     divmod(t, g.nblocks, c, b);
     const BlockSpan sp = block_span(g, c, b);
     uint8_t *blk = img + t * g.blocksize;
+    if (!geom_quads(g)) {
+        const int rowlen = (int)g.block[1], step = (int)blockDim.x, step_r = step / rowlen, step_c = step - step_r * rowlen;
+        int r = (i0s + (int)threadIdx.x) / rowlen, cc = i0s + (int)threadIdx.x - r * rowlen;
+        for (int i = i0s + threadIdx.x; i < i0s + cnt; i += step, r += step_r, cc += step_c) {
+            if (cc >= rowlen) { cc -= rowlen; r++; }
+            uint64_t x = 0;
+            if (r < sp.nr && cc < sp.nc) {
+                const uint8_t *src = in + ((sp.row0 + r) * ld + sp.col0 + cc) * TS;
+                x = TS == 8 ? __ldg(reinterpret_cast<const uint64_t *>(src)) : __ldg(reinterpret_cast<const uint32_t *>(src));
+            }
+#pragma unroll
+            for (int j = 0; j < TS; j++) blk[(int64_t)j * g.blockn + i] = (uint8_t)(x >> (8 * j));
+        }
+        return;
+    }
+    const int qpr = (int)(g.block[1] / 4), q0 = i0s / 4, nq = cnt / 4;
     // (row, quad column) of each thread's quad, advanced by a fixed step per iteration
     const int step_r = (int)blockDim.x / qpr, step_q = (int)blockDim.x - step_r * qpr;
-    int r = (int)threadIdx.x / qpr, q = (int)threadIdx.x - r * qpr;
-    for (int qd = threadIdx.x; qd < nq; qd += blockDim.x, r += step_r, q += step_q) {
+    int r = (q0 + (int)threadIdx.x) / qpr, q = q0 + (int)threadIdx.x - r * qpr;
+    for (int qd = q0 + threadIdx.x; qd < q0 + nq; qd += blockDim.x, r += step_r, q += step_q) {
         if (q >= qpr) { q -= qpr; r++; }
         const int i0 = qd * 4, cc = q * 4;
         const uint8_t *src = in + ((sp.row0 + r) * ld + sp.col0 + cc) * TS;
@@ -995,13 +1036,16 @@ template <int TS>
 __global__ void __launch_bounds__(256) k_gather_fast(Geom g, const uint8_t *__restrict__ in, int64_t ld,
                                                      uint8_t *__restrict__ img)
 {
-    const int64_t nbl = g.nchunks * g.nblocks;
-    for (int64_t t = blockIdx.x; t < nbl; t += gridDim.x) gather_fast_block<TS>(g, in, ld, img, t);
+    const int64_t nsl = (g.blockn + SC_ITEMS - 1) / SC_ITEMS, nu = g.nchunks * g.nblocks * nsl;
+    for (int64_t u = blockIdx.x; u < nu; u += gridDim.x) {
+        int64_t t, sl;
+        divmod(u, nsl, t, sl);
+        gather_fast_block<TS>(g, in, ld, img, t, (int)sl);
+    }
 }
 
 // E1 general path: dense -> byte-plane image (shuffled: plane j holds byte j of every
-// item; plain: items back to back).  Padding items are zero, as in Caterva.  With
-// skip_fast, nothing is done for partitions the fast path handles.
+// item; plain: items back to back).  Padding items are zero, as in Caterva.
 __device__ __forceinline__ void gather_tile(const Geom &g, const uint8_t *__restrict__ in, int64_t ld, bool shuffle,
                                             uint8_t *__restrict__ img, int64_t t, int64_t i0, uint8_t *planes)
 {
@@ -1032,7 +1076,7 @@ __device__ __forceinline__ void gather_tile(const Geom &g, const uint8_t *__rest
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) k_gather(Geom g, bool skip_fast, const uint8_t *__restrict__ in, int64_t ld,
+__global__ void __launch_bounds__(256) k_gather(Geom g, const uint8_t *__restrict__ in, int64_t ld,
                                                 bool shuffle, uint8_t *__restrict__ img)
 {
     __shared__ __align__(16) uint8_t planes[8 * TILE];
@@ -1040,7 +1084,6 @@ __global__ void __launch_bounds__(256) k_gather(Geom g, bool skip_fast, const ui
     const int64_t nwork = g.nchunks * g.nblocks * tpb;
     for (int64_t w = blockIdx.x; w < nwork; w += gridDim.x) {
         const int64_t t = w / tpb, i0 = (w - t * tpb) * TILE;
-        if (skip_fast && geom_fast(g)) continue;
         gather_tile(g, in, ld, shuffle, img, t, i0, planes);
     }
 }
@@ -2496,19 +2539,17 @@ int encode_gather(const Geom &g, const void *in, int64_t ld, bool shuffle, int s
     const int64_t blocks = std::min<int64_t>(nbl * tpb, (int64_t)sms * 8);
     const bool fast = shuffle && (ts == 4 || ts == 8);
     if (fast) {
-        const int64_t fb = std::min<int64_t>(nbl, (int64_t)sms * 8);
+        const int64_t fb = std::min<int64_t>(nbl * ceil_div(g.blockn, SC_ITEMS), (int64_t)sms * 8);
         if (ts == 8)
             IAB_TIMED("k_gather_fast", st, k_gather_fast<8><<<(unsigned)std::max<int64_t>(fb, 1), 256, 0, st>>>(
                 g, (const uint8_t *)in, ld, img));
         else
             IAB_TIMED("k_gather_fast", st, k_gather_fast<4><<<(unsigned)std::max<int64_t>(fb, 1), 256, 0, st>>>(
                 g, (const uint8_t *)in, ld, img));
-    }
-    // the general gather covers the partitions the fast one does not take
-    const bool all_fast = fast && !(g.block[1] & 3);
-    if (!all_fast)
+    } else {
         IAB_TIMED("k_gather", st, k_gather<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
-            g, fast, (const uint8_t *)in, ld, shuffle, img));
+            g, (const uint8_t *)in, ld, shuffle, img));
+    }
     return 0;
 }
 
@@ -2995,17 +3036,19 @@ __global__ void __launch_bounds__(256) k_scatter_g(const CodecItem *__restrict__
 
 template <int TS>
 __global__ void __launch_bounds__(256) k_gather_fast_g(const CodecItem *__restrict__ items,
-                                                       const int64_t *__restrict__ bstart, int n, int64_t nbl)
+                                                       const int64_t *__restrict__ sstart, int n, int64_t nsf)
 {
-    for (int64_t u = blockIdx.x; u < nbl; u += gridDim.x) {
-        const int k = group_find(bstart, n, u);
+    for (int64_t u = blockIdx.x; u < nsf; u += gridDim.x) {
+        const int k = group_find(sstart, n, u);
         const CodecItem &it = items[k];
-        gather_fast_block<TS>(it.g, it.dense, it.ld, it.img, u - bstart[k]);
+        int64_t t, sl;
+        divmod(u - sstart[k], (it.g.blockn + SC_ITEMS - 1) / SC_ITEMS, t, sl);
+        gather_fast_block<TS>(it.g, it.dense, it.ld, it.img, t, (int)sl);
     }
 }
 
 __global__ void __launch_bounds__(256) k_gather_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart,
-                                                  int n, int64_t nbl, int64_t tpb, bool skip_fast, bool shuffle)
+                                                  int n, int64_t nbl, int64_t tpb, bool shuffle)
 {
     __shared__ __align__(16) uint8_t planes[8 * TILE];
     for (int64_t w = blockIdx.x; w < nbl * tpb; w += gridDim.x) {
@@ -3013,7 +3056,6 @@ __global__ void __launch_bounds__(256) k_gather_g(const CodecItem *__restrict__ 
         const int k = group_find(bstart, n, gb);
         const CodecItem &it = items[k];
         if (i0 >= it.g.blockn) continue;
-        if (skip_fast && geom_fast(it.g)) continue;
         gather_tile(it.g, it.dense, it.ld, shuffle, it.img, gb - bstart[k], i0, planes);
     }
 }
@@ -3215,22 +3257,17 @@ int encode_group_launch(CodecGroup *grp, bool exact_lz4, bool memcpy_only, cudaS
     if (grp->nbl == 0) return 0;
     cudaMemsetAsync(grp->counters.p, 0, 128, st);
     const bool fast = grp->shuffle && (ts == 4 || ts == 8);
-    bool all_fast = fast;
-    for (const CodecItem &it : grp->h) {
-        const Geom &g = it.g;
-        all_fast = all_fast && !(g.block[1] & 3);
-    }
     const int64_t gb = std::max<int64_t>(std::min<int64_t>(grp->nbl, (int64_t)sms * 8), 1);
     if (fast && !grp->img_ready) {
+        const int64_t fb = std::max<int64_t>(std::min<int64_t>(grp->nsf, (int64_t)sms * 8), 1), *sstart = bstart + (n + 1);
         if (ts == 8)
-            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<8><<<(unsigned)gb, 256, 0, st>>>(items, bstart, n, grp->nbl));
+            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<8><<<(unsigned)fb, 256, 0, st>>>(items, sstart, n, grp->nsf));
         else
-            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<4><<<(unsigned)gb, 256, 0, st>>>(items, bstart, n, grp->nbl));
+            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<4><<<(unsigned)fb, 256, 0, st>>>(items, sstart, n, grp->nsf));
     }
-    if (!all_fast && !grp->img_ready) {
+    if (!fast && !grp->img_ready) {
         const int64_t tb = std::max<int64_t>(std::min<int64_t>(grp->nbl * grp->max_tpb, (int64_t)sms * 8), 1);
-        IAB_TIMED("k_gather", st, k_gather_g<<<(unsigned)tb, 256, 0, st>>>(items, bstart, n, grp->nbl, grp->max_tpb, fast,
-                                                                           grp->shuffle));
+        IAB_TIMED("k_gather", st, k_gather_g<<<(unsigned)tb, 256, 0, st>>>(items, bstart, n, grp->nbl, grp->max_tpb, grp->shuffle));
     }
     if (!memcpy_only)
         encode_streams(grp->img.as<uint8_t>(), grp->nbl * grp->nstreams, grp->nstreams, grp->neblock, grp->slots.as<uint8_t>(),
