@@ -22,6 +22,18 @@
 
 namespace iab {
 
+static int multiprocessors()
+{
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 148;
+    }
+    return n;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -318,111 +330,166 @@ void gemm_f64_grouped(int cfg, const GemmProblem *d_probs, int nprob, int total_
 }
 
 // ============================================================================ FP32 FFMA
+// BM x BN tile of C per CTA of 128 threads, BM/8 x BN/16 outputs per thread, rows in pairs:
+// fma.rn.f32x2 multiplies a pair of A values (neighbours in shared memory) with one B value in
+// both halves, two IEEE fused multiply-adds per issue slot.  Each output sums in k order, so the
+// result is the same for every tile shape.  The FP32 pipe takes a pair instruction every other
+// cycle; the slots between carry the fragment loads (a warp covers 4 x 8 threads, so an A load
+// touches 64 contiguous bytes and a B load 128) and the copies of B into both halves.  A goes
+// through registers into a k-major tile (its rows run along k), B by cp.async.
 namespace f32k {
-constexpr int BM = 128, BN = 128, BK = 8;
+constexpr int BK = 16, THREADS = 128;
+template <int BM, int BN> struct Cfg {
+    static constexpr int SA = BM + 4;                       // k-major A row
+    static constexpr int RP = BM / 16, NC = BN / 16;        // row pairs and columns per thread
+    static constexpr int AV = BM * BK / 4 / THREADS, BV = BN * BK / 4 / THREADS;
+};
+}
+
+__device__ __forceinline__ void ffma2(uint64_t &d, uint64_t a, uint64_t b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t both(float x)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
 }
 
 // Requires lda, ldb multiples of 4 and 16-byte aligned bases.
-__global__ void __launch_bounds__(256) k_gemm_f32(int M, int N, int K, const float *__restrict__ A, int64_t lda,
-                                                  const float *__restrict__ B, int64_t ldb, float *__restrict__ C,
-                                                  int64_t ldc)
+template <int BM, int BN>
+__global__ void __launch_bounds__(f32k::THREADS, 2) k_gemm_f32(int M, int N, int K, const float *__restrict__ A,
+                                                             int64_t lda, const float *__restrict__ B, int64_t ldb,
+                                                             float *__restrict__ C, int64_t ldc)
 {
     using namespace f32k;
-    __shared__ __align__(16) float sA[2][BK][BM + 4];
+    using G = Cfg<BM, BN>;
+    __shared__ __align__(16) float sA[2][BK][G::SA];
     __shared__ __align__(16) float sB[2][BK][BN];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;   // 16 x 16 threads, 8x8 each
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ty = (warp >> 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);   // 8 x 16 threads
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[8][8];
+    uint64_t acc[G::RP][G::NC];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < G::RP; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-    // A loads: 128 rows x 8 k = 256 float4 (row r, k-quad); stored transposed
-    const int ar = tid >> 1, ak = (tid & 1) * 4;
-    // B loads: 8 rows x 128 = 256 float4
-    const int br = tid >> 5, bc = (tid & 31) * 4;
+        for (int j = 0; j < G::NC; j++) acc[i][j] = 0;
     const int ktiles = (K + BK - 1) / BK;
-    float4 ra, rb;
-    auto gload = [&](int kt) {
-        const int k0 = kt * BK;
-        const int gr = m0 + ar, gk = k0 + ak;
-        ra = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gr < M) {
-            const float *p = A + (int64_t)gr * lda + gk;
-            if (gk + 3 < K) ra = *reinterpret_cast<const float4 *>(p);
-            else {
-                if (gk < K) ra.x = p[0];
-                if (gk + 1 < K) ra.y = p[1];
-                if (gk + 2 < K) ra.z = p[2];
-            }
-        }
-        const int gk2 = k0 + br, gn = n0 + bc;
-        rb = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gk2 < K) {
-            const float *p = B + (int64_t)gk2 * ldb + gn;
-            if (gn + 3 < N) rb = *reinterpret_cast<const float4 *>(p);
-            else {
-                if (gn < N) rb.x = p[0];
-                if (gn + 1 < N) rb.y = p[1];
-                if (gn + 2 < N) rb.z = p[2];
+    float4 ra[G::AV];
+    auto load_a = [&](int kt) {                             // row tid / 4 + 32 i, k tid % 4 * 4
+        const int gk = kt * BK + (tid & 3) * 4;
+#pragma unroll
+        for (int i = 0; i < G::AV; i++) {
+            const int gr = m0 + (tid >> 2) + i * 32;
+            ra[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (gr < M) {
+                const float *p = A + (int64_t)gr * lda + gk;
+                if (gk + 3 < K) ra[i] = *reinterpret_cast<const float4 *>(p);
+                else {
+                    if (gk < K) ra[i].x = p[0];
+                    if (gk + 1 < K) ra[i].y = p[1];
+                    if (gk + 2 < K) ra[i].z = p[2];
+                }
             }
         }
     };
-    auto sstore = [&](int s) {
-        sA[s][ak + 0][ar] = ra.x; sA[s][ak + 1][ar] = ra.y; sA[s][ak + 2][ar] = ra.z; sA[s][ak + 3][ar] = ra.w;
-        *reinterpret_cast<float4 *>(&sB[s][br][bc]) = rb;
+    auto store_a = [&](int s) {
+        const int k = (tid & 3) * 4;
+#pragma unroll
+        for (int i = 0; i < G::AV; i++) {
+            const int r = (tid >> 2) + i * 32;
+            sA[s][k][r] = ra[i].x; sA[s][k + 1][r] = ra[i].y; sA[s][k + 2][r] = ra[i].z; sA[s][k + 3][r] = ra[i].w;
+        }
     };
-    gload(0);
-    sstore(0);
+    auto load_b = [&](int kt, int s) {
+#pragma unroll
+        for (int i = 0; i < G::BV; i++) {
+            const int idx = tid + i * THREADS, r = idx / (BN / 4), c = (idx % (BN / 4)) * 4;
+            const int gk = kt * BK + r, gn = n0 + c;
+            const int nb = gk < K ? 4 * max(0, min(4, N - gn)) : 0;
+            cp_async16(&sB[s][r][c], nb ? (const void *)(B + (int64_t)gk * ldb + gn) : (const void *)B, nb);
+        }
+        cp_async_commit();
+    };
+    load_a(0);
+    load_b(0, 0);
+    store_a(0);
+    cp_async_wait<0>();
     __syncthreads();
     for (int kt = 0; kt < ktiles; kt++) {
         const int s = kt & 1;
-        if (kt + 1 < ktiles) gload(kt + 1);
-#pragma unroll
-        for (int k = 0; k < BK; k++) {
-            float a[8], b[8];
-            const float4 a0 = *reinterpret_cast<const float4 *>(&sA[s][k][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&sA[s][k][64 + ty * 4]);
-            const float4 b0 = *reinterpret_cast<const float4 *>(&sB[s][k][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4 *>(&sB[s][k][64 + tx * 4]);
-            a[0] = a0.x; a[1] = a0.y; a[2] = a0.z; a[3] = a0.w; a[4] = a1.x; a[5] = a1.y; a[6] = a1.z; a[7] = a1.w;
-            b[0] = b0.x; b[1] = b0.y; b[2] = b0.z; b[3] = b0.w; b[4] = b1.x; b[5] = b1.y; b[6] = b1.z; b[7] = b1.w;
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-#pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        const bool more = kt + 1 < ktiles;
+        if (more) {
+            load_a(kt + 1);
+            load_b(kt + 1, s ^ 1);
         }
-        if (kt + 1 < ktiles) {
-            sstore(s ^ 1);
+#pragma unroll
+        for (int half = 0; half < BK; half += 8) {          // k past the last whole group of 8 adds nothing
+            if (kt * BK + half >= K) break;
+#pragma unroll
+            for (int k = half; k < half + 8; k++) {
+                uint64_t a[G::RP], b[G::NC];
+#pragma unroll
+                for (int q = 0; q < G::RP / 2; q++) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(&sA[s][k][q * 32 + ty * 4]);
+                    a[2 * q] = v.x;
+                    a[2 * q + 1] = v.y;
+                }
+#pragma unroll
+                for (int h = 0; h < G::NC / 4; h++) {
+                    const float4 v = *reinterpret_cast<const float4 *>(&sB[s][k][h * 64 + tx * 4]);
+                    b[4 * h] = both(v.x); b[4 * h + 1] = both(v.y); b[4 * h + 2] = both(v.z); b[4 * h + 3] = both(v.w);
+                }
+#pragma unroll
+                for (int i = 0; i < G::RP; i++)
+#pragma unroll
+                    for (int j = 0; j < G::NC; j++) ffma2(acc[i][j], a[i], b[j]);
+            }
         }
+        if (more) store_a(s ^ 1);
+        cp_async_wait<0>();
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int r = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
+    for (int i = 0; i < 2 * G::RP; i++) {
+        const int r = m0 + (i >> 2) * 32 + ty * 4 + (i & 3);
         if (r >= M) continue;
+        float v[G::NC];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
+        for (int j = 0; j < G::NC; j++) v[j] = __uint_as_float((uint32_t)(acc[i >> 1][j] >> (32 * (i & 1))));
+#pragma unroll
+        for (int h = 0; h < G::NC / 4; h++) {
             const int c = n0 + h * 64 + tx * 4;
             float *cp = C + (int64_t)r * ldc + c;
-            const float v0 = acc[i][h * 4 + 0], v1 = acc[i][h * 4 + 1], v2 = acc[i][h * 4 + 2], v3 = acc[i][h * 4 + 3];
-            if (c + 3 < N) *reinterpret_cast<float4 *>(cp) = make_float4(v0, v1, v2, v3);
+            if (c + 3 < N) *reinterpret_cast<float4 *>(cp) = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
             else {
-                if (c < N) cp[0] = v0;
-                if (c + 1 < N) cp[1] = v1;
-                if (c + 2 < N) cp[2] = v2;
+                if (c < N) cp[0] = v[4 * h];
+                if (c + 1 < N) cp[1] = v[4 * h + 1];
+                if (c + 2 < N) cp[2] = v[4 * h + 2];
             }
         }
     }
 }
 
+template <int BM, int BN>
+static void launch_f32(int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C,
+                       int64_t ldc, cudaStream_t st)
+{
+    dim3 grid((unsigned)ceil_div(N, BN), (unsigned)ceil_div(M, BM));
+    IAB_TIMED("k_gemm_f32", st, k_gemm_f32<BM, BN><<<grid, f32k::THREADS, 0, st>>>((int)M, (int)N, (int)K, A, lda, B, ldb, C, ldc));
+}
+
+// The time of a launch is about the tiles of the busiest SM times a tile's area; the 64 x 64
+// tile loads twice the fragments per multiply-add.
 void gemm_f32_native(int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
                      float *C, int64_t ldc, cudaStream_t st)
 {
-    using namespace f32k;
-    dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM));
-    IAB_TIMED("k_gemm_f32", st, k_gemm_f32<<<grid, 256, 0, st>>>((int)M, (int)N, (int)K, A, lda, B, ldb, C, ldc));
+    const int64_t sms = multiprocessors();
+    const int64_t big = ceil_div(ceil_div(M, 128) * ceil_div(N, 128), sms) * 128 * 128;
+    const int64_t small = ceil_div(ceil_div(M, 64) * ceil_div(N, 64), sms) * 64 * 64;
+    if (small * 14 < big * 10) launch_f32<64, 64>(M, N, K, A, lda, B, ldb, C, ldc, st);
+    else launch_f32<128, 128>(M, N, K, A, lda, B, ldb, C, ldc, st);
 }
 
 // ============================================================================ GEMV
