@@ -8,9 +8,9 @@
 // (sum over K blocks of A_blk * B_blk == the dense product over the padded extents,
 // because Caterva's padding is zero).
 //
-// FP64: DMMA tensor-core tiles (mma.sync m16n8k16 .f64), 128x128x32 CTA tile,
-//       8 warps (64x32 each), 3-stage cp.async pipeline with zero-filled edges.
-// FP32: FFMA SIMT tiles, 128x128x8, 8x8 outer product per thread, double buffer.
+// FP64: DMMA tensor-core tiles (mma.sync m16n8k16 .f64), 64x64x32 or 32x32x32 CTA tile,
+//       8 warps, 3-stage cp.async pipeline with zero-filled edges.
+// FP32: paired FFMA SIMT tiles, 128x128x16 or 64x64x16, double buffer.
 // GEMV: one warp per row, 16-byte loads.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -60,7 +60,6 @@ template <int BM, int BN, int BK> struct Cfg {
     static constexpr int SMEM = STAGES * (A_STAGE + B_STAGE) * 8;
     static constexpr int MI = BM / 32, NJ = BN / 32;     // 2 x 4 warps, warp tile (BM/2) x (BN/4)
 };
-constexpr int BK_SINGLE = 32;
 }
 
 // D += A B for one 16x8 tile over k = 16 (a: rows g, g + 8 at columns q + 4u; b: rows q + 4u
@@ -178,33 +177,33 @@ __device__ __forceinline__ void f64_tile(int M, int N, int K, const double *__re
         }
 }
 
+template <int BM, int BN, int BK>
 __global__ void __launch_bounds__(256) k_gemm_f64(int M, int N, int K, const double *__restrict__ A, int64_t lda,
                                                   const double *__restrict__ B, int64_t ldb, double *__restrict__ C,
                                                   int64_t ldc)
 {
     extern __shared__ __align__(16) double smf64[];
-    f64_tile<128, 128, f64k::BK_SINGLE>(M, N, K, A, lda, B, ldb, C, ldc, blockIdx.y * 128, blockIdx.x * 128, smf64);
+    f64_tile<BM, BN, BK>(M, N, K, A, lda, B, ldb, C, ldc, blockIdx.y * BM, blockIdx.x * BN, smf64);
 }
 
 // The same product where the K ranges of zero-block pairs are left out: each CTA lists the
 // k-tiles its tile needs (zs_tile_active) in shared memory, compacted by warp ballots, and
 // multiplies only those.  K <= ZS_MAX_K.
 constexpr int ZS_MAX_K = 65536;
-constexpr int ZS_LIST_BYTES = (ZS_MAX_K / f64k::BK_SINGLE) * 3 + 64;    // flags + uint16 list + count
+template <int BM, int BN, int BK>
 __global__ void __launch_bounds__(256) k_gemm_f64_skip(int M, int N, int K, const double *__restrict__ A, int64_t lda,
                                                        const double *__restrict__ B, int64_t ldb, double *__restrict__ C,
                                                        int64_t ldc, ZeroSkip z)
 {
-    constexpr int BK = f64k::BK_SINGLE;
-    using G = f64k::Cfg<128, 128, BK>;
+    using G = f64k::Cfg<BM, BN, BK>;
     extern __shared__ __align__(16) double smf64[];
     uint8_t *extra = reinterpret_cast<uint8_t *>(smf64 + f64k::STAGES * (G::A_STAGE + G::B_STAGE));
     const int ktiles = (K + BK - 1) / BK;
     int *count = reinterpret_cast<int *>(extra);
     uint16_t *list = reinterpret_cast<uint16_t *>(extra + 16);
     uint8_t *flag = extra + 16 + 2 * ktiles;
-    const int m0 = blockIdx.y * 128, n0 = blockIdx.x * 128;
-    const int64_t r1 = min(m0 + 128, M), c1 = min(n0 + 128, N);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int64_t r1 = min(m0 + BM, M), c1 = min(n0 + BN, N);
     for (int kt = threadIdx.x; kt < ktiles; kt += blockDim.x)
         flag[kt] = zs_tile_active(z, m0, r1, n0, c1, (int64_t)kt * BK, min((kt + 1) * BK, K)) ? 1 : 0;
     __syncthreads();
@@ -220,28 +219,45 @@ __global__ void __launch_bounds__(256) k_gemm_f64_skip(int M, int N, int K, cons
         if (lane == 0) *count = c;
     }
     __syncthreads();
-    f64_tile<128, 128, BK>(M, N, K, A, lda, B, ldb, C, ldc, m0, n0, smf64, list, *count);
+    f64_tile<BM, BN, BK>(M, N, K, A, lda, B, ldb, C, ldc, m0, n0, smf64, list, *count);
 }
 
+template <int BM, int BN, int BK>
+static void launch_f64(int64_t M, int64_t N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
+                       int64_t ldc, cudaStream_t st, const ZeroSkip *zs)
+{
+    using G = f64k::Cfg<BM, BN, BK>;
+    constexpr int LIST = (ZS_MAX_K / BK) * 3 + 64;          // flags + uint16 list + count
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(k_gemm_f64<BM, BN, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+        cudaFuncSetAttribute(k_gemm_f64_skip<BM, BN, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM + LIST);
+        attr = true;
+    }
+    dim3 grid((unsigned)ceil_div(N, BN), (unsigned)ceil_div(M, BM));
+    if (zs && K <= ZS_MAX_K) {
+        const int smem = G::SMEM + 3 * (int)ceil_div(K, BK) + 64;
+        IAB_TIMED("k_gemm_f64", st, k_gemm_f64_skip<BM, BN, BK><<<grid, 256, smem, st>>>((int)M, (int)N, (int)K, A, lda, B, ldb,
+                                                                                       C, ldc, *zs));
+        return;
+    }
+    IAB_TIMED("k_gemm_f64", st, k_gemm_f64<BM, BN, BK><<<grid, 256, G::SMEM, st>>>((int)M, (int)N, (int)K, A, lda, B, ldb, C, ldc));
+}
+
+// Tile shape: the busiest SM's tiles times a tile's area, the 32 x 32 tile's fragments costing a
+// tenth more.  Measured (ms; 128x128x32, 64x64x32, 32x32x32 tiles): 300x200x257 0.049, 0.018,
+// 0.009; 1000^3 0.158, 0.086, 0.084; 1500x1800x1200 0.369, 0.234, 0.246; 8000x130x4000 0.596,
+// 0.466, 0.385; 4056x3712x3230 3.35, 3.06, 3.30; 5000x6000x3500 6.75, 6.52, 7.40.  (The large
+// tile reads shared memory least, but keeps one CTA per SM, whose barriers nothing covers.)
+// Every shape sums each output in the same order.
 void gemm_f64_native(int64_t M, int64_t N, int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb,
                      double *C, int64_t ldc, cudaStream_t st, const ZeroSkip *zs)
 {
-    using G = f64k::Cfg<128, 128, f64k::BK_SINGLE>;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_gemm_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-        cudaFuncSetAttribute(k_gemm_f64_skip, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM + ZS_LIST_BYTES);
-        attr = true;
-    }
-    dim3 grid((unsigned)((N + 127) / 128), (unsigned)((M + 127) / 128));
-    if (zs && K <= ZS_MAX_K) {
-        const int ktiles = (int)((K + f64k::BK_SINGLE - 1) / f64k::BK_SINGLE);
-        const int smem = G::SMEM + 3 * ktiles + 64;
-        IAB_TIMED("k_gemm_f64", st, k_gemm_f64_skip<<<grid, 256, smem, st>>>((int)M, (int)N, (int)K, A, lda, B, ldb, C,
-                                                                           ldc, *zs));
-        return;
-    }
-    IAB_TIMED("k_gemm_f64", st, k_gemm_f64<<<grid, 256, G::SMEM, st>>>((int)M, (int)N, (int)K, A, lda, B, ldb, C, ldc));
+    const int64_t sms = multiprocessors();
+    const int64_t big = ceil_div(ceil_div(M, 64) * ceil_div(N, 64), sms) * 64 * 64;
+    const int64_t small = ceil_div(ceil_div(M, 32) * ceil_div(N, 32), sms) * 32 * 32;
+    if (small * 11 < big * 10) launch_f64<32, 32, 32>(M, N, K, A, lda, B, ldb, C, ldc, st, zs);
+    else launch_f64<64, 64, 32>(M, N, K, A, lda, B, ldb, C, ldc, st, zs);
 }
 
 // Grouped form: one persistent launch over the tiles of many independent products.
@@ -480,8 +496,10 @@ static void launch_f32(int64_t M, int64_t N, int64_t K, const float *A, int64_t 
     IAB_TIMED("k_gemm_f32", st, k_gemm_f32<BM, BN><<<grid, f32k::THREADS, 0, st>>>((int)M, (int)N, (int)K, A, lda, B, ldb, C, ldc));
 }
 
-// The time of a launch is about the tiles of the busiest SM times a tile's area; the 64 x 64
-// tile loads twice the fragments per multiply-add.
+// Tile shape: the busiest SM's tiles times a tile's area; the 64 x 64 tile, which loads twice the
+// fragments per multiply-add, counted at 1.4.  Measured against 128x128x8 tiles of single FFMAs
+// (ms): 300x200x257 0.041 -> 0.016, 1000^3 0.139 -> 0.065, 5000x6000x3500 4.87 -> 3.73 (56 of the
+// pipe's nominal 74 TFLOP/s), 8192x8192x512 1.54 -> 1.19.
 void gemm_f32_native(int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
                      float *C, int64_t ldc, cudaStream_t st)
 {
