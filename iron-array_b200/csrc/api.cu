@@ -188,9 +188,10 @@ struct iarray_context_s {
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     cudaStream_t stream2 = nullptr;          // second stream (operand decode of the pipelined call)
     cudaEvent_t fork = nullptr, join = nullptr;
-    // iarray_b200_opt_gemm_cframes: copy streams, the encode stream, the chunk-table copy
+    // iarray_b200_opt_gemm_cframes: copy streams, the encode streams, the chunk-table copy
     // stream and pinned staging for chunk tables
-    cudaStream_t up = nullptr, down = nullptr, enc = nullptr, tabs = nullptr;
+    cudaStream_t up = nullptr, down = nullptr, tabs = nullptr;
+    cudaStream_t enc[4] = {nullptr, nullptr, nullptr, nullptr};
     void *pin = nullptr;
     size_t pin_n = 0;
 };
@@ -301,7 +302,7 @@ INA_API(void) iarray_context_free(iarray_context_t **ctx)
     if (c->stream2) { cudaStreamSynchronize(c->stream2); cudaStreamDestroy(c->stream2); }
     if (c->up) { cudaStreamSynchronize(c->up); cudaStreamDestroy(c->up); }
     if (c->down) { cudaStreamSynchronize(c->down); cudaStreamDestroy(c->down); }
-    if (c->enc) { cudaStreamSynchronize(c->enc); cudaStreamDestroy(c->enc); }
+    for (auto &e : c->enc) if (e) { cudaStreamSynchronize(e); cudaStreamDestroy(e); }
     if (c->tabs) { cudaStreamSynchronize(c->tabs); cudaStreamDestroy(c->tabs); }
     if (c->pin) cudaFreeHost(c->pin);
     if (c->fork) cudaEventDestroy(c->fork);
@@ -1701,9 +1702,13 @@ INA_API(ina_rc_t) iarray_b200_opt_gemm_cframes(iarray_context_t *ctx, const uint
 
     if (!ctx->up) cudaStreamCreateWithFlags(&ctx->up, cudaStreamNonBlocking);
     if (!ctx->down) cudaStreamCreateWithFlags(&ctx->down, cudaStreamNonBlocking);
-    if (!ctx->enc) cudaStreamCreateWithFlags(&ctx->enc, cudaStreamNonBlocking);
+    bool enc_ok = true;
+    for (auto &e : ctx->enc) {
+        if (!e) cudaStreamCreateWithFlags(&e, cudaStreamNonBlocking);
+        enc_ok = enc_ok && e;
+    }
     if (!ctx->tabs) cudaStreamCreateWithFlags(&ctx->tabs, cudaStreamNonBlocking);
-    if (!ctx->up || !ctx->down || !ctx->enc || !ctx->tabs || !ctx->stream2) return rc_err(IARRAY_ERR_GPU_FAILED);
+    if (!ctx->up || !ctx->down || !enc_ok || !ctx->tabs || !ctx->stream2) return rc_err(IARRAY_ERR_GPU_FAILED);
     cudaStream_t st = ctx->stream;
     const int isz = fa.g.itemsize;
     const int64_t lda = pad_ld(K), ldb = pad_ld(N), ldc = pad_ld(N);
@@ -1735,13 +1740,14 @@ INA_API(ina_rc_t) iarray_b200_opt_gemm_cframes(iarray_context_t *ctx, const uint
     for (int64_t r = 0; r < rowsB; r++) upload_row(fb, b_frame, db, r, ctx->up, evB.ev[(size_t)r]);
     for (int64_t r = 0; r < rowsA; r++) upload_row(fa, a_frame, da, r, ctx->up, evA.ev[(size_t)r]);
 
-    // Three compute streams: the second stream decodes (B's chunk rows, then A's, each as
-    // soon as it is uploaded), the context stream prepares B and multiplies each band, the
-    // encode stream encodes each finished band.  A band's decode and the previous band's
-    // encode are both latency-bound and run side by side.
-    cudaStream_t sd = ctx->stream2, se = ctx->enc;
+    // Compute streams: the second stream decodes (B's chunk rows, then A's, each as soon as it
+    // is uploaded), the context stream prepares B and multiplies each band, the encode streams
+    // take turns encoding the finished bands.  A band's decode and the previous bands' encodes
+    // are latency-bound and run side by side.
+    cudaStream_t sd = ctx->stream2;
+    constexpr int64_t NENC = sizeof(ctx->enc) / sizeof(ctx->enc[0]);
     cudaStreamWaitEvent(sd, ctx->fork, 0);
-    cudaStreamWaitEvent(se, ctx->fork, 0);
+    for (auto &e : ctx->enc) cudaStreamWaitEvent(e, ctx->fork, 0);
     Timer tm(ctx);                 // timings: [0] B decoded and prepared, [3] the bands, [4] total
     tm.mark(1);
     int err = 0;
@@ -1793,15 +1799,20 @@ INA_API(ina_rc_t) iarray_b200_opt_gemm_cframes(iarray_context_t *ctx, const uint
         }
         acc += bytes;
     };
-    int64_t queued = 0;            // bands whose encode is queued
+    int64_t queued = 0, drained = 0;   // bands whose encode, whose download is queued
+    const bool exact_lz4 = ctx->encoder == IARRAY_B200_ENCODER_LIBLZ4;
     for (int64_t k = 0; k < bands && !err; k++) {
         cudaStreamWaitEvent(st, evD.ev[(size_t)k], 0);
-        // split form: a band's product (about 1.6 ms for 2048 x 8192 x 8192) is shorter than
-        // the download of an encoded band, so the downloads bound the call once the first
-        // band is out; each product waits for the previous band's encode kernels, which then
-        // run alone instead of sharing the SMs with the product (the native form's products
-        // are the longer part and keep overlapping the encodes)
-        if (split && k > 0) cudaStreamWaitEvent(st, evK.ev[(size_t)k - 1], 0);
+        // split form, parallel encoder: a band's product (about 1.6 ms for 2048 x 8192 x 8192)
+        // is shorter than the download of an encoded band, so the downloads bound the call once
+        // the first band is out; each product waits for the previous band's encode kernels,
+        // which then run alone instead of sharing the SMs with the product (the native form's
+        // products are the longer part and keep overlapping the encodes).  The liblz4-identical
+        // encoder spends a band's time on the serial chains of its few compressible streams,
+        // one warp each, and leaves the SMs to the next bands: nothing waits for it (4096^3
+        // float64, bands of 1024 rows: 15.0 -> 9.5 ms).
+        cudaStream_t se = ctx->enc[k % NENC];
+        if (split && !exact_lz4 && k > 0) cudaStreamWaitEvent(st, evK.ev[(size_t)k - 1], 0);
         const int64_t r0 = k * gc.chunk[0], mk = row_geom(fa.g, k).shape[0];
         uint8_t *a_k = dA.as<uint8_t>() + r0 * lda * isz, *c_k = dC.as<uint8_t>() + r0 * ldc * isz;
         const Geom gk = row_geom(gc, k);
@@ -1826,7 +1837,7 @@ INA_API(ina_rc_t) iarray_b200_opt_gemm_cframes(iarray_context_t *ctx, const uint
         if (err) break;
         cudaEventRecord(evP.ev[(size_t)k], st);
         cudaStreamWaitEvent(se, evP.ev[(size_t)k], 0);
-        w.exact_lz4 = ctx->encoder == IARRAY_B200_ENCODER_LIBLZ4;
+        w.exact_lz4 = exact_lz4;
         w.memcpy_only = cc->clevel == 0;
         err = iab::encode_launch(gk, c_k, ldc, cc->shuffle, cc->splitmode, &cbuf[(size_t)k], &w, se);
         if (err) break;
@@ -1839,9 +1850,10 @@ INA_API(ina_rc_t) iarray_b200_opt_gemm_cframes(iarray_context_t *ctx, const uint
                         cudaMemcpyDeviceToHost, ctx->tabs);
         cudaEventRecord(evE.ev[(size_t)k], ctx->tabs);
         queued = k + 1;
-        if (k > 0) drain(k - 1);
+        while (drained < k && cudaEventQuery(evE.ev[(size_t)drained]) == cudaSuccess) drain(drained++);
+        if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();   // the query's, not an error
     }
-    if (!err) drain(bands - 1);
+    while (!err && drained < bands) drain(drained++);
     // the context stream waits for the other compute streams before the final timestamp
     cudaEventRecord(ctx->join, sd);
     cudaStreamWaitEvent(st, ctx->join, 0);
@@ -1849,7 +1861,12 @@ INA_API(ina_rc_t) iarray_b200_opt_gemm_cframes(iarray_context_t *ctx, const uint
     tm.mark(4);
     const cudaError_t ce1 = cudaStreamSynchronize(st), ce2 = cudaStreamSynchronize(ctx->down),
                       ce3 = cudaStreamSynchronize(ctx->up), ce4 = cudaStreamSynchronize(sd),
-                      ce5 = cudaStreamSynchronize(se), ce6 = cudaStreamSynchronize(ctx->tabs);
+                      ce6 = cudaStreamSynchronize(ctx->tabs);
+    cudaError_t ce5 = cudaSuccess;
+    for (auto &e : ctx->enc) {
+        const cudaError_t ce = cudaStreamSynchronize(e);
+        if (ce != cudaSuccess) ce5 = ce;
+    }
     tm.finish();
     if (err == -100) return rc_err(IARRAY_ERR_GPU_OUT_OF_MEMORY);
     if (err || ce1 != cudaSuccess || ce2 != cudaSuccess || ce3 != cudaSuccess || ce4 != cudaSuccess ||
