@@ -457,39 +457,29 @@ INA_API(void) iarray_container_free(iarray_context_t *ctx, iarray_container_t **
     *container = nullptr;
 }
 
-// Encode a dense device array (row-major, leading dimension ld) into c's store.
-static ina_rc_t encode_into(iarray_context_t *ctx, iarray_container_t *c, const void *dense, int64_t ld)
+// Encode a dense device array (row-major, leading dimension ld) into c's store; with `image`, from
+// the image that the product wrote into it (iab::encode_image_prepare) instead.
+static ina_rc_t encode_into(iarray_context_t *ctx, iarray_container_t *c, const void *dense, int64_t ld,
+                            iab::EncodeWork *image = nullptr)
 {
     ChunkStore &s = *c->store;
     DevBuf out;
     std::vector<int64_t> off;
     std::vector<int32_t> len;
-    int r = iab::encode_container(c->geom, dense, ld, c->shuffle, c->splitmode, &out, &off, &len, ctx->stream,
-                                  ctx->encoder == IARRAY_B200_ENCODER_LIBLZ4, c->clevel == 0);
+    iab::EncodeWork own, &w = image ? *image : own;
+    w.exact_lz4 = ctx->encoder == IARRAY_B200_ENCODER_LIBLZ4;
+    w.memcpy_only = c->clevel == 0;
+    const int r = image ? iab::encode_image_finish(c->geom, c->shuffle, c->splitmode, &out, &off, &len, ctx->stream, &w)
+                        : iab::encode_container(c->geom, dense, ld, c->shuffle, c->splitmode, &out, &off, &len, ctx->stream, &w);
     if (r == -100) return rc_err(IARRAY_ERR_GPU_OUT_OF_MEMORY);
     if (r != 0) return rc_err(IARRAY_ERR_GPU_FAILED);
     s.buf = std::move(out);
     s.off = std::move(off);
     s.len = std::move(len);
-    if (!s.upload_index()) return rc_err(IARRAY_ERR_GPU_OUT_OF_MEMORY);
-    return INA_SUCCESS;
-}
-
-// encode_into for an image the product wrote (iab::encode_image_prepare).
-static ina_rc_t encode_into_image(iarray_context_t *ctx, iarray_container_t *c, iab::EncodeWork *w)
-{
-    ChunkStore &s = *c->store;
-    DevBuf out;
-    std::vector<int64_t> off;
-    std::vector<int32_t> len;
-    int r = iab::encode_image_finish(c->geom, c->shuffle, c->splitmode, &out, &off, &len, ctx->stream,
-                                     ctx->encoder == IARRAY_B200_ENCODER_LIBLZ4, w);
-    if (r == -100) return rc_err(IARRAY_ERR_GPU_OUT_OF_MEMORY);
-    if (r != 0) return rc_err(IARRAY_ERR_GPU_FAILED);
-    s.buf = std::move(out);
-    s.off = std::move(off);
-    s.len = std::move(len);
-    if (!s.upload_index()) return rc_err(IARRAY_ERR_GPU_OUT_OF_MEMORY);
+    s.d_off = std::move(w.d_off);          // written by the encode's kernels
+    s.d_len = std::move(w.d_len);
+    s.cbytes = 0;
+    for (int32_t l : s.len) s.cbytes += l;
     return INA_SUCCESS;
 }
 
@@ -540,14 +530,17 @@ static ina_rc_t decode_pair(iarray_context_t *ctx, const iarray_container_t *a, 
          b->store->d_len.as<int32_t>(), db, ldb}};
     iab::DecodeQueue q;
     iab::DecodeWork w[2];
-    int r = iab::decode_queue_init(&q, iab::decode_max_jobs(a->geom) + iab::decode_max_jobs(b->geom), ctx->stream);
+    int r = iab::decode_queue_init(&q, iab::decode_max_jobs(a->geom) + iab::decode_max_jobs(b->geom), 2, ctx->stream);
     for (int k = 0; k < 2 && !r; k++)
         if (x[k]->geom.nchunks) r = iab::decode_parse(args[k], &q, &w[k], ctx->stream);
     if (!r) r = iab::decode_lz4(&q, ctx->stream);
     for (int k = 0; k < 2 && !r; k++)
         if (x[k]->geom.nchunks) r = iab::decode_scatter(args[k], &w[k], ctx->stream);
-    for (int k = 0; k < 2 && !r; k++)
-        if (x[k]->geom.nchunks) r = iab::decode_finish(&w[k], ctx->stream);
+    iab::DecodeWork *parsed[2];
+    int np = 0;
+    for (int k = 0; k < 2; k++)
+        if (x[k]->geom.nchunks) parsed[np++] = &w[k];
+    if (!r && np) r = iab::decode_finish_queue(&q, parsed, np, ctx->stream);
     if (r) cudaStreamSynchronize(ctx->stream);     // the work buffers go back to the pool idle
     for (int k = 0; k < 2 && !r; k++) {
         if (zf) zf[k] = std::move(w[k].zf);
@@ -1265,14 +1258,14 @@ static ina_rc_t gemv_fused(iarray_context_t *ctx, const iarray_container_t *a, c
     iab::DecodeQueue q;
     iab::DecodeWork w[2];
     const bool xc = b->geom.nchunks > 0;
-    int r = iab::decode_queue_init(&q, iab::decode_max_jobs(g) + iab::decode_max_jobs(b->geom), ctx->stream);
+    int r = iab::decode_queue_init(&q, iab::decode_max_jobs(g) + iab::decode_max_jobs(b->geom), 2, ctx->stream);
     if (!r) r = iab::decode_parse(args[0], &q, &w[0], ctx->stream);
     if (!r && xc) r = iab::decode_parse(args[1], &q, &w[1], ctx->stream);
     if (!r) r = iab::decode_lz4(&q, ctx->stream);
     if (!r && xc) r = iab::decode_scatter(args[1], &w[1], ctx->stream);
     if (!r) r = iab::decode_gemv(args[0], &w[0], dx, part.p, dy, ctx->stream);
-    if (!r) r = iab::decode_finish(&w[0], ctx->stream);
-    if (!r && xc) r = iab::decode_finish(&w[1], ctx->stream);
+    iab::DecodeWork *parsed[2] = {&w[0], &w[1]};
+    if (!r) r = iab::decode_finish_queue(&q, parsed, xc ? 2 : 1, ctx->stream);
     if (!r && skip != SKIP_NONE && w[0].nzero + (xc ? w[1].nzero : 0) > 0) {
         if (!dA->allocate((size_t)std::max<int64_t>(g.shape[0] * lda * g.itemsize, 16), ctx->device)) {
             cudaStreamSynchronize(ctx->stream);
@@ -1385,7 +1378,7 @@ static ina_rc_t run_matmul(iarray_context_t *ctx, iarray_container_t *a, iarray_
     // dA and dB stay allocated until the encode below has synchronised the stream: the pool is
     // shared by every context, so memory released while the product may still read it could be
     // handed to another stream
-    if (direct) rc = encode_into_image(ctx, c, &ew);
+    if (direct) rc = encode_into(ctx, c, nullptr, 0, &ew);
     else rc = c->geom.nchunks ? encode_into(ctx, c, dC.p, vec ? M : ldc) : fill_zero_chunks(c);
     if (INA_FAILED(rc)) return rc;
     tm.mark(4);

@@ -35,49 +35,89 @@ namespace iab {
 
 #define FULLMASK 0xffffffffu
 
+// 4 bytes at any address; the aligned words read hold at least one of them each.
 __device__ __forceinline__ int32_t ld_s32(const uint8_t *p)
 {
-    return (int32_t)((uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24));
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~uintptr_t(3));
+    const uint32_t sh = (uint32_t)(a & 3) * 8;
+    return (int32_t)__funnelshift_r(__ldg(w), sh ? __ldg(w + 1) : 0u, sh);
 }
 
 __device__ __forceinline__ void dev_fail(int *err, int code) { atomicCAS(err, 0, code); }
 
+// q = a / b, r = a - q b for a >= 0, b > 0: 32-bit division when both fit (the usual case),
+// 64-bit otherwise.
+__device__ __forceinline__ void divmod(int64_t a, int64_t b, int64_t &q, int64_t &r)
+{
+    if (((a | b) >> 31) == 0) {
+        const uint32_t q32 = (uint32_t)a / (uint32_t)b;
+        q = q32;
+        r = a - (int64_t)q32 * b;
+    } else {
+        q = a / b;
+        r = a - q * b;
+    }
+}
+
 // ============================================================================ decode
-// D0: parse one (chunk, block) per thread.
+// D0: parse one (chunk, block) per thread.  What bounds it is the chain of loads: chunk offset,
+// header, block start, and one size word after the other, each where the stream before it ends.
+// So every word is one load (two when it straddles words), the block start is loaded beside the
+// header, and the size words are loaded at once where they lie when the streams before them are
+// raw, the usual case but for the last planes; a word that lies elsewhere is loaded when its
+// place is known.
 // zf (optional): per (chunk, block) zero flags of the reference's block-pair products:
 // bit 0 = block_is_zeros (src/linalg/iarray_gemm.c:28-77: no memcpyed or special chunk, and
 // the first typesize csize words from the block's bstart are all 0: Blosc2 v5 chunks always
 // carry the flag bit the reference reads as "split"), bit 1 = chunk_is_zeros (:17-26:
 // special value ZERO); nzero counts the flagged blocks.
+struct ParsedBlock {
+    uint32_t lz;               // bit j: stream j is an LZ4 stream
+    int32_t q[8], cs[8];       // its payload's place in the chunk, its size
+    int32_t neblock;
+    const uint8_t *chunk;
+};
 __device__ __forceinline__ void parse_block(const Geom &g, const uint8_t *__restrict__ ch, const int64_t *__restrict__ off,
-                                            const int32_t *__restrict__ len, BlockDesc *bd, StreamDesc *sd,
-                                            Lz4Job *jobs, int *njobs, int64_t jcap, int *err, uint8_t *scratch,
-                                            uint8_t *zf, int *nzero, int64_t t)
+                                            const int32_t *__restrict__ len, BlockDesc *bd, StreamDesc *sd, int *err,
+                                            uint8_t *zf, int *nzero, int64_t t, ParsedBlock &pb)
 {
+    pb.lz = 0;
     do {
-        const int64_t c = t / g.nblocks, b = t % g.nblocks;
-        const uint8_t *p = ch + off[c];
+        int64_t c, b;
+        divmod(t, g.nblocks, c, b);
+        const int64_t coff = off[c];
+        const uint8_t *p = ch + coff;
         const int32_t clen = len[c];
         BlockDesc d;
         d.mode = BM_PLAIN; d.nstreams = 1; d.neblock = (int32_t)g.blocksize; d.pad = 0; d.value_src = 0;
         StreamDesc *s = sd + t * 8;
         for (int j = 0; j < 8; j++) { s[j].kind = SK_RUN; s[j].len = 0; s[j].src = 0; }
         bool ok = clen >= 32;
-        int32_t nbytes = 0, bsz = 0, cbytes = 0;
-        uint8_t flags = 0, ts = 0, bflags = 0;
+        int32_t w0 = 0, nbytes = 0, bsz = 0, cbytes = 0, w16 = 0, w20 = 0, w28 = 0;
+        int64_t bstart = 0;
         if (ok) {
-            flags = p[2]; ts = p[3]; bflags = p[31];
-            nbytes = ld_s32(p + 4); bsz = ld_s32(p + 8); cbytes = ld_s32(p + 12);
-            ok = (flags & 0x05) == 0x05 && nbytes == g.chunk_nbytes && cbytes >= 32 && cbytes <= clen;
+            w0 = ld_s32(p); nbytes = ld_s32(p + 4); bsz = ld_s32(p + 8); cbytes = ld_s32(p + 12);
+            w16 = ld_s32(p + 16); w20 = ld_s32(p + 20); w28 = ld_s32(p + 28);
+            if (36 + 4 * b <= clen) bstart = ld_s32(p + 32 + 4 * b);
         }
+        const uint8_t flags = (uint8_t)(w0 >> 16), ts = (uint8_t)((uint32_t)w0 >> 24), bflags = (uint8_t)((uint32_t)w28 >> 24);
+        if (ok) ok = (flags & 0x05) == 0x05 && nbytes == g.chunk_nbytes && cbytes >= 32 && cbytes <= clen;
         if (!ok) { dev_fail(err, DE_HEADER); bd[t] = d; if (zf) zf[t] = 0; continue; }
+        // the size words of a split block whose streams before them are raw
+        const int32_t neb = (int32_t)(g.blocksize / g.itemsize);
+        int32_t pre[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int64_t q = bstart + (int64_t)j * (neb + 4);
+            pre[j] = j < g.itemsize && bstart >= 32 && q + 4 <= cbytes ? ld_s32(p + q) : 0;
+        }
         const int special = (bflags >> 4) & 7;
         if (zf) {
             uint8_t zflag = special == 1 ? 2 : 0;
             if (!special && !(flags & 0x02) && 32 + 4 * (b + 1) <= cbytes) {
-                const int64_t q0 = ld_s32(p + 32 + 4 * b);
-                bool z = q0 >= 32 && q0 + 4 * (int64_t)ts <= cbytes;
-                for (int j = 0; z && j < ts; j++) z = ld_s32(p + q0 + 4 * j) == 0;
+                bool z = bstart >= 32 && bstart + 4 * (int64_t)ts <= cbytes && (ts == 0 || pre[0] == 0);
+                for (int j = 1; z && j < ts; j++) z = ld_s32(p + bstart + 4 * j) == 0;
                 if (z) zflag |= 1;
             }
             zf[t] = zflag;
@@ -87,73 +127,115 @@ __device__ __forceinline__ void parse_block(const Geom &g, const uint8_t *__rest
             if (special == 2) d.mode = BM_NAN;
             else if (special == 3) {
                 if (cbytes < 32 + (int32_t)g.itemsize) dev_fail(err, DE_HEADER);
-                d.mode = BM_VALUE; d.value_src = off[c] + 32;
+                d.mode = BM_VALUE; d.value_src = coff + 32;
             } else if (special != 1 && special != 4) dev_fail(err, DE_HEADER);
             bd[t] = d;
             continue;
         }
         if (flags & 0x02) {                      // memcpyed: raw blocked items
             if (cbytes < 32 + nbytes) { dev_fail(err, DE_BOUNDS); bd[t] = d; continue; }
-            s[0].kind = SK_RAW; s[0].len = (int32_t)g.blocksize; s[0].src = off[c] + 32 + b * g.blocksize;
+            s[0].kind = SK_RAW; s[0].len = (int32_t)g.blocksize; s[0].src = coff + 32 + b * g.blocksize;
             bd[t] = d;
             continue;
         }
         // filters: only SHUFFLE (slot 5 == 1) or none are produced on this path
-        bool filt_ok = p[16] == 0 && p[17] == 0 && p[18] == 0 && p[19] == 0 && p[20] == 0 && p[21] <= 1;
+        const uint8_t filter5 = (uint8_t)((uint32_t)w20 >> 8);
+        const bool filt_ok = w16 == 0 && (w20 & 0xFF) == 0 && filter5 <= 1;
         if (bsz != g.blocksize || ts != g.itemsize || !filt_ok) { dev_fail(err, DE_HEADER); bd[t] = d; continue; }
         const bool split = !(flags & 0x10);
-        const bool shuffle = p[21] == 1 && ts > 1;
+        const bool shuffle = filter5 == 1 && ts > 1;
         const int nstreams = split ? ts : 1;
         const int neblock = (int)(g.blocksize / nstreams);
         d.mode = shuffle ? BM_SHUFFLED : BM_PLAIN;
         d.nstreams = nstreams; d.neblock = neblock;
+        pb.neblock = neblock;
+        pb.chunk = p;
         const int64_t bs_end = 32 + 4 * g.nblocks;
         if (bs_end > cbytes) { d.mode = BM_PLAIN; dev_fail(err, DE_BOUNDS); bd[t] = d; continue; }
-        int64_t q = ld_s32(p + 32 + 4 * b);
+        int64_t q = bstart;
         if (q < bs_end || q >= cbytes) { d.mode = BM_PLAIN; dev_fail(err, DE_BOUNDS); bd[t] = d; continue; }
-        for (int j = 0; j < nstreams; j++) {
+        uint32_t lz = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (j >= nstreams || !ok) break;
             if (q + 4 > cbytes) { dev_fail(err, DE_BOUNDS); ok = false; break; }
-            const int32_t cs = ld_s32(p + q);
+            const int32_t cs = q == bstart + (int64_t)j * (neb + 4) ? pre[j] : ld_s32(p + q);
             q += 4;
-            if (cs == 0) { s[j].kind = SK_RUN; s[j].len = 0; s[j].src = 0; continue; }
+            if (cs == 0) continue;
             if (cs < 0) {
                 if (q + 1 > cbytes || !(p[q] & 1) || cs < -255) { dev_fail(err, DE_RUN_TOKEN); ok = false; break; }
                 q += 1;
-                s[j].kind = SK_RUN; s[j].len = -cs; s[j].src = 0;
+                s[j].len = -cs;
                 continue;
             }
             if (q + cs > cbytes || cs > neblock) { dev_fail(err, DE_BOUNDS); ok = false; break; }
-            s[j].src = off[c] + q;
+            s[j].src = coff + q;
             s[j].len = cs;
             if (cs == neblock) {
                 s[j].kind = SK_RAW;
             } else {
                 s[j].kind = SK_LZ4;
-                const int k = atomicAdd(njobs, 1);
-                if (k < jcap) {
-                    Lz4Job jb;
-                    jb.src = ch + off[c] + q; jb.dst = scratch + t * g.blocksize + (int64_t)j * neblock; jb.err = err;
-                    jb.csize = cs; jb.dlen = neblock;
-                    jobs[k] = jb;
-                } else {
-                    dev_fail(err, DE_BOUNDS);                            // queue full: left undecoded
-                }
+                lz |= 1u << j;
+                pb.q[j] = (int32_t)q;
+                pb.cs[j] = cs;
             }
             q += cs;
         }
         if (!ok) { for (int j = 0; j < nstreams; j++) { s[j].kind = SK_RUN; s[j].len = 0; } }
+        else pb.lz = lz;
         bd[t] = d;
     } while (false);
 }
 
+// Queues the LZ4 streams of a warp's blocks (every lane calls): stream j of a block goes to region
+// j of the queue, counted by njobs[j], so that the decoder gets the streams plane by plane.  (The
+// first planes of smooth floats are the longest streams, the last one the shortest: handed out in
+// the blocks' order instead, the decode of a 20000 x 20000 float32 matrix takes 6.45 ms, by planes 6.0.)
+// The eight counters are bumped by one instruction per warp.
+__device__ __forceinline__ void queue_streams(const ParsedBlock &pb, uint8_t *blk_scratch, int *err, Lz4Job *jobs,
+                                              int *njobs, int64_t jcap)
+{
+    const int lane = threadIdx.x & 31;
+    if (!__any_sync(FULLMASK, pb.lz != 0)) return;
+    const int64_t region = jcap / 8;
+    int mine = 0;                          // lane j: streams of plane j
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int n = __popc(__ballot_sync(FULLMASK, (pb.lz >> j) & 1u));
+        if (lane == j) mine = n;
+    }
+    int at = 0;
+    if (mine) at = atomicAdd(njobs + lane, mine);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const bool has = (pb.lz >> j) & 1u;
+        const unsigned m = __ballot_sync(FULLMASK, has);
+        const int64_t k = (int64_t)__shfl_sync(FULLMASK, at, j) + __popc(m & ((1u << lane) - 1u));
+        if (!has) continue;
+        if (k < region) {
+            Lz4Job jb;
+            jb.src = pb.chunk + pb.q[j]; jb.dst = blk_scratch + (int64_t)j * pb.neblock; jb.err = err;
+            jb.csize = pb.cs[j]; jb.dlen = pb.neblock;
+            jobs[j * region + k] = jb;
+        } else {
+            dev_fail(err, DE_BOUNDS);                                // (a region holds a stream of every block)
+        }
+    }
+}
+
+// (blockDim.x is a multiple of 32)
 __global__ void k_parse(Geom g, const uint8_t *__restrict__ ch, const int64_t *__restrict__ off,
                         const int32_t *__restrict__ len, BlockDesc *bd, StreamDesc *sd, Lz4Job *jobs,
                         int *njobs, int64_t jcap, int *err, uint8_t *scratch, uint8_t *zf, int *nzero)
 {
     const int64_t total = g.nchunks * g.nblocks;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x)
-        parse_block(g, ch, off, len, bd, sd, jobs, njobs, jcap, err, scratch, zf, nzero, t);
+    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x; t0 < total; t0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t t = t0 + threadIdx.x;
+        ParsedBlock pb;
+        pb.lz = 0;
+        if (t < total) parse_block(g, ch, off, len, bd, sd, err, zf, nzero, t, pb);
+        queue_streams(pb, scratch + t * g.blocksize, err, jobs, njobs, jcap);
+    }
 }
 
 // D1: LZ4 stream decode, one CTA (256 threads) per stream, streams handed out
@@ -260,14 +342,14 @@ __device__ __forceinline__ uint16_t dcta_next(const uint8_t *win, int q, int n, 
 }
 
 __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Job *__restrict__ jobs,
-                                                                  const int *__restrict__ njobs_p, int64_t jcap,
+                                                                  const int *__restrict__ planes, int64_t jcap,
                                                                   unsigned *next_job)
 {
     using namespace dcta;
     extern __shared__ __align__(16) uint8_t sm_dcta[];
     Smem &S = *reinterpret_cast<Smem *>(sm_dcta);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int njobs = (int)min((int64_t)*njobs_p, jcap);
+    const int64_t region = jcap / 8;               // the queue's part for one plane
     if (tid == 0) S.nlong = S.nvlong = 0;          // first use follows the barriers below
     // 16 bytes of the window at p from its 16-byte boundary; every block read holds a byte of the stream
     auto fetch = [&](const uint8_t *in, int p, int isz) -> uint4 {
@@ -279,9 +361,15 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
         __syncthreads();
         if (tid == 0) S.scal[0] = (int)atomicAdd(next_job, 1u);
         __syncthreads();
-        const int jid = S.scal[0];
-        if (jid >= njobs) break;
-        const Lz4Job jb = jobs[jid];
+        int64_t jid = (unsigned)S.scal[0];
+        int plane = 0;
+        for (; plane < 8; plane++) {
+            const int64_t n = min((int64_t)planes[plane], region);
+            if (jid < n) break;
+            jid -= n;
+        }
+        if (plane == 8) break;
+        const Lz4Job jb = jobs[plane * region + jid];
         const uint8_t *__restrict__ in = jb.src;
         const int isz = jb.csize;
         uint8_t *out = jb.dst;
@@ -645,20 +733,6 @@ __device__ __forceinline__ bool geom_quads(const Geom &g) { return !(g.block[1] 
 
 // Block b of chunk c: its first logical row and column, and how many of its rows (nr) and
 // columns (nc) hold logical items (the rest is chunk or array padding; 0 when none do).
-// q = a / b, r = a - q b for a >= 0, b > 0: 32-bit division when both fit (the usual case),
-// 64-bit otherwise.
-__device__ __forceinline__ void divmod(int64_t a, int64_t b, int64_t &q, int64_t &r)
-{
-    if (((a | b) >> 31) == 0) {
-        const uint32_t q32 = (uint32_t)a / (uint32_t)b;
-        q = q32;
-        r = a - (int64_t)q32 * b;
-    } else {
-        q = a / b;
-        r = a - q * b;
-    }
-}
-
 struct BlockSpan {
     int64_t row0, col0;
     int nr, nc;
@@ -684,9 +758,9 @@ __device__ __forceinline__ BlockSpan block_span(const Geom &g, int64_t c, int64_
 // padding only are skipped): 4 consecutive items from one 4-byte word per plane where block rows
 // hold whole groups of 4, else one item from a byte per plane, consecutive lanes taking
 // consecutive items (4000 x 6000 float64 in blocks of 100 x 150: 0.12 ms, 0.79 by the general
-// path's bytewise tiles).  Every other block is
-// appended to the list `rest` for the general path.
+// path's bytewise tiles).  Blocks of other kinds go by the general path.
 constexpr int SC_ITEMS = 4096;
+constexpr int GA_ITEMS = 16384;                    // items of a gather slice
 constexpr int SC_PLANE = SC_ITEMS + 32;            // a slice of a plane from its 16-byte boundary
 constexpr uint32_t SC_WAIT_POLLS = 1u << 22;
 
@@ -703,25 +777,84 @@ __device__ __forceinline__ bool sc_wait(uint64_t *bar, uint32_t parity)
     return false;
 }
 
+// D2 general path: unshuffle one tile of TILE items of one block through shared memory
+// and scatter it to the dense array (other item sizes; plain, special and unsplit blocks).
+__device__ __forceinline__ void scatter_tile(const Geom &g, const uint8_t *__restrict__ ch,
+                                             const BlockDesc *__restrict__ bd, const StreamDesc *__restrict__ sd,
+                                             const uint8_t *__restrict__ scratch, uint8_t *__restrict__ out, int64_t ld,
+                                             int64_t t, int64_t i0, uint8_t *planes)
+{
+    const int ts = g.itemsize;
+    const int cnt = (int)min((int64_t)TILE, g.blockn - i0);
+    const int64_t c = t / g.nblocks, b = t - c * g.nblocks;
+    const BlockDesc d = bd[t];
+    const StreamDesc *s = sd + t * 8;
+    const uint8_t *blk_scratch = scratch + t * g.blocksize;
+    if (d.mode == BM_SHUFFLED) {
+        for (int j = 0; j < ts; j++) {
+            const int64_t pos = (int64_t)j * g.blockn + i0;
+            const int sidx = (int)(pos / d.neblock);
+            const int64_t so = pos - (int64_t)sidx * d.neblock;
+            const StreamDesc q = s[sidx];
+            uint8_t *pl = planes + j * TILE;
+            if (q.kind == SK_RUN) {
+                for (int x = threadIdx.x; x < cnt; x += blockDim.x) pl[x] = (uint8_t)q.len;
+            } else if (q.kind == SK_RAW) {
+                const uint8_t *src = ch + q.src + so;
+                for (int x = threadIdx.x; x < cnt; x += blockDim.x) pl[x] = __ldg(src + x);
+            } else {
+                const uint8_t *src = blk_scratch + (int64_t)sidx * d.neblock + so;
+                for (int x = threadIdx.x; x < cnt; x += blockDim.x) pl[x] = __ldcg(src + x);
+            }
+        }
+    } else if (d.mode == BM_PLAIN) {
+        for (int x = threadIdx.x; x < cnt * ts; x += blockDim.x) {
+            const int64_t pos = i0 * ts + x;
+            const int sidx = (int)(pos / d.neblock);
+            const int64_t so = pos - (int64_t)sidx * d.neblock;
+            const StreamDesc q = s[sidx];
+            uint8_t v;
+            if (q.kind == SK_RUN) v = (uint8_t)q.len;
+            else if (q.kind == SK_RAW) v = __ldg(ch + q.src + so);
+            else v = __ldcg(blk_scratch + (int64_t)sidx * d.neblock + so);
+            planes[x] = v;
+        }
+    }
+    __syncthreads();
+    for (int x = threadIdx.x; x < cnt; x += blockDim.x) {
+        int64_t row, col;
+        if (!item_pos(g, c, b, i0 + x, row, col)) continue;
+        uint8_t *o = out + (row * ld + col) * ts;
+        uint64_t v = 0;
+        if (d.mode == BM_SHUFFLED) {
+            for (int j = 0; j < ts; j++) v |= (uint64_t)planes[j * TILE + x] << (8 * j);
+        } else if (d.mode == BM_PLAIN) {
+            for (int j = 0; j < ts; j++) v |= (uint64_t)planes[x * ts + j] << (8 * j);
+        } else if (d.mode == BM_NAN) {
+            v = ts == 8 ? 0x7FF8000000000000ull : 0x7FC00000ull;
+        } else {
+            v = load_item_bytes(ch + d.value_src, ts);
+        }
+        store_item(o, ts, v);
+    }
+    __syncthreads();
+}
+
 // One slice (t, sl) of the fast scatter; false when a bounded wait gave up (the CTA must
-// leave).  rest_id: the block's entry for the general path's list.
+// leave).  Blocks of other kinds are left out and set `general`.
 template <int TS>
 __device__ __forceinline__ bool scatter_fast_unit(const Geom &g, const uint8_t *__restrict__ ch, const uint8_t *ch_end,
                                                   const BlockDesc *__restrict__ bd, const StreamDesc *__restrict__ sd,
                                                   const uint8_t *__restrict__ scratch, const uint8_t *scratch_end,
-                                                  uint8_t *__restrict__ out, int64_t ld, int *rest, int *nrest,
-                                                  int rest_id, int *err, int64_t t, int sl, uint8_t (*stage)[SC_PLANE],
-                                                  uint64_t *bar, uint32_t &parity, int *abort_all)
+                                                  uint8_t *__restrict__ out, int64_t ld, int *err, int64_t t, int sl, uint8_t (*stage)[SC_PLANE],
+                                                  uint64_t *bar, uint32_t &parity, int *abort_all, bool &general)
 {
     const int tid = threadIdx.x;
     const int rowlen = (int)g.block[1];
     int64_t c, b;
     divmod(t, g.nblocks, c, b);
     const BlockDesc d = bd[t];
-    if (d.mode != BM_SHUFFLED || d.nstreams != TS) {
-        if (tid == 0 && sl == 0) rest[atomicAdd(nrest, 1)] = rest_id;   // left to k_scatter
-        return true;
-    }
+    if (d.mode != BM_SHUFFLED || d.nstreams != TS) { general = true; return true; }
     const BlockSpan sp = block_span(g, c, b);
     const int i0s = sl * SC_ITEMS, cnt = (int)min((int64_t)SC_ITEMS, g.blockn - i0s);
     if (sp.nc == 0 || i0s / rowlen >= sp.nr) return true;             // the slice holds only padding
@@ -857,13 +990,12 @@ __device__ __forceinline__ bool scatter_fast_unit(const Geom &g, const uint8_t *
     return true;
 }
 
-template <int TS>
+template <int TS, bool ALL>
 __global__ void __launch_bounds__(256, 6) k_scatter_fast(Geom g, const uint8_t *__restrict__ ch, const uint8_t *ch_end,
                                                       const BlockDesc *__restrict__ bd,
                                                       const StreamDesc *__restrict__ sd,
                                                       const uint8_t *__restrict__ scratch, const uint8_t *scratch_end,
-                                                      uint8_t *__restrict__ out, int64_t ld, int *rest, int *nrest,
-                                                      int *err)
+                                                      uint8_t *__restrict__ out, int64_t ld, int *err)
 {
     __shared__ __align__(128) uint8_t stage[TS][SC_PLANE];
     __shared__ __align__(8) uint64_t bar;
@@ -878,91 +1010,51 @@ __global__ void __launch_bounds__(256, 6) k_scatter_fast(Geom g, const uint8_t *
     const int64_t nbl = g.nchunks * g.nblocks;
     const int64_t nsl = (g.blockn + SC_ITEMS - 1) / SC_ITEMS;
     uint32_t parity = 0;
+    bool general = false;
     for (int64_t u = blockIdx.x; u < nbl * nsl; u += gridDim.x) {
         int64_t t, s64;
         divmod(u, nsl, t, s64);
         const int sl = (int)s64;
-        if (!scatter_fast_unit<TS>(g, ch, ch_end, bd, sd, scratch, scratch_end, out, ld, rest, nrest, (int)t, err, t, sl,
-                                   stage, &bar, parity, &abort_all))
+        if (!scatter_fast_unit<TS>(g, ch, ch_end, bd, sd, scratch, scratch_end, out, ld, err, t, sl,
+                                   stage, &bar, parity, &abort_all, general))
             return;
     }
+    // the blocks of other kinds among this CTA's slices (no bulk copy follows: the stage is free)
+    for (int64_t u = blockIdx.x; ALL && general && u < nbl * nsl; u += gridDim.x) {
+        int64_t t, sl;
+        divmod(u, nsl, t, sl);
+        if (bd[t].mode == BM_SHUFFLED && bd[t].nstreams == TS) continue;
+        const int64_t end = min(g.blockn, (sl + 1) * SC_ITEMS);
+        for (int64_t i0 = sl * SC_ITEMS; i0 < end; i0 += TILE)
+            scatter_tile(g, ch, bd, sd, scratch, out, ld, t, i0, stage[0]);
+    }
 }
 
-// D2 general path: unshuffle one tile of TILE items of one block through shared memory
-// and scatter it to the dense array (padded edge blocks, other item sizes, plain and
-// special chunks).  With a `rest` list, only the blocks listed there; else every block.
-__device__ __forceinline__ void scatter_tile(const Geom &g, const uint8_t *__restrict__ ch,
-                                             const BlockDesc *__restrict__ bd, const StreamDesc *__restrict__ sd,
-                                             const uint8_t *__restrict__ scratch, uint8_t *__restrict__ out, int64_t ld,
-                                             int64_t t, int64_t i0, uint8_t *planes)
-{
-    const int ts = g.itemsize;
-    const int cnt = (int)min((int64_t)TILE, g.blockn - i0);
-    const int64_t c = t / g.nblocks, b = t - c * g.nblocks;
-    const BlockDesc d = bd[t];
-    const StreamDesc *s = sd + t * 8;
-    const uint8_t *blk_scratch = scratch + t * g.blocksize;
-    if (d.mode == BM_SHUFFLED) {
-        for (int j = 0; j < ts; j++) {
-            const int64_t pos = (int64_t)j * g.blockn + i0;
-            const int sidx = (int)(pos / d.neblock);
-            const int64_t so = pos - (int64_t)sidx * d.neblock;
-            const StreamDesc q = s[sidx];
-            uint8_t *pl = planes + j * TILE;
-            if (q.kind == SK_RUN) {
-                for (int x = threadIdx.x; x < cnt; x += blockDim.x) pl[x] = (uint8_t)q.len;
-            } else if (q.kind == SK_RAW) {
-                const uint8_t *src = ch + q.src + so;
-                for (int x = threadIdx.x; x < cnt; x += blockDim.x) pl[x] = __ldg(src + x);
-            } else {
-                const uint8_t *src = blk_scratch + (int64_t)sidx * d.neblock + so;
-                for (int x = threadIdx.x; x < cnt; x += blockDim.x) pl[x] = __ldcg(src + x);
-            }
-        }
-    } else if (d.mode == BM_PLAIN) {
-        for (int x = threadIdx.x; x < cnt * ts; x += blockDim.x) {
-            const int64_t pos = i0 * ts + x;
-            const int sidx = (int)(pos / d.neblock);
-            const int64_t so = pos - (int64_t)sidx * d.neblock;
-            const StreamDesc q = s[sidx];
-            uint8_t v;
-            if (q.kind == SK_RUN) v = (uint8_t)q.len;
-            else if (q.kind == SK_RAW) v = __ldg(ch + q.src + so);
-            else v = __ldcg(blk_scratch + (int64_t)sidx * d.neblock + so);
-            planes[x] = v;
-        }
-    }
-    __syncthreads();
-    for (int x = threadIdx.x; x < cnt; x += blockDim.x) {
-        int64_t row, col;
-        if (!item_pos(g, c, b, i0 + x, row, col)) continue;
-        uint8_t *o = out + (row * ld + col) * ts;
-        uint64_t v = 0;
-        if (d.mode == BM_SHUFFLED) {
-            for (int j = 0; j < ts; j++) v |= (uint64_t)planes[j * TILE + x] << (8 * j);
-        } else if (d.mode == BM_PLAIN) {
-            for (int j = 0; j < ts; j++) v |= (uint64_t)planes[x * ts + j] << (8 * j);
-        } else if (d.mode == BM_NAN) {
-            v = ts == 8 ? 0x7FF8000000000000ull : 0x7FC00000ull;
-        } else {
-            v = load_item_bytes(ch + d.value_src, ts);
-        }
-        store_item(o, ts, v);
-    }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(256) k_scatter(Geom g, const int *__restrict__ rest, const int *__restrict__ nrest,
-                                                 const uint8_t *__restrict__ ch,
+__global__ void __launch_bounds__(256) k_scatter(Geom g, int fast_streams, const uint8_t *__restrict__ ch,
                                                  const BlockDesc *__restrict__ bd, const StreamDesc *__restrict__ sd,
                                                  const uint8_t *__restrict__ scratch, uint8_t *__restrict__ out, int64_t ld)
 {
     __shared__ __align__(16) uint8_t planes[8 * TILE];
     const int64_t tpb = (g.blockn + TILE - 1) / TILE;
-    const int64_t nwork = (rest ? (int64_t)*nrest : g.nchunks * g.nblocks) * tpb;
-    for (int64_t w = blockIdx.x; w < nwork; w += gridDim.x) {
-        const int64_t k = w / tpb, t = rest ? rest[k] : k, i0 = (w - k * tpb) * TILE;
-        scatter_tile(g, ch, bd, sd, scratch, out, ld, t, i0, planes);
+    const int64_t nwork = g.nchunks * g.nblocks * tpb;
+    // Up to 32 tiles are looked at together, a lane each, the same in every warp: where k_scatter_fast
+    // took them all, that look is the whole kernel.  The groups are an even division of a CTA's
+    // share, for where it took none.
+    const int64_t share = (nwork + gridDim.x - 1) / gridDim.x, rounds = (share + 31) / 32;
+    const int group = (int)((share + rounds - 1) / rounds);
+    const int lane = threadIdx.x & 31;
+    for (int64_t w0 = (int64_t)blockIdx.x * group; w0 < nwork; w0 += (int64_t)gridDim.x * group) {
+        int64_t t = 0, i0 = 0;
+        bool mine = lane < group && w0 + lane < nwork;
+        if (mine) {
+            divmod(w0 + lane, tpb, t, i0);
+            mine = !(bd[t].mode == BM_SHUFFLED && bd[t].nstreams == fast_streams);
+        }
+        for (unsigned m = __ballot_sync(FULLMASK, mine); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            scatter_tile(g, ch, bd, sd, scratch, out, ld, __shfl_sync(FULLMASK, t, l), __shfl_sync(FULLMASK, i0, l) * TILE,
+                         planes);
+        }
     }
 }
 
@@ -972,12 +1064,11 @@ __global__ void __launch_bounds__(256) k_scatter(Geom g, const int *__restrict__
 // row and writes one 4-byte word into each byte plane of the image.  Other blocks, whose planes
 // may start at any byte: one item per thread, a byte into each plane, the bytes of a warp
 // next to each other (5000 x 6000 float32 in blocks of 125 x 150: 0.13 ms, 0.29 by the
-// general path).  In slices of SC_ITEMS items, so that a few large blocks spread over the SMs.
+// general path).  In slices of GA_ITEMS items, so that a few large blocks spread over the SMs.
 template <int TS>
 __device__ __forceinline__ void gather_fast_block(const Geom &g, const uint8_t *__restrict__ in, int64_t ld,
-                                                  uint8_t *__restrict__ img, int64_t t, int sl)
+                                                  uint8_t *__restrict__ img, int64_t t, int i0s, int cnt)
 {
-    const int i0s = sl * SC_ITEMS, cnt = (int)min((int64_t)SC_ITEMS, g.blockn - i0s);
     int64_t c, b;
     divmod(t, g.nblocks, c, b);
     const BlockSpan sp = block_span(g, c, b);
@@ -1036,11 +1127,11 @@ template <int TS>
 __global__ void __launch_bounds__(256) k_gather_fast(Geom g, const uint8_t *__restrict__ in, int64_t ld,
                                                      uint8_t *__restrict__ img)
 {
-    const int64_t nsl = (g.blockn + SC_ITEMS - 1) / SC_ITEMS, nu = g.nchunks * g.nblocks * nsl;
+    const int64_t nsl = (g.blockn + GA_ITEMS - 1) / GA_ITEMS, nu = g.nchunks * g.nblocks * nsl;
     for (int64_t u = blockIdx.x; u < nu; u += gridDim.x) {
         int64_t t, sl;
         divmod(u, nsl, t, sl);
-        gather_fast_block<TS>(g, in, ld, img, t, (int)sl);
+        gather_fast_block<TS>(g, in, ld, img, t, (int)sl * GA_ITEMS, (int)min((int64_t)GA_ITEMS, g.blockn - sl * GA_ITEMS));
     }
 }
 
@@ -2214,23 +2305,16 @@ __device__ __forceinline__ void layout_chunk(const Geom &g, int nstreams, int ne
     }
 }
 
-__global__ void __launch_bounds__(LAYOUT_T) k_layout(Geom g, int nstreams, int neblock, EncStream *es, EncChunk *ec,
-                                                    int memcpy_only)
+// Chunk offsets: exclusive scan of the chunk sizes (one CTA); off / len (optional): the chunk
+// index as the decoder reads it.
+__device__ __forceinline__ void chunk_offsets(int64_t nchunks, EncChunk *ec, int64_t *total, int64_t *off, int32_t *len,
+                                              int64_t *wsum)
 {
-    __shared__ int64_t wsum[LAYOUT_T / 32];
-    __shared__ int64_t s_before;
-    __shared__ int s_first;
-    layout_chunk(g, nstreams, neblock, es, ec, memcpy_only, blockIdx.x, wsum, s_before, s_first);
-}
-
-// Chunk offsets: exclusive scan of the chunk sizes (one CTA).
-__device__ __forceinline__ void chunk_offsets(int64_t nchunks, EncChunk *ec, int64_t *total, int64_t *wsum)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)blockDim.x >> 5;
     int64_t base = 0;
-    for (int64_t r0 = 0; r0 < nchunks; r0 += 1024) {
+    for (int64_t r0 = 0; r0 < nchunks; r0 += blockDim.x) {
         const int64_t i = r0 + threadIdx.x;
-        const int64_t v = i < nchunks ? ec[i].cbytes : 0;
+        const int32_t v = i < nchunks ? __ldcg(&ec[i].cbytes) : 0;
         int64_t incl = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -2240,21 +2324,37 @@ __device__ __forceinline__ void chunk_offsets(int64_t nchunks, EncChunk *ec, int
         if (lane == 31) wsum[warp] = incl;
         __syncthreads();
         int64_t before = base + incl - v, all = 0;
-        for (int w = 0; w < 32; w++) {
+        for (int w = 0; w < warps; w++) {
             before += w < warp ? wsum[w] : 0;
             all += wsum[w];
         }
-        if (i < nchunks) ec[i].offset = before;
+        if (i < nchunks) {
+            ec[i].offset = before;
+            if (off) { off[i] = before; len[i] = v; }
+        }
         base += all;
         __syncthreads();
     }
     if (threadIdx.x == 0) *total = base;
 }
 
-__global__ void __launch_bounds__(1024) k_chunk_offsets(int64_t nchunks, EncChunk *ec, int64_t *total)
+// One CTA per chunk; the last one to finish (tot[2] counts them) adds the chunks' offsets: no
+// launch of its own, and no upload of the index by the host.
+__global__ void __launch_bounds__(LAYOUT_T) k_layout(Geom g, int nstreams, int neblock, EncStream *es, EncChunk *ec,
+                                                    int memcpy_only, int64_t *tot, int64_t *off, int32_t *len)
 {
-    __shared__ int64_t wsum[32];
-    chunk_offsets(nchunks, ec, total, wsum);
+    __shared__ int64_t wsum[LAYOUT_T / 32];
+    __shared__ int64_t s_before;
+    __shared__ int s_first;
+    layout_chunk(g, nstreams, neblock, es, ec, memcpy_only, blockIdx.x, wsum, s_before, s_first);
+    if (threadIdx.x == 0) {                        // (thread 0 wrote the chunk's size)
+        __threadfence();
+        s_first = atomicAdd(reinterpret_cast<unsigned long long *>(tot + 2), 1ull) + 1 == gridDim.x;
+    }
+    __syncthreads();
+    if (!s_first) return;
+    __threadfence();
+    chunk_offsets(g.nchunks, ec, tot, off, len, wsum);
 }
 
 // Copies len bytes with the whole CTA: 16-byte aligned stores to dst, each fed by five
@@ -2386,6 +2486,23 @@ int decode_container(const Geom &g, const uint8_t *d_chunks, int64_t chunks_byte
     return decode_finish(&w, st);
 }
 
+int decode_finish_queue(DecodeQueue *q, DecodeWork *const *w, int n, cudaStream_t st)
+{
+    int h[64];
+    const int slots = q->slots;
+    if (slots < 0 || (slots + 1) * 16 > 64) return -101;
+    cudaMemcpyAsync(h, q->counters.p, 64 * (size_t)(slots + 1), cudaMemcpyDeviceToHost, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return -101;
+    int r = 0;
+    for (int k = 0; k < n; k++) {
+        const int64_t at = w[k]->ext_counters ? w[k]->ext_counters - q->counters.as<int>() : 0;
+        if (at < 16 || at > 16 * slots) return -101;
+        w[k]->nzero = h[at + 4];
+        if (!r) r = h[at + 1];
+    }
+    return r;
+}
+
 int decode_finish(DecodeWork *w, cudaStream_t st)
 {
     int h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -2403,7 +2520,7 @@ static int64_t scatter_fast_grid(const Geom &g, int64_t nbl)
     static int per_sm = 0;
     if (!per_sm) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_scatter_fast<TS>, 256, 0) != cudaSuccess || n < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_scatter_fast<TS, true>, 256, 0) != cudaSuccess || n < 1) {
             cudaGetLastError();
             n = 4;
         }
@@ -2415,14 +2532,17 @@ static int64_t scatter_fast_grid(const Geom &g, int64_t nbl)
 
 int64_t decode_max_jobs(const Geom &g) { return g.nchunks * g.nblocks * 8; }
 
-int decode_queue_init(DecodeQueue *q, int64_t max_jobs, cudaStream_t st)
+int decode_queue_init(DecodeQueue *q, int64_t max_jobs, int slots, cudaStream_t st)
 {
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!q->jobs.allocate(sizeof(Lz4Job) * (size_t)std::max<int64_t>(max_jobs, 1), dev) || !q->counters.allocate(64, dev))
+    const size_t bytes = 64 * (size_t)(1 + slots);
+    if (!q->jobs.allocate(sizeof(Lz4Job) * (size_t)std::max<int64_t>(max_jobs, 1), dev) || !q->counters.allocate(bytes, dev))
         return -100;
     q->cap = max_jobs;
-    cudaMemsetAsync(q->counters.p, 0, 64, st);
+    q->slots = slots;
+    q->used = 0;
+    cudaMemsetAsync(q->counters.p, 0, bytes, st);
     return 0;
 }
 
@@ -2433,10 +2553,15 @@ int decode_parse(const DecodeArgs &a, DecodeQueue *q, DecodeWork *w, cudaStream_
     const Geom &g = a.g;
     const int64_t nbl = g.nchunks * g.nblocks;
     if (!w->bd.allocate(sizeof(BlockDesc) * nbl, dev) || !w->sd.allocate(sizeof(StreamDesc) * nbl * 8, dev) ||
-        !w->scratch.allocate((size_t)(nbl * g.blocksize), dev) || (!w->ext_counters && !w->counters.allocate(64, dev)))
+        !w->scratch.allocate((size_t)(nbl * g.blocksize), dev))
         return -100;
+    if (!w->ext_counters && q->used < q->slots) {
+        w->ext_counters = q->counters.as<int>() + 16 * ++q->used;      // zeroed with the queue's counters
+    } else {
+        if (!w->ext_counters && !w->counters.allocate(64, dev)) return -100;
+        cudaMemsetAsync(w->ext_counters ? (void *)w->ext_counters : w->counters.p, 0, 64, st);
+    }
     int *cnt = w->ext_counters ? w->ext_counters : w->counters.as<int>();
-    cudaMemsetAsync(cnt, 0, 64, st);
     const int threads = 128;
     const int64_t blocks = std::min<int64_t>((nbl + threads - 1) / threads, (int64_t)sm_count() * 16);
     if (!w->zf.allocate((size_t)std::max<int64_t>(nbl, 1), dev)) return -100;
@@ -2456,38 +2581,49 @@ int decode_lz4(DecodeQueue *q, cudaStream_t st)
     }
     int *qc = q->counters.as<int>();
     IAB_TIMED("k_lz4_decode_cta", st, k_lz4_decode_cta<<<sm_count() * 6, dcta::THREADS, smem, st>>>(
-        q->jobs.as<Lz4Job>(), qc, q->cap, reinterpret_cast<unsigned *>(qc + 1)));
+        q->jobs.as<Lz4Job>(), qc, q->cap, reinterpret_cast<unsigned *>(qc + 8)));
     return 0;
+}
+
+// The decoded streams to the dense array.  Small containers by one launch, the blocks the fast
+// path does not take included; from SC_SPLIT bytes on those have a launch of their own, because
+// the registers of the kernel that holds both paths spill: 0.81 against 0.86 ms for three 512 MiB
+// float64 arrays, where the launch that mostly finds nothing costs 6 us.  Items of 1 and 2 bytes
+// go by the general path.
+constexpr int64_t SC_SPLIT = int64_t(64) << 20;
+template <int TS>
+static void scatter_launch(const Geom &g, bool all, const uint8_t *chunks, const uint8_t *cend, const BlockDesc *bd,
+                           const StreamDesc *sd, const uint8_t *scratch, const uint8_t *send, void *out, int64_t ld, int *err,
+                           cudaStream_t st)
+{
+    const unsigned grid = (unsigned)scatter_fast_grid<TS>(g, g.nchunks * g.nblocks);
+    if (all)
+        IAB_TIMED("k_scatter_fast", st, k_scatter_fast<TS, true><<<grid, 256, 0, st>>>(
+            g, chunks, cend, bd, sd, scratch, send, (uint8_t *)out, ld, err));
+    else
+        IAB_TIMED("k_scatter_fast", st, k_scatter_fast<TS, false><<<grid, 256, 0, st>>>(
+            g, chunks, cend, bd, sd, scratch, send, (uint8_t *)out, ld, err));
+}
+static void scatter_launch(const Geom &g, const uint8_t *chunks, int64_t chunks_bytes, const BlockDesc *bd, const StreamDesc *sd,
+                           const uint8_t *scratch, void *out, int64_t ld, int *err, cudaStream_t st)
+{
+    const int64_t nbl = g.nchunks * g.nblocks;
+    const uint8_t *cend = chunks + chunks_bytes, *send = scratch + nbl * g.blocksize;
+    const bool fast = g.itemsize == 8 || g.itemsize == 4, all = fast && nbl * g.blocksize < SC_SPLIT;
+    if (g.itemsize == 8) scatter_launch<8>(g, all, chunks, cend, bd, sd, scratch, send, out, ld, err, st);
+    else if (g.itemsize == 4) scatter_launch<4>(g, all, chunks, cend, bd, sd, scratch, send, out, ld, err, st);
+    if (!all) {
+        const int64_t blocks = std::min<int64_t>(nbl * ceil_div(g.blockn, TILE), (int64_t)sm_count() * 8);
+        IAB_TIMED("k_scatter", st, k_scatter<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
+            g, fast ? g.itemsize : 0, chunks, bd, sd, scratch, (uint8_t *)out, ld));
+    }
 }
 
 int decode_scatter(const DecodeArgs &a, DecodeWork *w, cudaStream_t st)
 {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const Geom &g = a.g;
-    const int64_t nbl = g.nchunks * g.nblocks;
     int *cnt = w->ext_counters ? w->ext_counters : w->counters.as<int>();
-    const int sms = sm_count();
-    const uint8_t *scratch = w->scratch.as<uint8_t>();
-    const int64_t tpb = (g.blockn + TILE - 1) / TILE;
-    const int64_t blocks = std::min<int64_t>(nbl * tpb, (int64_t)sms * 8);
-    const bool fast = g.itemsize == 4 || g.itemsize == 8;
-    int *rest = nullptr, *nrest = cnt + 3;
-    if (fast) {
-        if (!w->rest.allocate(sizeof(int) * (size_t)nbl, dev)) return -100;
-        rest = w->rest.as<int>();
-        const uint8_t *cend = a.chunks + a.chunks_bytes, *send = scratch + nbl * g.blocksize;
-        if (g.itemsize == 8)
-            IAB_TIMED("k_scatter_fast", st, k_scatter_fast<8><<<(unsigned)scatter_fast_grid<8>(g, nbl), 256, 0, st>>>(
-                g, a.chunks, cend, w->bd.as<BlockDesc>(), w->sd.as<StreamDesc>(), scratch, send, (uint8_t *)a.out, a.ld,
-                rest, nrest, cnt + 1));
-        else
-            IAB_TIMED("k_scatter_fast", st, k_scatter_fast<4><<<(unsigned)scatter_fast_grid<4>(g, nbl), 256, 0, st>>>(
-                g, a.chunks, cend, w->bd.as<BlockDesc>(), w->sd.as<StreamDesc>(), scratch, send, (uint8_t *)a.out, a.ld,
-                rest, nrest, cnt + 1));
-    }
-    IAB_TIMED("k_scatter", st, k_scatter<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
-        g, rest, nrest, a.chunks, w->bd.as<BlockDesc>(), w->sd.as<StreamDesc>(), scratch, (uint8_t *)a.out, a.ld));
+    scatter_launch(a.g, a.chunks, a.chunks_bytes, w->bd.as<BlockDesc>(), w->sd.as<StreamDesc>(), w->scratch.as<uint8_t>(),
+                   a.out, a.ld, cnt + 1, st);
     return 0;
 }
 
@@ -2495,7 +2631,7 @@ int decode_launch(const Geom &g, const uint8_t *d_chunks, int64_t chunks_bytes, 
                   int64_t ld, cudaStream_t st, DecodeWork *w)
 {
     const DecodeArgs a{g, d_chunks, chunks_bytes, d_off, d_len, out, ld};
-    int r = decode_queue_init(&w->queue, decode_max_jobs(g), st);
+    int r = decode_queue_init(&w->queue, decode_max_jobs(g), 1, st);
     if (!r) r = decode_parse(a, &w->queue, w, st);
     if (!r) r = decode_lz4(&w->queue, st);
     if (!r) r = decode_scatter(a, w, st);
@@ -2539,7 +2675,7 @@ int encode_gather(const Geom &g, const void *in, int64_t ld, bool shuffle, int s
     const int64_t blocks = std::min<int64_t>(nbl * tpb, (int64_t)sms * 8);
     const bool fast = shuffle && (ts == 4 || ts == 8);
     if (fast) {
-        const int64_t fb = std::min<int64_t>(nbl * ceil_div(g.blockn, SC_ITEMS), (int64_t)sms * 8);
+        const int64_t fb = std::min<int64_t>(nbl * ceil_div(g.blockn, GA_ITEMS), (int64_t)sms * 8);
         if (ts == 8)
             IAB_TIMED("k_gather_fast", st, k_gather_fast<8><<<(unsigned)std::max<int64_t>(fb, 1), 256, 0, st>>>(
                 g, (const uint8_t *)in, ld, img));
@@ -2595,9 +2731,12 @@ int encode_emit(const Geom &g, bool shuffle, int splitmode, DevBuf *d_out, Encod
     const uint8_t *slots = ext ? w->ext_slots : w->slots.as<uint8_t>();
     EncStream *es = ext ? w->ext_es : w->es.as<EncStream>();
     EncChunk *ec = w->ext_chunks ? w->ext_chunks : w->ec.as<EncChunk>();
+    if (!w->d_off.allocate(sizeof(int64_t) * (size_t)std::max<int64_t>(g.nchunks, 1), dev) ||
+        !w->d_len.allocate(sizeof(int32_t) * (size_t)std::max<int64_t>(g.nchunks, 1), dev))
+        return -100;
     IAB_TIMED("k_layout", st, k_layout<<<(unsigned)std::max<int64_t>(g.nchunks, 1), LAYOUT_T, 0, st>>>(
-        g, nstreams, neblock, es, ec, w->memcpy_only ? 1 : 0));
-    IAB_TIMED("k_chunk_offsets", st, k_chunk_offsets<<<1, 1024, 0, st>>>(g.nchunks, ec, w->tot.as<int64_t>()));
+        g, nstreams, neblock, es, ec, w->memcpy_only ? 1 : 0, w->tot.as<int64_t>(), w->d_off.as<int64_t>(),
+        w->d_len.as<int32_t>()));
     const int64_t blocks = std::min<int64_t>(nbl, (int64_t)sm_count() * 8);
     IAB_TIMED("k_emit", st, k_emit<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
         g, nstreams, neblock, shuffle, encode_split(g, shuffle, splitmode) ? 1 : 0, img, slots, img_bytes, es, ec,
@@ -2650,26 +2789,19 @@ int encode_image_prepare(const Geom &g, EncodeWork *w)
 }
 
 int encode_image_finish(const Geom &g, bool shuffle, int splitmode, DevBuf *d_out, std::vector<int64_t> *h_off,
-                        std::vector<int32_t> *h_len, cudaStream_t st, bool exact_lz4, EncodeWork *w)
+                        std::vector<int32_t> *h_len, cudaStream_t st, EncodeWork *w)
 {
     if (!w->img_ready) return -1;
-    w->exact_lz4 = exact_lz4;
     w->memcpy_only = false;
-    const int r = encode_launch(g, nullptr, 0, shuffle, splitmode, d_out, w, st);
-    if (r) return r;
-    return encode_finish(w, h_off, h_len, st);
+    return encode_container(g, nullptr, 0, shuffle, splitmode, d_out, h_off, h_len, st, w);
 }
 
 int encode_container(const Geom &g, const void *in, int64_t ld, bool shuffle, int splitmode, DevBuf *d_out,
-                     std::vector<int64_t> *h_off, std::vector<int32_t> *h_len, cudaStream_t st, bool exact_lz4,
-                     bool memcpy_only)
+                     std::vector<int64_t> *h_off, std::vector<int32_t> *h_len, cudaStream_t st, EncodeWork *w)
 {
-    EncodeWork w;
-    w.exact_lz4 = exact_lz4;
-    w.memcpy_only = memcpy_only;
-    const int r = encode_launch(g, in, ld, shuffle, splitmode, d_out, &w, st);
+    const int r = encode_launch(g, in, ld, shuffle, splitmode, d_out, w, st);
     if (r) return r;
-    return encode_finish(&w, h_off, h_len, st);
+    return encode_finish(w, h_off, h_len, st);
 }
 
 // ============================================================================ decode-fused GEMV
@@ -2979,19 +3111,27 @@ __global__ void k_group_reset(const CodecItem *__restrict__ items, int n)
 __global__ void k_parse_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart, int n, int64_t nbl,
                           Lz4Job *jobs, int *njobs, int64_t jcap)
 {
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nbl; u += (int64_t)gridDim.x * blockDim.x) {
-        const int k = group_find(bstart, n, u);
-        const CodecItem &it = items[k];
-        parse_block(it.g, it.ch, it.off, it.len, it.bd, it.sd, jobs, njobs, jcap, it.cnt + 1, it.scratch, nullptr,
-                    nullptr, u - bstart[k]);
+    for (int64_t u0 = (int64_t)blockIdx.x * blockDim.x; u0 < nbl; u0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t u = u0 + threadIdx.x;
+        ParsedBlock pb;
+        pb.lz = 0;
+        uint8_t *blk = nullptr;
+        int *err = nullptr;
+        if (u < nbl) {
+            const int k = group_find(bstart, n, u);
+            const CodecItem &it = items[k];
+            const int64_t t = u - bstart[k];
+            err = it.cnt + 1;
+            blk = it.scratch + t * it.g.blocksize;
+            parse_block(it.g, it.ch, it.off, it.len, it.bd, it.sd, err, nullptr, nullptr, t, pb);
+        }
+        queue_streams(pb, blk, err, jobs, njobs, jcap);
     }
 }
 
 template <int TS>
 __global__ void __launch_bounds__(256, 4) k_scatter_fast_g(const CodecItem *__restrict__ items,
-                                                        const int64_t *__restrict__ bstart,
-                                                        const int64_t *__restrict__ sstart, int n, int64_t nsf,
-                                                        int *rest, int *nrest)
+                                                        const int64_t *__restrict__ sstart, int n, int64_t nsf)
 {
     __shared__ __align__(128) uint8_t stage[TS][SC_PLANE];
     __shared__ __align__(8) uint64_t bar;
@@ -3004,6 +3144,7 @@ __global__ void __launch_bounds__(256, 4) k_scatter_fast_g(const CodecItem *__re
     }
     __syncthreads();
     uint32_t parity = 0;
+    bool general = false;
     for (int64_t u = blockIdx.x; u < nsf; u += gridDim.x) {
         const int k = group_find(sstart, n, u);
         const CodecItem &it = items[k];
@@ -3012,21 +3153,29 @@ __global__ void __launch_bounds__(256, 4) k_scatter_fast_g(const CodecItem *__re
         const int sl = (int)(lu - t * nsl);
         const int64_t nbk = it.g.nchunks * it.g.nblocks;
         if (!scatter_fast_unit<TS>(it.g, it.ch, it.ch + it.ch_bytes, it.bd, it.sd, it.scratch,
-                                   it.scratch + nbk * it.g.blocksize, it.dense, it.ld, rest, nrest,
-                                   (int)(bstart[k] + t), it.cnt + 1, t, sl, stage, &bar, parity, &abort_all))
+                                   it.scratch + nbk * it.g.blocksize, it.dense, it.ld, it.cnt + 1, t, sl, stage, &bar, parity, &abort_all,
+                                   general))
             return;
+    }
+    for (int64_t u = blockIdx.x; general && u < nsf; u += gridDim.x) {      // as in k_scatter_fast
+        const int k = group_find(sstart, n, u);
+        const CodecItem &it = items[k];
+        int64_t t, sl;
+        divmod(u - sstart[k], (it.g.blockn + SC_ITEMS - 1) / SC_ITEMS, t, sl);
+        if (it.bd[t].mode == BM_SHUFFLED && it.bd[t].nstreams == TS) continue;
+        const int64_t end = min(it.g.blockn, (sl + 1) * SC_ITEMS);
+        for (int64_t i0 = sl * SC_ITEMS; i0 < end; i0 += TILE)
+            scatter_tile(it.g, it.ch, it.bd, it.sd, it.scratch, it.dense, it.ld, t, i0, stage[0]);
     }
 }
 
-// General scatter over the listed blocks (global block numbers), or every block without a list.
+// General scatter over every block.
 __global__ void __launch_bounds__(256) k_scatter_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart,
-                                                   int n, const int *__restrict__ rest, const int *__restrict__ nrest,
-                                                   int64_t nbl, int64_t tpb)
+                                                   int n, int64_t nbl, int64_t tpb)
 {
     __shared__ __align__(16) uint8_t planes[8 * TILE];
-    const int64_t nwork = (rest ? (int64_t)*nrest : nbl) * tpb;
-    for (int64_t w = blockIdx.x; w < nwork; w += gridDim.x) {
-        const int64_t kk = w / tpb, gb = rest ? rest[kk] : kk, i0 = (w - kk * tpb) * TILE;
+    for (int64_t w = blockIdx.x; w < nbl * tpb; w += gridDim.x) {
+        const int64_t gb = w / tpb, i0 = (w - gb * tpb) * TILE;
         const int k = group_find(bstart, n, gb);
         const CodecItem &it = items[k];
         if (i0 >= it.g.blockn) continue;
@@ -3036,14 +3185,12 @@ __global__ void __launch_bounds__(256) k_scatter_g(const CodecItem *__restrict__
 
 template <int TS>
 __global__ void __launch_bounds__(256) k_gather_fast_g(const CodecItem *__restrict__ items,
-                                                       const int64_t *__restrict__ sstart, int n, int64_t nsf)
+                                                       const int64_t *__restrict__ bstart, int n, int64_t nbl)
 {
-    for (int64_t u = blockIdx.x; u < nsf; u += gridDim.x) {
-        const int k = group_find(sstart, n, u);
+    for (int64_t u = blockIdx.x; u < nbl; u += gridDim.x) {
+        const int k = group_find(bstart, n, u);
         const CodecItem &it = items[k];
-        int64_t t, sl;
-        divmod(u - sstart[k], (it.g.blockn + SC_ITEMS - 1) / SC_ITEMS, t, sl);
-        gather_fast_block<TS>(it.g, it.dense, it.ld, it.img, t, (int)sl);
+        gather_fast_block<TS>(it.g, it.dense, it.ld, it.img, u - bstart[k], 0, (int)it.g.blockn);
     }
 }
 
@@ -3077,7 +3224,7 @@ __global__ void __launch_bounds__(1024) k_chunk_offsets_g(CodecItem *items)
 {
     __shared__ int64_t wsum[32];
     CodecItem &it = items[blockIdx.x];
-    chunk_offsets(it.g.nchunks, it.ec, &it.out_bytes, wsum);
+    chunk_offsets(it.g.nchunks, it.ec, &it.out_bytes, nullptr, nullptr, wsum);
 }
 
 __global__ void __launch_bounds__(256) k_emit_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart,
@@ -3137,10 +3284,9 @@ int decode_group_setup(const std::vector<DecodeArgs> &a, const std::vector<int *
     }
     if (!grp->bd.allocate(sizeof(BlockDesc) * (size_t)std::max<int64_t>(nbl, 1), dev) ||
         !grp->sd.allocate(sizeof(StreamDesc) * 8 * (size_t)std::max<int64_t>(nbl, 1), dev) ||
-        !grp->scratch.allocate((size_t)std::max<int64_t>(img, 16), dev) ||
-        !grp->rest.allocate(sizeof(int) * (size_t)std::max<int64_t>(nbl, 1), dev) || !grp->counters.allocate(128, dev))
+        !grp->scratch.allocate((size_t)std::max<int64_t>(img, 16), dev))
         return -100;
-    int r = decode_queue_init(&grp->q, jobs, st);
+    int r = decode_queue_init(&grp->q, jobs, 0, st);
     if (r) return r;
     grp->h.assign((size_t)n, CodecItem{});
     int64_t bo = 0, io = 0;
@@ -3166,9 +3312,7 @@ int decode_group_launch(CodecGroup *grp, cudaStream_t st)
     const int n = grp->n, sms = sm_count();
     const CodecItem *items = grp->items.as<CodecItem>();
     const int64_t *bstart = grp->starts.as<int64_t>(), *sstart = bstart + (n + 1);
-    int *gc = grp->counters.as<int>();
     cudaMemsetAsync(grp->q.counters.p, 0, 64, st);
-    cudaMemsetAsync(gc, 0, 128, st);
     IAB_TIMED("k_group_reset", st, k_group_reset<<<(unsigned)((n * 16 + 255) / 256), 256, 0, st>>>(items, n));
     if (grp->nbl == 0) return 0;
     const int64_t pb = std::min<int64_t>((grp->nbl + 127) / 128, (int64_t)sms * 16);
@@ -3190,14 +3334,16 @@ int decode_group_launch(CodecGroup *grp, cudaStream_t st)
         const int64_t grid = std::max<int64_t>(std::min<int64_t>(grp->nsf, (int64_t)sms * per_sm[slot]), 1);
         if (slot)
             IAB_TIMED("k_scatter_fast", st, k_scatter_fast_g<8><<<(unsigned)grid, 256, 0, st>>>(
-                items, bstart, sstart, n, grp->nsf, grp->rest.as<int>(), gc));
+                items, sstart, n, grp->nsf));
         else
             IAB_TIMED("k_scatter_fast", st, k_scatter_fast_g<4><<<(unsigned)grid, 256, 0, st>>>(
-                items, bstart, sstart, n, grp->nsf, grp->rest.as<int>(), gc));
+                items, sstart, n, grp->nsf));
     }
-    const int64_t sb = std::min<int64_t>(grp->nbl * grp->max_tpb, (int64_t)sms * 8);
-    IAB_TIMED("k_scatter", st, k_scatter_g<<<(unsigned)std::max<int64_t>(sb, 1), 256, 0, st>>>(
-        items, bstart, n, fast ? grp->rest.as<int>() : nullptr, fast ? gc : nullptr, grp->nbl, grp->max_tpb));
+    if (!fast) {
+        const int64_t sb = std::min<int64_t>(grp->nbl * grp->max_tpb, (int64_t)sms * 8);
+        IAB_TIMED("k_scatter", st, k_scatter_g<<<(unsigned)std::max<int64_t>(sb, 1), 256, 0, st>>>(
+            items, bstart, n, grp->nbl, grp->max_tpb));
+    }
     return 0;
 }
 
@@ -3259,11 +3405,10 @@ int encode_group_launch(CodecGroup *grp, bool exact_lz4, bool memcpy_only, cudaS
     const bool fast = grp->shuffle && (ts == 4 || ts == 8);
     const int64_t gb = std::max<int64_t>(std::min<int64_t>(grp->nbl, (int64_t)sms * 8), 1);
     if (fast && !grp->img_ready) {
-        const int64_t fb = std::max<int64_t>(std::min<int64_t>(grp->nsf, (int64_t)sms * 8), 1), *sstart = bstart + (n + 1);
         if (ts == 8)
-            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<8><<<(unsigned)fb, 256, 0, st>>>(items, sstart, n, grp->nsf));
+            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<8><<<(unsigned)gb, 256, 0, st>>>(items, bstart, n, grp->nbl));
         else
-            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<4><<<(unsigned)fb, 256, 0, st>>>(items, sstart, n, grp->nsf));
+            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<4><<<(unsigned)gb, 256, 0, st>>>(items, bstart, n, grp->nbl));
     }
     if (!fast && !grp->img_ready) {
         const int64_t tb = std::max<int64_t>(std::min<int64_t>(grp->nbl * grp->max_tpb, (int64_t)sms * 8), 1);
@@ -3299,8 +3444,7 @@ constexpr size_t NA_LEN = na_align(NA_OFF + sizeof(int64_t) * NA_MAX_BLOCKS);
 constexpr size_t NA_BD = na_align(NA_LEN + sizeof(int32_t) * NA_MAX_BLOCKS);
 constexpr size_t NA_SD = na_align(NA_BD + sizeof(BlockDesc) * NA_MAX_BLOCKS);
 constexpr size_t NA_JOBS = na_align(NA_SD + sizeof(StreamDesc) * 8 * NA_MAX_BLOCKS);
-constexpr size_t NA_REST = na_align(NA_JOBS + sizeof(Lz4Job) * 8 * NA_MAX_BLOCKS);
-constexpr size_t NA_IMG = na_align(NA_REST + sizeof(int) * NA_MAX_BLOCKS);
+constexpr size_t NA_IMG = na_align(NA_JOBS + sizeof(Lz4Job) * 8 * NA_MAX_BLOCKS);
 constexpr size_t NA_TOTAL = NA_IMG + (size_t)NOALLOC_MAX_BYTES;
 
 static __device__ __align__(256) uint8_t g_noalloc_scratch[NA_TOTAL];
@@ -3359,7 +3503,7 @@ int decode_noalloc(const Geom &g, const uint8_t *d_chunks, int64_t chunks_bytes,
     StreamDesc *sd = reinterpret_cast<StreamDesc *>(base + NA_SD);
     Lz4Job *jobs = reinterpret_cast<Lz4Job *>(base + NA_JOBS);
     uint8_t *img = base + NA_IMG;
-    int *njobs = counters, *err = counters + 1;
+    int *njobs = counters, *err = counters + 9;
     // the job count, the status word and the job cursor must start at zero; descriptors,
     // the chunk index and the image are fully rewritten before they are read
     if (cudaMemsetAsync(counters, 0, 64, st) != cudaSuccess) return -101;
@@ -3374,25 +3518,9 @@ int decode_noalloc(const Geom &g, const uint8_t *d_chunks, int64_t chunks_bytes,
     }
     {
         IAB_TIMED("k_lz4_decode_cta", st, k_lz4_decode_cta<<<sms * 6, dcta::THREADS, (int)sizeof(dcta::Smem), st>>>(
-            jobs, njobs, 8 * NA_MAX_BLOCKS, reinterpret_cast<unsigned *>(counters + 2)));
+            jobs, njobs, 8 * NA_MAX_BLOCKS, reinterpret_cast<unsigned *>(counters + 8)));
     }
-    {
-        const int64_t tpb = (g.blockn + TILE - 1) / TILE;
-        const int64_t blocks = std::min<int64_t>(nbl * tpb, (int64_t)sms * 8);
-        const bool fast = g.itemsize == 4 || g.itemsize == 8;
-        int *rest = fast ? reinterpret_cast<int *>(base + NA_REST) : nullptr, *nrest = counters + 3;
-        if (fast) {
-            const uint8_t *cend = d_chunks + chunks_bytes, *send = img + nbl * g.blocksize;
-            if (g.itemsize == 8)
-                IAB_TIMED("k_scatter_fast", st, k_scatter_fast<8><<<(unsigned)scatter_fast_grid<8>(g, nbl), 256, 0, st>>>(
-                    g, d_chunks, cend, bd, sd, img, send, (uint8_t *)out, ld, rest, nrest, err));
-            else
-                IAB_TIMED("k_scatter_fast", st, k_scatter_fast<4><<<(unsigned)scatter_fast_grid<4>(g, nbl), 256, 0, st>>>(
-                    g, d_chunks, cend, bd, sd, img, send, (uint8_t *)out, ld, rest, nrest, err));
-        }
-        IAB_TIMED("k_scatter", st, k_scatter<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
-            g, rest, nrest, d_chunks, bd, sd, img, (uint8_t *)out, ld));
-    }
+    scatter_launch(g, d_chunks, chunks_bytes, bd, sd, img, out, ld, err, st);
     // a launch that failed (a bad configuration, or an error left by earlier work) never
     // wrote the status word: report it instead of the zero it still holds
     if (cudaPeekAtLastError() != cudaSuccess) return -101;

@@ -163,16 +163,18 @@ struct DecodeArgs {
     int64_t ld;             // its leading dimension in items
 };
 struct DecodeQueue {
-    DevBuf jobs, counters;  // counters: [0] jobs queued, [1] the next job to hand out
+    DevBuf jobs, counters;  // jobs: a region of cap / 8 for each stream number; counters:
+                            // [0..7] jobs in each, [8] the next job to hand out; then 16 ints per slot
     int64_t cap = 0;
+    int slots = 0, used = 0;   // status slots for containers without their own, handed out by decode_parse
 };
 // Asynchronous form: decode_launch enqueues the kernels on `st` (work buffers held in
 // *w until decode_finish, which synchronises `st` and returns the DevErr).
 struct DecodeWork {
-    DevBuf bd, sd, scratch, counters, rest;
+    DevBuf bd, sd, scratch, counters;
     DevBuf zf;                     // per (chunk, block) zero flags of the block-pair products (k_parse)
     DecodeQueue queue;             // the job queue of decode_launch (unused by decode_parse / _scatter)
-    int *ext_counters = nullptr;   // optional caller-owned 16-int status slot (device) instead of `counters`
+    int *ext_counters = nullptr;   // 16-int status slot (device) of the caller or of the queue, instead of `counters`
     int nzero = 0;                 // flagged blocks, read back by decode_finish
 };
 int decode_launch(const Geom &g, const uint8_t *d_chunks, int64_t chunks_bytes, const int64_t *d_off, const int32_t *d_len,
@@ -185,7 +187,10 @@ int decode_finish(DecodeWork *w, cudaStream_t st);
 // container (after the LZ4 launch); decode_finish(w) per container as above.  The LZ4
 // streams of all containers are handed out from one queue, so the LZ4 kernel's CTAs stay
 // busy across container boundaries.
-int decode_queue_init(DecodeQueue *q, int64_t max_jobs, cudaStream_t st);
+int decode_queue_init(DecodeQueue *q, int64_t max_jobs, int slots, cudaStream_t st);
+// decode_finish for containers whose status slots are the queue's: one copy for all of them (at
+// most 3); the first error.
+int decode_finish_queue(DecodeQueue *q, DecodeWork *const *w, int n, cudaStream_t st);
 int64_t decode_max_jobs(const Geom &g);
 int decode_parse(const DecodeArgs &a, DecodeQueue *q, DecodeWork *w, cudaStream_t st);
 int decode_lz4(DecodeQueue *q, cudaStream_t st);
@@ -214,18 +219,20 @@ inline bool noalloc_fits(const Geom &g)
 }
 int decode_noalloc(const Geom &g, const uint8_t *d_chunks, int64_t chunks_bytes, void *out, int64_t ld, cudaStream_t st);
 
-// Encode a dense row-major array into Blosc2 chunks.  On return *d_out holds the
-// chunks back-to-back, h_off / h_len (host) their offsets and lengths.
-// exact_lz4: streams byte-identical to liblz4 1.9.4 LZ4_compress_fast(acceleration 1); else
+struct EncodeWork;
+// Encode a dense row-major array into Blosc2 chunks.  On return *d_out holds the chunks
+// back-to-back, h_off / h_len (host) and w->d_off / w->d_len (device) their offsets and lengths.
+// w->exact_lz4: streams byte-identical to liblz4 1.9.4 LZ4_compress_fast(acceleration 1); else
 // the parallel-parse encoder (valid LZ4, different bytes).
-// memcpy_only: compression level 0, every chunk stored memcpyed.
+// w->memcpy_only: compression level 0, every chunk stored memcpyed.
 int encode_container(const Geom &g, const void *in, int64_t ld, bool shuffle, int splitmode,
                      DevBuf *d_out, std::vector<int64_t> *h_off, std::vector<int32_t> *h_len,
-                     cudaStream_t st, bool exact_lz4, bool memcpy_only = false);
+                     cudaStream_t st, EncodeWork *w);
 // Asynchronous form: encode_launch enqueues the kernels (no host synchronisation; work
 // buffers held in *w), encode_finish synchronises and reads the chunk table.
 struct EncodeWork {
     DevBuf img, slots, es, ec, tot;
+    DevBuf d_off, d_len;              // the output's chunk index (int64 offsets, int32 lengths)
     bool exact_lz4 = true;            // liblz4-identical streams (see encode_container)
     bool memcpy_only = false;         // compression level 0: every chunk stored memcpyed (c-blosc2's clevel 0)
     bool img_ready = false;           // img already holds the byte-plane image (written by the product)
@@ -245,7 +252,7 @@ int encode_launch(const Geom &g, const void *in, int64_t ld, bool shuffle, int s
 bool encode_image_ok(const Geom &g, bool shuffle, bool memcpy_only);
 int encode_image_prepare(const Geom &g, EncodeWork *w);
 int encode_image_finish(const Geom &g, bool shuffle, int splitmode, DevBuf *d_out, std::vector<int64_t> *h_off,
-                        std::vector<int32_t> *h_len, cudaStream_t st, bool exact_lz4, EncodeWork *w);
+                        std::vector<int32_t> *h_len, cudaStream_t st, EncodeWork *w);
 
 // encode_launch in stages, so that several containers can share one LZ4 launch:
 // encode_gather (dense -> byte-plane image), encode_streams (LZ4 over ns streams of neblock
@@ -289,7 +296,7 @@ struct CodecGroup {
     bool shuffle = true, split = true;     // encode: byte shuffle, one stream per item byte
     std::vector<CodecItem> h;              // host copy of the table
     DevBuf items, starts;                  // device table; starts: blocks, slices, chunks ([n + 1] each)
-    DevBuf bd, sd, scratch, rest, counters;   // decode work shared by the group; counters: [0] rest length, [2..] LZ4 cursor
+    DevBuf bd, sd, scratch, counters;      // work shared by the group; counters: the encode's LZ4 cursor
     DevBuf img, slots, es, outsz;          // encode work shared by the group
     bool img_ready = false;                // encode: the producer writes img itself (no gather)
     DecodeQueue q;
