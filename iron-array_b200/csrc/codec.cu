@@ -1738,7 +1738,9 @@ __global__ void __launch_bounds__(32, XCTAS) k_lz4_encode(const uint8_t *__restr
 //     its bucket among the previous rounds of PT positions (the table keeps the largest
 //     position written, so it is the same whatever the order of the writes), and the
 //     previous position is a second candidate (runs); the longer match is kept, measured
-//     up to PCAP bytes.  Every position enters the table.
+//     up to PCAP bytes.  Every position enters the table.  A round's candidates are loaded
+//     together, 16 bytes each; what is longer is measured by the warp, once for a row of positions
+//     at one distance, and candidates inside runs from the lengths of the two runs.
 //  B. the greedy parse (from the parse position, take the first position with a match of
 //     at least 4 bytes, continue after it) is a chain over match positions: J[q] = the first
 //     match position at or after q + L(q).  The chain is located by pointer doubling (J,
@@ -1746,6 +1748,13 @@ __global__ void __launch_bounds__(32, XCTAS) k_lz4_encode(const uint8_t *__restr
 //     output sizes are prefix-summed across the CTA, and every thread writes its own
 //     sequences.  A chain ends at the window end, after the window's last match, or at a
 //     match of PCAP bytes or more, which is extended exactly before it is written.
+// The bytes of the next window are loaded before B and stored after it; literal runs of more than
+// 16 bytes are copied by a warp.
+// What bounds it: the latency of a window's steps (seven streams an SM, each a chain of some
+// 25,000 cycles per window; 45% of the issue slots), and where zero padding makes every match long,
+// the measuring of lengths, once 46,000 of a window's 68,000 cycles and now 16,000 of 40,000.  A batch
+// of 40 float64 products with extents of 64 to 2048: 14.7 -> 13.2 ms; the 16384 x 16384 float32
+// result of a split product 3.83 -> 3.6 ms.
 // Format rules kept: offsets 1..65535, matches start at least 12 bytes before the end and
 // end at least 5 bytes before it, so the block ends with >= 5 literals.
 constexpr int PW = 1024;
@@ -1792,7 +1801,7 @@ __device__ __forceinline__ int lz4_seq_bytes(int lit, int ml)
 }
 
 // One sequence (literals src[anchor, q), match at q, distance d, length L) at dst + o.
-__device__ __forceinline__ void lz4_put_seq(const EncSrc &s, uint8_t *o, int anchor, int q, int d, int L)
+__device__ __forceinline__ void lz4_put_seq(const EncSrc &s, uint8_t *o, int anchor, int q, int d, int L, bool literals)
 {
     const int lit = q - anchor, ml = L - 4;
     int k = 1;
@@ -1801,7 +1810,8 @@ __device__ __forceinline__ void lz4_put_seq(const EncSrc &s, uint8_t *o, int anc
         for (; rem >= 255; rem -= 255) o[k++] = 255;
         o[k++] = (uint8_t)rem;
     }
-    for (int x = 0; x < lit; x++) o[k + x] = (uint8_t)es_byte(s, anchor + x);
+    if (literals)
+        for (int x = 0; x < lit; x++) o[k + x] = (uint8_t)es_byte(s, anchor + x);
     k += lit;
     o[0] = (uint8_t)(((lit >= 15 ? 15 : lit) << 4) | (ml >= 15 ? 15 : ml));
     o[k] = (uint8_t)d;
@@ -1879,8 +1889,58 @@ __device__ __forceinline__ int cta_lz4_compress_par(const uint8_t *__restrict__ 
     __syncthreads();
     int op = 0, anchor = 0, pos = 0;
     const int mfl1 = n - 11, mlimit = n - 5;
+    int ahead = -1;                                      // where `next` goes (-1: nowhere)
+    uint32_t next[2][2];
+    // Lengths past 16 bytes of the lanes that `need` them (position p, distance d, at most lim; every
+    // lane calls).  A lane whose neighbour has the same distance has one byte more than that one;
+    // for the last of such a row the warp compares 4 bytes a lane, which reaches PCAP.
+    auto extend = [&](bool need, int p, int d, int lim) -> int {
+        const unsigned nm = __ballot_sync(FULLMASK, need);
+        if (!nm) return 0;
+        const int dn = __shfl_down_sync(FULLMASK, d, 1);
+        const unsigned hm = __ballot_sync(FULLMASK, need && !(lane < 31 && ((nm >> (lane + 1)) & 1u) && dn == d));
+        if (__popc(hm) > 6) {                            // every lane by itself
+            int l = 16;
+            while (need && l < lim) {
+                const uint32_t x = par_rd32(ring_s, p + l) ^ (p - d >= s.lo ? par_rd32(ring_s, p - d + l) : ld4u(src + p - d + l));
+                l += x ? (__ffs((int)x) - 1) >> 3 : 4;
+                if (x) break;
+            }
+            return min(l, lim);
+        }
+        const int head = __ffs((int)(hm & (FULLMASK << lane))) - 1;
+        int got = 0;
+        for (unsigned m = hm; m; m &= m - 1) {
+            const int l = __ffs((int)m) - 1;
+            const int ph = __shfl_sync(FULLMASK, p, l), dh = __shfl_sync(FULLMASK, d, l), lh = __shfl_sync(FULLMASK, lim, l);
+            const int a = ph + 16 + 4 * lane;
+            int eq = 0;
+            if (a < ph + lh) {
+                const uint32_t x = par_rd32(ring_s, a) ^ (ph - dh >= s.lo ? par_rd32(ring_s, a - dh) : ld4u(src + a - dh));
+                eq = x ? (__ffs((int)x) - 1) >> 3 : 4;
+            }
+            const int f = __ffs((int)__ballot_sync(FULLMASK, eq < 4)) - 1;   // (at most 28 lanes compare)
+            const int L = min(16 + 4 * f + __shfl_sync(FULLMASK, eq, f), lh);
+            if (head == l) got = L + l - lane;
+        }
+        return min(got, lim);
+    };
     for (int w0 = 0; n >= 13 && w0 < mfl1; w0 += PW) {
         const int wend = min(w0 + PW, mfl1), wn = wend - w0;
+        if (ahead == s.hi) {                             // the bytes loaded during the last window
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int o = (ahead + k * ESEG + tid * 4) & (ERING - 1);
+                const uint32_t v = __funnelshift_r(next[k][0], next[k][1], (uint32_t)(reinterpret_cast<uintptr_t>(src) & 3) * 8);
+                *reinterpret_cast<uint32_t *>(s.r + o) = v;
+                if (o < EMIRROR) *reinterpret_cast<uint32_t *>(s.r + ERING + o) = v;
+            }
+            s.hi = ahead + 2 * ESEG;
+            s.lo = max(s.lo, s.hi - ERING);
+            __syncthreads();
+        }
+        ahead = -1;
         cta_fill(s, wend + PCAP + 32);
         // ---- A: candidates and lengths.  Positions p .. p + PCAP + 4 lie in the window;
         // a candidate is read from the window when it is still there, else from global memory.
@@ -1889,47 +1949,90 @@ __device__ __forceinline__ int cta_lz4_compress_par(const uint8_t *__restrict__ 
         // in one round of PT, so that short streams keep table candidates for most positions.
         for (int q0 = 0, rsz; q0 < PW; q0 += rsz) {
             rsz = w0 + q0 < PT ? 32 : w0 + q0 < 2 * PT ? PT : 2 * PT;
-            int p2[2];
-            bool valid[2];
-            uint32_t v2[2], h2[2], tv2[2];
+            int c2[2];
+            uint32_t v2[2], h2[2], n2[2][3], cw2[2][5];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const int q = q0 + tid + k * PT;
-                p2[k] = w0 + q;
-                valid[k] = tid + k * PT < rsz && p2[k] < wend;
-                v2[k] = valid[k] ? par_rd32(ring_s, p2[k]) : 0u;
+                const int p = w0 + q0 + tid + k * PT;
+                const bool valid = tid + k * PT < rsz && p < wend;
+                const uint32_t o = (uint32_t)p & (ERING - 1), wa = ring_s + (o & ~3u), sh = (o & 3) * 8;
+                const uint32_t a0 = lds32(wa), a1 = lds32(wa + 4), a2 = lds32(wa + 8), a3 = lds32(wa + 12), a4 = lds32(wa + 16);
+                v2[k] = __funnelshift_r(a0, a1, sh);
+                n2[k][0] = __funnelshift_r(a1, a2, sh);
+                n2[k][1] = __funnelshift_r(a2, a3, sh);
+                n2[k][2] = __funnelshift_r(a3, a4, sh);
                 h2[k] = (v2[k] * 2654435761u) >> (32 - 12);
-                tv2[k] = valid[k] ? S.tab32[h2[k]] : 0u;
+                c2[k] = valid ? (int)S.tab32[h2[k]] - 1 : -1;
+            }
+            // 16 bytes at the candidates: all loads of the round are under way together
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int c = max(c2[k], 0);
+                const uint32_t *w = c >= s.lo
+                                        ? reinterpret_cast<const uint32_t *>(S.ring) + ((c & (ERING - 1)) >> 2)
+                                        : reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(src + c) & ~uintptr_t(3));
+#pragma unroll
+                for (int i = 0; i < 5; i++) cw2[k][i] = w[i];
             }
             __syncthreads();                             // every read of this round precedes its writes
 #pragma unroll
-            for (int k = 0; k < 2; k++)
-                if (valid[k]) atomicMax(&S.tab32[h2[k]], (uint32_t)p2[k] + 1u);
+            for (int k = 0; k < 2; k++) {
+                const int p = w0 + q0 + tid + k * PT;
+                if (tid + k * PT < rsz && p < wend) atomicMax(&S.tab32[h2[k]], (uint32_t)p + 1u);
+            }
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const int p = p2[k];
+                const int q = q0 + tid + k * PT, p = w0 + q, cand = c2[k];
+                const bool valid = tid + k * PT < rsz && p < wend;
                 const uint32_t v = v2[k];
-                const int cand = (int)tv2[k] - 1;
-                int L = 0, best = cand;
                 const int lim = min(mlimit - p, PCAP);
-#pragma unroll
-                for (int t = 0; t < 2; t++) {
-                    const int c = t ? p - 1 : cand;
-                    if (!valid[k] || c >= p || c < 0 || p - c > 65535 || (t && c == cand)) continue;
-                    // the previous position matches only inside a run: the 4 bytes at p are equal
-                    if (t && v != (v & 0xFFu) * 0x01010101u) continue;
-                    const bool inring = c >= s.lo;
-                    if ((inring ? par_rd32(ring_s, c) : ld4u(src + c)) != v) continue;
-                    int l = 4;
-                    while (l < lim) {
-                        const uint32_t x = par_rd32(ring_s, p + l) ^ (inring ? par_rd32(ring_s, c + l) : ld4u(src + c + l));
-                        if (x) { l += (__ffs((int)x) - 1) >> 3; break; }
-                        l += 4;
+                const uint32_t sh = (cand >= s.lo ? (uint32_t)cand & 3u
+                                                  : (uint32_t)(reinterpret_cast<uintptr_t>(src + max(cand, 0)) & 3)) * 8;
+                const bool hit = cand >= 0 && p - cand <= 65535 && __funnelshift_r(cw2[k][0], cw2[k][1], sh) == v;
+                const uint32_t x0 = n2[k][0] ^ __funnelshift_r(cw2[k][1], cw2[k][2], sh),
+                               x1 = n2[k][1] ^ __funnelshift_r(cw2[k][2], cw2[k][3], sh),
+                               x2 = n2[k][2] ^ __funnelshift_r(cw2[k][3], cw2[k][4], sh);
+                const uint32_t x = x0 ? x0 : x1 ? x1 : x2;
+                const int len = (x0 ? 4 : x1 ? 8 : 12) + (x ? (__ffs((int)x) - 1) >> 3 : 4);
+                int L = hit ? min(len, lim) : 0, best = cand;
+                bool need = hit && len == 16 && lim > 16;
+                // a run from p on, R bytes equal
+                const bool flat = valid && v == (v & 0xFFu) * 0x01010101u;
+                if (__any_sync(FULLMASK, flat)) {
+                    const uint32_t y0 = n2[k][0] ^ v, y1 = n2[k][1] ^ v, y2 = n2[k][2] ^ v;
+                    const uint32_t y = y0 ? y0 : y1 ? y1 : y2;
+                    int R = min((y0 ? 4 : y1 ? 8 : 12) + (y ? (__ffs((int)y) - 1) >> 3 : 4), lim);
+                    const bool far = flat && !(y0 | y1 | y2) && lim > 16;
+                    const int l = extend(far, p, 1, lim);
+                    if (far) R = l;
+                    // Candidates inside a run: the positions of a round have the same one, each at another
+                    // distance.  The shorter run is the match (two of the same length are compared on).
+                    const bool in = far && need;
+                    for (unsigned m = __ballot_sync(FULLMASK, in); m;) {
+                        const int i = __ffs((int)m) - 1, c = __shfl_sync(FULLMASK, cand, i), a = c + 16 + 4 * lane;
+                        const uint32_t b = __shfl_sync(FULLMASK, v, i);
+                        const unsigned mates = __ballot_sync(FULLMASK, in && cand == c);
+                        int eq = 0;
+                        if (lane < (PCAP - 16) / 4) {
+                            const uint32_t z = (c >= s.lo ? par_rd32(ring_s, a) : ld4u(src + a)) ^ b;
+                            eq = z ? (__ffs((int)z) - 1) >> 3 : 4;
+                        }
+                        const int f = __ffs((int)__ballot_sync(FULLMASK, eq < 4)) - 1;
+                        const int C = 16 + 4 * f + __shfl_sync(FULLMASK, eq, f);
+                        if (((mates >> lane) & 1u) && (R >= lim || C != R)) { L = min(C, R); need = false; }
+                        m &= ~mates;
                     }
-                    l = min(l, lim);
-                    if (l > L) { L = l; best = c; }
+                    const int g = extend(need, p, p - cand, lim);
+                    if (need) L = g;
+                    // the previous position matches too when the byte before p is the run's
+                    if (flat && p > 0 && cand != p - 1 && R > L && S.ring[(p - 1) & (ERING - 1)] == (uint8_t)v) {
+                        L = R;
+                        best = p - 1;
+                    }
+                } else {
+                    const int g = extend(need, p, p - cand, lim);
+                    if (need) L = g;
                 }
-                const int q = q0 + tid + k * PT;
                 if (tid + k * PT < rsz) {
                     S.w.cw[q] = (uint16_t)(p - best);
                     S.w.lw[q] = (uint8_t)L;
@@ -1939,20 +2042,37 @@ __device__ __forceinline__ int cta_lz4_compress_par(const uint8_t *__restrict__ 
             }
             __syncthreads();                             // this round's writes precede the next reads
         }
+        // the next window's bytes, on their way while this one's sequences are found and written
+        if (s.hi + 2 * ESEG + 8 <= n && wend + PW + PCAP + 32 > s.hi) {
+            ahead = s.hi;
+#pragma unroll
+            for (int k = 0; k < 2; k++) {                // (whole words; shifted when they are stored)
+                const uint32_t *w = reinterpret_cast<const uint32_t *>(
+                    reinterpret_cast<uintptr_t>(src + ahead + k * ESEG + tid * 4) & ~uintptr_t(3));
+                next[k][0] = __ldg(w);
+                next[k][1] = __ldg(w + 1);
+            }
+        }
         // ---- B: chains of matches from the parse position
         while (pos < wend) {
             const uint32_t s0 = par_next_match(S.bits, pos - w0);
             if (s0 >= (uint32_t)wn) { pos = wend; break; }   // no match left: literals run on
             // J[q]: the match after the one at q, or why the chain stops there
-            for (int q = tid; q < wn; q += PT) {
-                const int L = S.w.lw[q];
-                uint16_t j = PJ_NONE;
-                if (L >= PCAP) j = PJ_LONG;
-                else if (L >= 4) {
-                    const uint32_t nx = par_next_match(S.bits, q + L);
-                    j = nx >= (uint32_t)wn ? (q + L >= wn ? PJ_OUT : PJ_NONE) : (uint16_t)nx;
+            const unsigned nz = __ballot_sync(FULLMASK, S.bits[lane] != 0);
+#pragma unroll
+            for (int k = 0; k < PW / PT; k++) {
+                const int q = tid + k * PT, L = S.w.lw[q], e = q + L, sg = min(e >> 5, 31);
+                uint32_t r = S.bits[sg] & (FULLMASK << (e & 31));
+                const unsigned more = sg < 31 ? nz & (FULLMASK << (sg + 1)) : 0u;
+                int s2 = sg;
+                if (!r && more) {
+                    s2 = __ffs((int)more) - 1;
+                    r = S.bits[s2];
                 }
-                S.w.J[q] = j;
+                uint32_t v = r ? (uint32_t)(s2 * 32 + __ffs((int)r) - 1) : (uint32_t)PJ_NONE;
+                if (e >= wn) v = PJ_OUT;
+                if (L >= PCAP) v = PJ_LONG;
+                S.w.J[q] = (uint16_t)v;
             }
             __syncthreads();
             // The chain from s0 by segment walks (warp 0): lane t walks J from the first match
@@ -2032,48 +2152,57 @@ __device__ __forceinline__ int cta_lz4_compress_par(const uint8_t *__restrict__ 
                     if (cnum < PT) break;
                 }
             }
-            // output sizes
-            int mine = 0;
-            for (int i = tid; i < cnt; i += PT) {
-                const int q = w0 + S.w.path[i];
-                const int prev_end = i ? w0 + S.w.path[i - 1] + S.w.lw[S.w.path[i - 1]] : anchor;
-                const int L = (i == cnt - 1) ? lastL : S.w.lw[S.w.path[i]];
-                mine += lz4_seq_bytes(q - prev_end, L - 4);
-            }
-            const int total = cta_sum(mine, S.red);
-            if (op + total + 1 + 6 > cap) return 0;
-            // write: exclusive scan per round of PT sequences
-            int base = op;
-            for (int i0 = 0; i0 < cnt; i0 += PT) {
-                const int i = i0 + tid;
-                int sz = 0, q = 0, prev_end = 0, L = 0, d = 0;
+            // output sizes, their exclusive scan (two sequences a thread; at most PW / 4), the sequences
+            int q2[2], e2[2], L2[2], d2[2], sz2[2];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int i = 2 * tid + k;
+                q2[k] = e2[k] = L2[k] = d2[k] = sz2[k] = 0;
                 if (i < cnt) {
-                    q = w0 + S.w.path[i];
-                    prev_end = i ? w0 + S.w.path[i - 1] + S.w.lw[S.w.path[i - 1]] : anchor;
-                    L = (i == cnt - 1) ? lastL : S.w.lw[S.w.path[i]];
-                    d = S.w.cw[S.w.path[i]];
-                    sz = lz4_seq_bytes(q - prev_end, L - 4);
+                    const int q = S.w.path[i], before = i ? S.w.path[i - 1] : 0;
+                    e2[k] = i ? w0 + before + S.w.lw[before] : anchor;
+                    q2[k] = w0 + q;
+                    L2[k] = i == cnt - 1 ? lastL : S.w.lw[q];
+                    d2[k] = S.w.cw[q];
+                    sz2[k] = lz4_seq_bytes(q2[k] - e2[k], L2[k] - 4);
                 }
-                int incl = sz;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(FULLMASK, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                if (lane == 31) S.red[warp] = incl;
-                __syncthreads();
-                int before = 0, all = 0;
-#pragma unroll
-                for (int k = 0; k < PT / 32; k++) {
-                    const int t = S.red[k];
-                    before += k < warp ? t : 0;
-                    all += t;
-                }
-                if (i < cnt) lz4_put_seq(s, dst + base + before + incl - sz, prev_end, q, d, L);
-                base += all;
-                __syncthreads();
             }
-            op = base;
+            const int both = sz2[0] + sz2[1];
+            int incl = both;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(FULLMASK, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) S.red[warp] = incl;
+            __syncthreads();
+            int before = 0, total = 0;
+#pragma unroll
+            for (int k = 0; k < PT / 32; k++) {
+                const int t = S.red[k];
+                before += k < warp ? t : 0;
+                total += t;
+            }
+            if (op + total + 1 + 6 <= cap) {
+                int o = op + before + incl - both;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const int lit = q2[k] - e2[k];
+                    if (sz2[k]) lz4_put_seq(s, dst + o, e2[k], q2[k], d2[k], L2[k], lit <= 16);
+                    // longer literal runs by the warp
+                    const int at = o + 1 + (lit >= 15 ? 1 + (lit - 15) / 255 : 0);
+                    for (unsigned m = __ballot_sync(FULLMASK, sz2[k] && lit > 16); m; m &= m - 1) {
+                        const int i = __ffs((int)m) - 1;
+                        const int to = __shfl_sync(FULLMASK, at, i), from = __shfl_sync(FULLMASK, e2[k], i),
+                                  cnt = __shfl_sync(FULLMASK, lit, i);
+                        for (int x = lane; x < cnt; x += 32) dst[to + x] = (uint8_t)es_byte(s, from + x);
+                    }
+                    o += sz2[k];
+                }
+            }
+            __syncthreads();
+            if (op + total + 1 + 6 > cap) return 0;
+            op += total;
             anchor = lastq + lastL;
             pos = anchor;
             if (term == PJ_NONE) { pos = max(pos, wend); }
