@@ -61,130 +61,142 @@ __device__ __forceinline__ void divmod(int64_t a, int64_t b, int64_t &q, int64_t
 }
 
 // ============================================================================ decode
-// D0: parse one (chunk, block) per thread.  What bounds it is the chain of loads: chunk offset,
-// header, block start, and one size word after the other, each where the stream before it ends.
-// So every word is one load (two when it straddles words), the block start is loaded beside the
-// header, and the size words are loaded at once where they lie when the streams before them are
-// raw, the usual case but for the last planes; a word that lies elsewhere is loaded when its
-// place is known.
+// D0: parse one (chunk, block) per 8 lanes, lane j for stream j.  What bounds it is the chain of
+// loads (chunk offset, header, block start, and one size word after the other, each where the
+// stream before it ends) and, as every warp runs the code once, fetching the instructions: so a
+// lane loads one header word and one size word, the latter at once where it lies when the streams
+// before it are raw, the usual case but for the last planes; the group then goes through the
+// streams in a loop of a few instructions, loading only the size words that lie elsewhere, and
+// lane j stores stream j's descriptor.  (One thread per block, its loops unrolled: 16 us a
+// launch for an operand of some ten blocks, timed with its events; now 12.)
 // zf (optional): per (chunk, block) zero flags of the reference's block-pair products:
 // bit 0 = block_is_zeros (src/linalg/iarray_gemm.c:28-77: no memcpyed or special chunk, and
 // the first typesize csize words from the block's bstart are all 0: Blosc2 v5 chunks always
 // carry the flag bit the reference reads as "split"), bit 1 = chunk_is_zeros (:17-26:
 // special value ZERO); nzero counts the flagged blocks.
-struct ParsedBlock {
-    uint32_t lz;               // bit j: stream j is an LZ4 stream
-    int32_t q[8], cs[8];       // its payload's place in the chunk, its size
-    int32_t neblock;
+struct ParsedStream {
+    bool lz4;                  // an LZ4 stream
+    int32_t q, cs, neblock;    // its payload's place in the chunk, its size, its output's
     const uint8_t *chunk;
 };
 __device__ __forceinline__ void parse_block(const Geom &g, const uint8_t *__restrict__ ch, const int64_t *__restrict__ off,
                                             const int32_t *__restrict__ len, BlockDesc *bd, StreamDesc *sd, int *err,
-                                            uint8_t *zf, int *nzero, int64_t t, ParsedBlock &pb)
+                                            uint8_t *zf, int *nzero, int64_t t, bool valid, ParsedStream &ps)
 {
-    pb.lz = 0;
-    do {
-        int64_t c, b;
+    const int j = threadIdx.x & 7;
+    int64_t c = 0, b = 0, coff = 0;
+    int32_t clen = 0;
+    if (valid) {
         divmod(t, g.nblocks, c, b);
-        const int64_t coff = off[c];
-        const uint8_t *p = ch + coff;
-        const int32_t clen = len[c];
-        BlockDesc d;
-        d.mode = BM_PLAIN; d.nstreams = 1; d.neblock = (int32_t)g.blocksize; d.pad = 0; d.value_src = 0;
-        StreamDesc *s = sd + t * 8;
-        for (int j = 0; j < 8; j++) { s[j].kind = SK_RUN; s[j].len = 0; s[j].src = 0; }
-        bool ok = clen >= 32;
-        int32_t w0 = 0, nbytes = 0, bsz = 0, cbytes = 0, w16 = 0, w20 = 0, w28 = 0;
-        int64_t bstart = 0;
-        if (ok) {
-            w0 = ld_s32(p); nbytes = ld_s32(p + 4); bsz = ld_s32(p + 8); cbytes = ld_s32(p + 12);
-            w16 = ld_s32(p + 16); w20 = ld_s32(p + 20); w28 = ld_s32(p + 28);
-            if (36 + 4 * b <= clen) bstart = ld_s32(p + 32 + 4 * b);
-        }
-        const uint8_t flags = (uint8_t)(w0 >> 16), ts = (uint8_t)((uint32_t)w0 >> 24), bflags = (uint8_t)((uint32_t)w28 >> 24);
-        if (ok) ok = (flags & 0x05) == 0x05 && nbytes == g.chunk_nbytes && cbytes >= 32 && cbytes <= clen;
-        if (!ok) { dev_fail(err, DE_HEADER); bd[t] = d; if (zf) zf[t] = 0; continue; }
-        // the size words of a split block whose streams before them are raw
-        const int32_t neb = (int32_t)(g.blocksize / g.itemsize);
-        int32_t pre[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int64_t q = bstart + (int64_t)j * (neb + 4);
-            pre[j] = j < g.itemsize && bstart >= 32 && q + 4 <= cbytes ? ld_s32(p + q) : 0;
-        }
-        const int special = (bflags >> 4) & 7;
-        if (zf) {
-            uint8_t zflag = special == 1 ? 2 : 0;
-            if (!special && !(flags & 0x02) && 32 + 4 * (b + 1) <= cbytes) {
-                bool z = bstart >= 32 && bstart + 4 * (int64_t)ts <= cbytes && (ts == 0 || pre[0] == 0);
-                for (int j = 1; z && j < ts; j++) z = ld_s32(p + bstart + 4 * j) == 0;
-                if (z) zflag |= 1;
-            }
+        coff = off[c];
+        clen = len[c];
+    }
+    const uint8_t *p = ch + coff;
+    bool ok = clen >= 32;
+    const int32_t hw = ok ? ld_s32(p + 4 * j) : 0;
+    const int32_t bstart = ok && 36 + 4 * b <= clen ? ld_s32(p + 32 + 4 * b) : 0;
+    const uint32_t w0 = (uint32_t)__shfl_sync(FULLMASK, hw, 0, 8);
+    const int32_t nbytes = __shfl_sync(FULLMASK, hw, 1, 8), bsz = __shfl_sync(FULLMASK, hw, 2, 8),
+                  cbytes = __shfl_sync(FULLMASK, hw, 3, 8), w16 = __shfl_sync(FULLMASK, hw, 4, 8),
+                  w20 = __shfl_sync(FULLMASK, hw, 5, 8);
+    const uint32_t w28 = (uint32_t)__shfl_sync(FULLMASK, hw, 7, 8);
+    const uint8_t flags = (uint8_t)(w0 >> 16), ts = (uint8_t)(w0 >> 24);
+    ok = ok && (flags & 0x05) == 0x05 && nbytes == g.chunk_nbytes && cbytes >= 32 && cbytes <= clen;
+    int fail = ok || !valid ? 0 : DE_HEADER;
+    // the size word of stream j where the streams before it are raw
+    const int32_t step = (int32_t)(g.blocksize / g.itemsize) + 4;
+    int32_t pre = 0;
+    {
+        const int64_t at = bstart + (int64_t)j * step;
+        if (ok && j < g.itemsize && bstart >= 32 && at + 4 <= cbytes) pre = ld_s32(p + at);
+    }
+    const int special = (int)(w28 >> 28) & 7;
+    if (zf) {
+        bool z = ok && !special && !(flags & 0x02) && 32 + 4 * (b + 1) <= cbytes && bstart >= 32 &&
+                 bstart + 4 * (int64_t)ts <= cbytes;
+        for (int i = j; z && i < ts; i += 8) z = ld_s32(p + bstart + 4 * i) == 0;
+        const unsigned group = 0xffu << (threadIdx.x & 24);
+        z = (__ballot_sync(FULLMASK, z) & group) == group;
+        if (valid && j == 0) {
+            const uint8_t zflag = ok ? (special == 1 ? 2 : 0) | (z ? 1 : 0) : 0;
             zf[t] = zflag;
             if (zflag && nzero) atomicAdd(nzero, 1);
         }
+    }
+    int mode = BM_PLAIN, nstreams = 1, neblock = (int)g.blocksize;
+    int64_t value_src = 0, src = 0;
+    int kind = SK_RUN, slen = 0;
+    bool streams = false;                          // a block of size words and payloads
+    if (ok) {
         if (special) {
-            if (special == 2) d.mode = BM_NAN;
+            if (special == 2) mode = BM_NAN;
             else if (special == 3) {
-                if (cbytes < 32 + (int32_t)g.itemsize) dev_fail(err, DE_HEADER);
-                d.mode = BM_VALUE; d.value_src = coff + 32;
-            } else if (special != 1 && special != 4) dev_fail(err, DE_HEADER);
-            bd[t] = d;
-            continue;
+                if (cbytes < 32 + (int32_t)g.itemsize) fail = DE_HEADER;
+                mode = BM_VALUE; value_src = coff + 32;
+            } else if (special != 1 && special != 4) fail = DE_HEADER;
+        } else if (flags & 0x02) {                 // memcpyed: raw blocked items
+            if (cbytes < 32 + nbytes) fail = DE_BOUNDS;
+            else if (j == 0) { kind = SK_RAW; slen = (int)g.blocksize; src = coff + 32 + b * g.blocksize; }
+        } else {
+            // filters: only SHUFFLE (slot 5 == 1) or none are produced on this path
+            const uint8_t filter5 = (uint8_t)((uint32_t)w20 >> 8);
+            const bool filt_ok = w16 == 0 && (w20 & 0xFF) == 0 && filter5 <= 1;
+            const int64_t bs_end = 32 + 4 * g.nblocks;
+            if (bsz != g.blocksize || ts != g.itemsize || !filt_ok) {
+                fail = DE_HEADER;
+            } else {
+                nstreams = !(flags & 0x10) ? ts : 1;
+                neblock = (int)(g.blocksize / nstreams);
+                if (bs_end > cbytes || bstart < bs_end || bstart >= cbytes) fail = DE_BOUNDS;
+                else {
+                    streams = true;
+                    if (filter5 == 1 && ts > 1) mode = BM_SHUFFLED;
+                }
+            }
         }
-        if (flags & 0x02) {                      // memcpyed: raw blocked items
-            if (cbytes < 32 + nbytes) { dev_fail(err, DE_BOUNDS); bd[t] = d; continue; }
-            s[0].kind = SK_RAW; s[0].len = (int32_t)g.blocksize; s[0].src = coff + 32 + b * g.blocksize;
-            bd[t] = d;
-            continue;
-        }
-        // filters: only SHUFFLE (slot 5 == 1) or none are produced on this path
-        const uint8_t filter5 = (uint8_t)((uint32_t)w20 >> 8);
-        const bool filt_ok = w16 == 0 && (w20 & 0xFF) == 0 && filter5 <= 1;
-        if (bsz != g.blocksize || ts != g.itemsize || !filt_ok) { dev_fail(err, DE_HEADER); bd[t] = d; continue; }
-        const bool split = !(flags & 0x10);
-        const bool shuffle = filter5 == 1 && ts > 1;
-        const int nstreams = split ? ts : 1;
-        const int neblock = (int)(g.blocksize / nstreams);
-        d.mode = shuffle ? BM_SHUFFLED : BM_PLAIN;
-        d.nstreams = nstreams; d.neblock = neblock;
-        pb.neblock = neblock;
-        pb.chunk = p;
-        const int64_t bs_end = 32 + 4 * g.nblocks;
-        if (bs_end > cbytes) { d.mode = BM_PLAIN; dev_fail(err, DE_BOUNDS); bd[t] = d; continue; }
+    }
+    bool whole = streams;
+    int32_t at = 0;
+    {
         int64_t q = bstart;
-        if (q < bs_end || q >= cbytes) { d.mode = BM_PLAIN; dev_fail(err, DE_BOUNDS); bd[t] = d; continue; }
-        uint32_t lz = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (j >= nstreams || !ok) break;
-            if (q + 4 > cbytes) { dev_fail(err, DE_BOUNDS); ok = false; break; }
-            const int32_t cs = q == bstart + (int64_t)j * (neb + 4) ? pre[j] : ld_s32(p + q);
+#pragma unroll 1
+        for (int k = 0; k < 8; k++) {
+            const int32_t ahead = __shfl_sync(FULLMASK, pre, k, 8);
+            if (!whole || k >= nstreams) continue;
+            if (q + 4 > cbytes) { fail = DE_BOUNDS; whole = false; continue; }
+            const int32_t cs = q == bstart + (int64_t)k * step ? ahead : ld_s32(p + q);
             q += 4;
             if (cs == 0) continue;
             if (cs < 0) {
-                if (q + 1 > cbytes || !(p[q] & 1) || cs < -255) { dev_fail(err, DE_RUN_TOKEN); ok = false; break; }
+                if (q + 1 > cbytes || !(p[q] & 1) || cs < -255) { fail = DE_RUN_TOKEN; whole = false; continue; }
                 q += 1;
-                s[j].len = -cs;
+                if (k == j) slen = -cs;
                 continue;
             }
-            if (q + cs > cbytes || cs > neblock) { dev_fail(err, DE_BOUNDS); ok = false; break; }
-            s[j].src = coff + q;
-            s[j].len = cs;
-            if (cs == neblock) {
-                s[j].kind = SK_RAW;
-            } else {
-                s[j].kind = SK_LZ4;
-                lz |= 1u << j;
-                pb.q[j] = (int32_t)q;
-                pb.cs[j] = cs;
+            if (q + cs > cbytes || cs > neblock) { fail = DE_BOUNDS; whole = false; continue; }
+            if (k == j) {
+                kind = cs == neblock ? SK_RAW : SK_LZ4;
+                slen = cs;
+                src = coff + q;
+                at = (int32_t)q;
             }
             q += cs;
         }
-        if (!ok) { for (int j = 0; j < nstreams; j++) { s[j].kind = SK_RUN; s[j].len = 0; } }
-        else pb.lz = lz;
-        bd[t] = d;
-    } while (false);
+    }
+    if (streams && !whole) { kind = SK_RUN; slen = 0; }
+    if (valid) {
+        if (j == 0) {
+            BlockDesc d;
+            d.mode = mode; d.nstreams = nstreams; d.neblock = neblock; d.pad = 0; d.value_src = value_src;
+            bd[t] = d;
+            if (fail) dev_fail(err, fail);
+        }
+        StreamDesc d;
+        d.kind = kind; d.len = slen; d.src = src;
+        sd[t * 8 + j] = d;
+    }
+    ps.lz4 = valid && kind == SK_LZ4;
+    ps.q = at; ps.cs = slen; ps.neblock = neblock; ps.chunk = p;
 }
 
 // Queues the LZ4 streams of a warp's blocks (every lane calls): stream j of a block goes to region
@@ -192,50 +204,44 @@ __device__ __forceinline__ void parse_block(const Geom &g, const uint8_t *__rest
 // first planes of smooth floats are the longest streams, the last one the shortest: handed out in
 // the blocks' order instead, the decode of a 20000 x 20000 float32 matrix takes 6.45 ms, by planes 6.0.)
 // The eight counters are bumped by one instruction per warp.
-__device__ __forceinline__ void queue_streams(const ParsedBlock &pb, uint8_t *blk_scratch, int *err, Lz4Job *jobs,
+__device__ __forceinline__ void queue_streams(const ParsedStream &ps, uint8_t *blk_scratch, int *err, Lz4Job *jobs,
                                               int *njobs, int64_t jcap)
 {
-    const int lane = threadIdx.x & 31;
-    if (!__any_sync(FULLMASK, pb.lz != 0)) return;
-    const int64_t region = jcap / 8;
-    int mine = 0;                          // lane j: streams of plane j
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int n = __popc(__ballot_sync(FULLMASK, (pb.lz >> j) & 1u));
-        if (lane == j) mine = n;
-    }
-    int at = 0;
-    if (mine) at = atomicAdd(njobs + lane, mine);
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const bool has = (pb.lz >> j) & 1u;
-        const unsigned m = __ballot_sync(FULLMASK, has);
-        const int64_t k = (int64_t)__shfl_sync(FULLMASK, at, j) + __popc(m & ((1u << lane) - 1u));
-        if (!has) continue;
-        if (k < region) {
-            Lz4Job jb;
-            jb.src = pb.chunk + pb.q[j]; jb.dst = blk_scratch + (int64_t)j * pb.neblock; jb.err = err;
-            jb.csize = pb.cs[j]; jb.dlen = pb.neblock;
-            jobs[j * region + k] = jb;
-        } else {
-            dev_fail(err, DE_BOUNDS);                                // (a region holds a stream of every block)
-        }
+    const int lane = threadIdx.x & 31, j = lane & 7;
+    const unsigned m = __ballot_sync(FULLMASK, ps.lz4) & (0x01010101u << j);   // the plane's
+    if (!__any_sync(FULLMASK, ps.lz4)) return;
+    int base = 0;
+    if (lane < 8 && m) base = atomicAdd(njobs + j, __popc(m));
+    const int64_t region = jcap / 8, k = (int64_t)__shfl_sync(FULLMASK, base, j) + __popc(m & ((1u << lane) - 1u));
+    if (!ps.lz4) return;
+    if (k < region) {
+        Lz4Job jb;
+        jb.src = ps.chunk + ps.q; jb.dst = blk_scratch + (int64_t)j * ps.neblock; jb.err = err;
+        jb.csize = ps.cs; jb.dlen = ps.neblock;
+        jobs[j * region + k] = jb;
+    } else {
+        dev_fail(err, DE_BOUNDS);                                // (a region holds a stream of every block)
     }
 }
 
-// (blockDim.x is a multiple of 32)
-__global__ void k_parse(Geom g, const uint8_t *__restrict__ ch, const int64_t *__restrict__ off,
-                        const int32_t *__restrict__ len, BlockDesc *bd, StreamDesc *sd, Lz4Job *jobs,
-                        int *njobs, int64_t jcap, int *err, uint8_t *scratch, uint8_t *zf, int *nzero)
+// (blockDim.x is a multiple of 32; 8 threads a block)
+constexpr int PARSE_T = 128;
+__global__ void __launch_bounds__(PARSE_T) k_parse(Geom g, const uint8_t *__restrict__ ch, const int64_t *__restrict__ off,
+                                                   const int32_t *__restrict__ len, BlockDesc *bd, StreamDesc *sd,
+                                                   Lz4Job *jobs, int *njobs, int64_t jcap, int *err, uint8_t *scratch,
+                                                   uint8_t *zf, int *nzero)
 {
     const int64_t total = g.nchunks * g.nblocks;
-    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x; t0 < total; t0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = t0 + threadIdx.x;
-        ParsedBlock pb;
-        pb.lz = 0;
-        if (t < total) parse_block(g, ch, off, len, bd, sd, err, zf, nzero, t, pb);
-        queue_streams(pb, scratch + t * g.blocksize, err, jobs, njobs, jcap);
+    for (int64_t t0 = (int64_t)blockIdx.x * (PARSE_T / 8); t0 < total; t0 += (int64_t)gridDim.x * (PARSE_T / 8)) {
+        const int64_t t = t0 + threadIdx.x / 8;
+        ParsedStream ps;
+        parse_block(g, ch, off, len, bd, sd, err, zf, nzero, t, t < total, ps);
+        queue_streams(ps, scratch + t * g.blocksize, err, jobs, njobs, jcap);
     }
+}
+static unsigned parse_grid(int64_t nbl, int sms)
+{
+    return (unsigned)std::max<int64_t>(std::min<int64_t>(ceil_div(nbl, PARSE_T / 8), (int64_t)sms * 16), 1);
 }
 
 // D1: LZ4 stream decode, one CTA (256 threads) per stream, streams handed out
@@ -2691,10 +2697,8 @@ int decode_parse(const DecodeArgs &a, DecodeQueue *q, DecodeWork *w, cudaStream_
         cudaMemsetAsync(w->ext_counters ? (void *)w->ext_counters : w->counters.p, 0, 64, st);
     }
     int *cnt = w->ext_counters ? w->ext_counters : w->counters.as<int>();
-    const int threads = 128;
-    const int64_t blocks = std::min<int64_t>((nbl + threads - 1) / threads, (int64_t)sm_count() * 16);
     if (!w->zf.allocate((size_t)std::max<int64_t>(nbl, 1), dev)) return -100;
-    IAB_TIMED("k_parse", st, k_parse<<<(unsigned)std::max<int64_t>(blocks, 1), threads, 0, st>>>(
+    IAB_TIMED("k_parse", st, k_parse<<<parse_grid(nbl, sm_count()), PARSE_T, 0, st>>>(
         g, a.chunks, a.off, a.len, w->bd.as<BlockDesc>(), w->sd.as<StreamDesc>(), q->jobs.as<Lz4Job>(),
         q->counters.as<int>(), q->cap, cnt + 1, w->scratch.as<uint8_t>(), w->zf.as<uint8_t>(), cnt + 4));
     return 0;
@@ -3237,24 +3241,18 @@ __global__ void k_group_reset(const CodecItem *__restrict__ items, int n)
     if (x < (int64_t)n * 16) items[x >> 4].cnt[x & 15] = 0;
 }
 
-__global__ void k_parse_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart, int n, int64_t nbl,
-                          Lz4Job *jobs, int *njobs, int64_t jcap)
+__global__ void __launch_bounds__(PARSE_T) k_parse_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart,
+                                                     int n, int64_t nbl, Lz4Job *jobs, int *njobs, int64_t jcap)
 {
-    for (int64_t u0 = (int64_t)blockIdx.x * blockDim.x; u0 < nbl; u0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t u = u0 + threadIdx.x;
-        ParsedBlock pb;
-        pb.lz = 0;
-        uint8_t *blk = nullptr;
-        int *err = nullptr;
-        if (u < nbl) {
-            const int k = group_find(bstart, n, u);
-            const CodecItem &it = items[k];
-            const int64_t t = u - bstart[k];
-            err = it.cnt + 1;
-            blk = it.scratch + t * it.g.blocksize;
-            parse_block(it.g, it.ch, it.off, it.len, it.bd, it.sd, err, nullptr, nullptr, t, pb);
-        }
-        queue_streams(pb, blk, err, jobs, njobs, jcap);
+    for (int64_t u0 = (int64_t)blockIdx.x * (PARSE_T / 8); u0 < nbl; u0 += (int64_t)gridDim.x * (PARSE_T / 8)) {
+        const int64_t u = u0 + threadIdx.x / 8;
+        const bool valid = u < nbl;
+        const int k = group_find(bstart, n, valid ? u : nbl - 1);
+        const CodecItem &it = items[k];
+        const int64_t t = u - bstart[k];
+        ParsedStream ps;
+        parse_block(it.g, it.ch, it.off, it.len, it.bd, it.sd, it.cnt + 1, nullptr, nullptr, t, valid, ps);
+        queue_streams(ps, it.scratch + t * it.g.blocksize, it.cnt + 1, jobs, njobs, jcap);
     }
 }
 
@@ -3444,8 +3442,7 @@ int decode_group_launch(CodecGroup *grp, cudaStream_t st)
     cudaMemsetAsync(grp->q.counters.p, 0, 64, st);
     IAB_TIMED("k_group_reset", st, k_group_reset<<<(unsigned)((n * 16 + 255) / 256), 256, 0, st>>>(items, n));
     if (grp->nbl == 0) return 0;
-    const int64_t pb = std::min<int64_t>((grp->nbl + 127) / 128, (int64_t)sms * 16);
-    IAB_TIMED("k_parse", st, k_parse_g<<<(unsigned)pb, 128, 0, st>>>(items, bstart, n, grp->nbl, grp->q.jobs.as<Lz4Job>(),
+    IAB_TIMED("k_parse", st, k_parse_g<<<parse_grid(grp->nbl, sms), PARSE_T, 0, st>>>(items, bstart, n, grp->nbl, grp->q.jobs.as<Lz4Job>(),
                                                                      grp->q.counters.as<int>(), grp->q.cap));
     int r = decode_lz4(&grp->q, st);
     if (r) return r;
@@ -3638,13 +3635,8 @@ int decode_noalloc(const Geom &g, const uint8_t *d_chunks, int64_t chunks_bytes,
     if (cudaMemsetAsync(counters, 0, 64, st) != cudaSuccess) return -101;
     const int sms = sm_count();
     IAB_TIMED("k_chunk_walk", st, k_chunk_walk<<<1, 32, 0, st>>>(d_chunks, chunks_bytes, g.nchunks, off, len));
-    {
-        const int threads = 128;
-        const int64_t blocks = std::min<int64_t>((nbl + threads - 1) / threads, (int64_t)sms * 16);
-        IAB_TIMED("k_parse", st, k_parse<<<(unsigned)std::max<int64_t>(blocks, 1), threads, 0, st>>>(g, d_chunks, off, len, bd, sd, jobs, njobs,
-                                                                                      8 * NA_MAX_BLOCKS, err, img,
-                                                                                      nullptr, nullptr));
-    }
+    IAB_TIMED("k_parse", st, k_parse<<<parse_grid(nbl, sms), PARSE_T, 0, st>>>(g, d_chunks, off, len, bd, sd, jobs, njobs,
+                                                                              8 * NA_MAX_BLOCKS, err, img, nullptr, nullptr));
     {
         IAB_TIMED("k_lz4_decode_cta", st, k_lz4_decode_cta<<<sms * 6, dcta::THREADS, (int)sizeof(dcta::Smem), st>>>(
             jobs, njobs, 8 * NA_MAX_BLOCKS, reinterpret_cast<unsigned *>(counters + 8)));
