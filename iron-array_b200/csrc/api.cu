@@ -1214,8 +1214,9 @@ struct ZeroRule {
         if (!za.allocate((size_t)(RB * KB), ctx->device) || !zb.allocate((size_t)(KB * JB), ctx->device) ||
             !nfa.allocate((size_t)(RB * KB), ctx->device) || !nfb.allocate((size_t)(KB * JB), ctx->device))
             return false;
-        iab::zero_grid(ga, zf[0].as<uint8_t>(), rule == SKIP_BOTH || rule == SKIP_A_CHUNKS, za.as<uint8_t>(), ctx->stream);
-        iab::zero_grid(gb, zf[1].as<uint8_t>(), rule == SKIP_BOTH || rule == SKIP_B_CHUNKS, zb.as<uint8_t>(), ctx->stream);
+        iab::zero_grids({ga, zf[0].as<uint8_t>(), rule == SKIP_BOTH || rule == SKIP_A_CHUNKS, za.as<uint8_t>(), nfa.as<uint8_t>()},
+                        {gb, zf[1].as<uint8_t>(), rule == SKIP_BOTH || rule == SKIP_B_CHUNKS, zb.as<uint8_t>(), nfb.as<uint8_t>()},
+                        ctx->stream);
         zs = iab::ZeroSkip{za.as<uint8_t>(), zb.as<uint8_t>(),
                            ga.chunk[0], ga.block[0], ga.bgrid[0],
                            ga.chunk[1], ga.block[1], ga.bgrid[1],
@@ -1228,12 +1229,10 @@ struct ZeroRule {
              int64_t ldb, void *C, int64_t ldc)
     {
         if (!on) return;
-        cudaMemsetAsync(nfa.p, 0, nfa.n, ctx->stream);
-        cudaMemsetAsync(nfb.p, 0, nfb.n, ctx->stream);
-        iab::block_nonfinite(isz, M, K, A, lda, zs.r_chunk, zs.r_block, zs.r_bg, zs.k_chunk, zs.k_block, zs.k_bg, zs.KB,
-                             nfa.as<uint8_t>(), ctx->stream);
-        iab::block_nonfinite(isz, K, N, B, ldb, zs.k_chunk, zs.k_block, zs.k_bg, zs.c_chunk, zs.c_block, zs.c_bg, zs.JB,
-                             nfb.as<uint8_t>(), ctx->stream);
+        iab::blocks_nonfinite(isz,
+                              {M, K, A, lda, zs.r_chunk, zs.r_block, zs.r_bg, zs.k_chunk, zs.k_block, zs.k_bg, zs.KB, nfa.as<uint8_t>()},
+                              {K, N, B, ldb, zs.k_chunk, zs.k_block, zs.k_bg, zs.c_chunk, zs.c_block, zs.c_bg, zs.JB, nfb.as<uint8_t>()},
+                              ctx->stream);
         iab::zero_fix(isz, M, N, K, A, lda, B, ldb, C, ldc, zs, nfa.as<uint8_t>(), nfb.as<uint8_t>(), ctx->stream);
     }
 };

@@ -426,10 +426,20 @@ int gemm_f32_bf16_split(int64_t M, int64_t N, int64_t K, const float *A, int64_t
                         const float *B, int64_t ldb, float *C, int64_t ldc, int products, cudaStream_t st);
 
 // Zero-block rule of the block-pair products (zero.cu, zskip.cuh).
-void zero_grid(const Geom &g, const uint8_t *zf, bool use_chunk, uint8_t *grid, cudaStream_t st);
-void block_nonfinite(int itemsize, int64_t rows, int64_t cols, const void *x, int64_t ld, int64_t r_chunk,
-                     int64_t r_block, int64_t r_bg, int64_t c_chunk, int64_t c_block, int64_t c_bg, int64_t CB,
-                     uint8_t *flags, cudaStream_t st);
+struct ZeroGrid {           // one operand: its flags from the parse, its two grids
+    Geom g;
+    const uint8_t *zf;
+    int use_chunk;
+    uint8_t *grid, *nf;
+};
+struct NonFinite {          // one dense operand and its blocks
+    int64_t rows, cols;
+    const void *x;
+    int64_t ld, r_chunk, r_block, r_bg, c_chunk, c_block, c_bg, CB;
+    uint8_t *flags;
+};
+void zero_grids(const ZeroGrid &a, const ZeroGrid &b, cudaStream_t st);
+void blocks_nonfinite(int itemsize, const NonFinite &a, const NonFinite &b, cudaStream_t st);
 void zero_fix(int itemsize, int64_t M, int64_t N, int64_t K, const void *A, int64_t lda, const void *B, int64_t ldb,
               void *C, int64_t ldc, const ZeroSkip &z, const uint8_t *nfa, const uint8_t *nfb, cudaStream_t st);
 

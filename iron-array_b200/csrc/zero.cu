@@ -15,33 +15,46 @@
 namespace iab {
 
 // Logical block grid [RB][CB] of a container from the decoder's per (chunk, block) flags:
-// 1 where the block is skipped (block_is_zeros, or chunk_is_zeros when `use_chunk`).
-__global__ void k_zero_grid(Geom g, const uint8_t *__restrict__ zf, int use_chunk, uint8_t *__restrict__ grid)
+// 1 where the block is skipped (block_is_zeros, or chunk_is_zeros when `use_chunk`); the block's
+// non-finite flag is cleared.  Both operands in one launch (blockIdx.y).
+__global__ void k_zero_grid(ZeroGrid a, ZeroGrid b)
 {
+    const ZeroGrid &o = blockIdx.y ? b : a;
+    const Geom &g = o.g;
     const int64_t RB = g.cgrid[0] * g.bgrid[0], CB = g.cgrid[1] * g.bgrid[1];
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < RB * CB; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t ib = t / CB, jb = t - ib * CB;
         const int64_t ic = ib / g.bgrid[0], bi = ib - ic * g.bgrid[0];
         const int64_t jc = jb / g.bgrid[1], bj = jb - jc * g.bgrid[1];
-        const uint8_t f = zf[(ic * g.cgrid[1] + jc) * g.nblocks + bi * g.bgrid[1] + bj];
-        grid[t] = (f & 1) || (use_chunk && (f & 2)) ? 1 : 0;
+        const uint8_t f = o.zf[(ic * g.cgrid[1] + jc) * g.nblocks + bi * g.bgrid[1] + bj];
+        o.grid[t] = (f & 1) || (o.use_chunk && (f & 2)) ? 1 : 0;
+        o.nf[t] = 0;
     }
 }
 
 // flags[rb * CB + cb] = 1 when the block holds a NaN or an infinity (rows x cols dense,
-// leading dimension ld; blocks as in zskip.cuh).  `flags` starts zeroed.
+// leading dimension ld; blocks as in zskip.cuh).  `flags` starts zeroed.  Both operands in one
+// launch (blockIdx.y); a CTA takes pieces of a row, so that no item costs a division.  Bound by
+// HBM: operands of 4056 x 3712 and 3712 x 3904 float64, 0.078 ms by items in two launches, now 0.050.
+constexpr int NF_PIECE = 1024;
 template <typename T>
-__global__ void k_block_nonfinite(int64_t rows, int64_t cols, const T *__restrict__ x, int64_t ld, int64_t r_chunk,
-                                  int64_t r_block, int64_t r_bg, int64_t c_chunk, int64_t c_block, int64_t c_bg,
-                                  int64_t CB, uint8_t *__restrict__ flags)
+__global__ void __launch_bounds__(256) k_block_nonfinite(NonFinite a, NonFinite b)
 {
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows * cols; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / cols, j = t - i * cols;
-        if (!isfinite(x[i * ld + j])) {
+    const NonFinite &o = blockIdx.y ? b : a;
+    const int64_t np = (o.cols + NF_PIECE - 1) / NF_PIECE;
+    for (int64_t u = blockIdx.x; u < o.rows * np; u += gridDim.x) {
+        const int64_t i = u / np, j0 = (u - i * np) * NF_PIECE + threadIdx.x;
+        const T *x = (const T *)o.x + i * o.ld;
+        T v[NF_PIECE / 256];
+#pragma unroll
+        for (int k = 0; k < NF_PIECE / 256; k++) v[k] = j0 + k * 256 < o.cols ? x[j0 + k * 256] : (T)0;
+#pragma unroll
+        for (int k = 0; k < NF_PIECE / 256; k++) {
+            if (isfinite(v[k])) continue;
             int64_t nx;
-            const int64_t rb = zs_block_of(i, r_chunk, r_block, r_bg, &nx);
-            const int64_t cb = zs_block_of(j, c_chunk, c_block, c_bg, &nx);
-            flags[rb * CB + cb] = 1;
+            const int64_t rb = zs_block_of(i, o.r_chunk, o.r_block, o.r_bg, &nx);
+            const int64_t cb = zs_block_of(j0 + k * 256, o.c_chunk, o.c_block, o.c_bg, &nx);
+            o.flags[rb * o.CB + cb] = 1;
         }
     }
 }
@@ -94,24 +107,20 @@ static int grid_of(int64_t n)
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 8));
 }
 
-void zero_grid(const Geom &g, const uint8_t *zf, bool use_chunk, uint8_t *grid, cudaStream_t st)
+void zero_grids(const ZeroGrid &a, const ZeroGrid &b, cudaStream_t st)
 {
-    const int64_t n = g.cgrid[0] * g.bgrid[0] * g.cgrid[1] * g.bgrid[1];
-    if (n == 0) return;
-    IAB_TIMED("k_zero_grid", st, k_zero_grid<<<grid_of(n), 256, 0, st>>>(g, zf, use_chunk ? 1 : 0, grid));
+    int64_t n = 1;
+    for (const Geom *g : {&a.g, &b.g}) n = std::max(n, g->cgrid[0] * g->bgrid[0] * g->cgrid[1] * g->bgrid[1]);
+    IAB_TIMED("k_zero_grid", st, k_zero_grid<<<dim3((unsigned)grid_of(n), 2), 256, 0, st>>>(a, b));
 }
 
-void block_nonfinite(int itemsize, int64_t rows, int64_t cols, const void *x, int64_t ld, int64_t r_chunk,
-                     int64_t r_block, int64_t r_bg, int64_t c_chunk, int64_t c_block, int64_t c_bg, int64_t CB,
-                     uint8_t *flags, cudaStream_t st)
+void blocks_nonfinite(int itemsize, const NonFinite &a, const NonFinite &b, cudaStream_t st)
 {
-    if (rows * cols == 0) return;
-    if (itemsize == 8)
-        IAB_TIMED("k_block_nonfinite", st, k_block_nonfinite<double><<<grid_of(rows * cols), 256, 0, st>>>(
-            rows, cols, (const double *)x, ld, r_chunk, r_block, r_bg, c_chunk, c_block, c_bg, CB, flags));
-    else
-        IAB_TIMED("k_block_nonfinite", st, k_block_nonfinite<float><<<grid_of(rows * cols), 256, 0, st>>>(
-            rows, cols, (const float *)x, ld, r_chunk, r_block, r_bg, c_chunk, c_block, c_bg, CB, flags));
+    int64_t n = 1;
+    for (const NonFinite *x : {&a, &b}) n = std::max(n, x->rows * ((x->cols + NF_PIECE - 1) / NF_PIECE));
+    const dim3 grid((unsigned)grid_of(n * 256), 2);
+    if (itemsize == 8) IAB_TIMED("k_block_nonfinite", st, k_block_nonfinite<double><<<grid, 256, 0, st>>>(a, b));
+    else IAB_TIMED("k_block_nonfinite", st, k_block_nonfinite<float><<<grid, 256, 0, st>>>(a, b));
 }
 
 void zero_fix(int itemsize, int64_t M, int64_t N, int64_t K, const void *A, int64_t lda, const void *B, int64_t ldb,
