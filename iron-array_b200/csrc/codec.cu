@@ -761,10 +761,11 @@ __device__ __forceinline__ BlockSpan block_span(const Geom &g, int64_t c, int64_
 // in place from raw streams or the LZ4 scratch) into shared memory with bulk asynchronous
 // copies completing on an mbarrier; then each thread rebuilds items and writes the logical ones
 // to the dense row (edge blocks: the items in chunk or array padding are not written; slices of
-// padding only are skipped): 4 consecutive items from one 4-byte word per plane where block rows
-// hold whole groups of 4, else one item from a byte per plane, consecutive lanes taking
-// consecutive items (4000 x 6000 float64 in blocks of 100 x 150: 0.12 ms, 0.79 by the general
-// path's bytewise tiles).  Blocks of other kinds go by the general path.
+// padding only are skipped): 4 consecutive items from one 4-byte word per plane, stored as they lie
+// in a row where block rows hold whole groups of 4, else as two pairs where they are of an even
+// width, else one by one (4000 x 6000 float64 in blocks of 100 x 150: 0.12 ms; 0.15 by one byte
+// per plane and item, 0.79 by the general path's bytewise tiles).  Blocks of other kinds go by the
+// general path.
 constexpr int SC_ITEMS = 4096;
 constexpr int GA_ITEMS = 16384;                    // items of a gather slice
 constexpr int SC_PLANE = SC_ITEMS + 32;            // a slice of a plane from its 16-byte boundary
@@ -925,24 +926,61 @@ __device__ __forceinline__ bool scatter_fast_unit(const Geom &g, const uint8_t *
     uint8_t *const obase = out + (sp.row0 * ld + sp.col0) * TS;
     const int nr = sp.nr, nc = sp.nc;
     if (!geom_quads(g)) {
-        const int step = (int)blockDim.x, step_r = step / rowlen, step_c = step - step_r * rowlen;
-        int r = (i0s + tid) / rowlen, cc = i0s + tid - r * rowlen;
-        for (int i = tid; i < cnt; i += step, r += step_r, cc += step_c) {
+        // quads as two pairs, each in one row, or (rows of an odd width) item by item
+        const bool pairs = rowlen % 2 == 0;
+        const int step = (int)blockDim.x * 4, step_r = step / rowlen, step_c = step - step_r * rowlen;
+        int r = (i0s + tid * 4) / rowlen, cc = i0s + tid * 4 - r * rowlen;
+        for (int qd = tid; qd * 4 < cnt; qd += blockDim.x, r += step_r, cc += step_c) {
             if (cc >= rowlen) { cc -= rowlen; r++; }
-            if (r >= nr || cc >= nc) continue;                            // padding items
-            uint32_t v[TS / 4];
+            uint32_t w[TS];
 #pragma unroll
-            for (int w = 0; w < TS / 4; w++) {
-                v[w] = 0;
+            for (int j = 0; j < TS; j++) {
+                if (code[j] >= 256) { w[j] = (uint32_t)(code[j] - 256) * 0x01010101u; continue; }
+                const uint32_t *pw = reinterpret_cast<const uint32_t *>(stage[j]);
+                const int byte = code[j] + qd * 4, wi = byte >> 2;
+                w[j] = __funnelshift_r(pw[wi], pw[wi + 1], (byte & 3) * 8);
+            }
+            uint32_t v[4], h[4];
+            transpose4x4(w[0], w[1], w[2], w[3], v[0], v[1], v[2], v[3]);
+            if constexpr (TS == 8) transpose4x4(w[4], w[5], w[6], w[7], h[0], h[1], h[2], h[3]);
+            int rr = r, c2 = cc;
+            if (!pairs) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int k = w * 4 + j;
-                    v[w] |= (code[k] >= 256 ? (uint32_t)(code[k] - 256) : (uint32_t)stage[k][code[k] + i]) << (8 * j);
+                for (int u = 0; u < 4; u++) {
+                    if (u && ++c2 >= rowlen) { c2 = 0; rr++; }
+                    if (qd * 4 + u >= cnt || rr >= nr || c2 >= nc) continue;
+                    uint8_t *o = obase + ((int64_t)rr * ld + c2) * TS;
+                    if constexpr (TS == 8) *reinterpret_cast<uint2 *>(o) = make_uint2(v[u], h[u]);
+                    else *reinterpret_cast<uint32_t *>(o) = v[u];
+                }
+                continue;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+                if (u) {
+                    c2 += 2;
+                    if (c2 >= rowlen) { c2 = 0; rr++; }
+                    if (qd * 4 + 2 >= cnt) break;
+                }
+                if (rr >= nr || c2 >= nc) continue;                       // padding items
+                uint8_t *o = obase + ((int64_t)rr * ld + c2) * TS;
+                const bool both = c2 + 1 < nc;
+                if constexpr (TS == 8) {
+                    if (both && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+                        *reinterpret_cast<uint4 *>(o) = make_uint4(v[u], h[u], v[u + 1], h[u + 1]);
+                    } else {
+                        *reinterpret_cast<uint2 *>(o) = make_uint2(v[u], h[u]);
+                        if (both) *reinterpret_cast<uint2 *>(o + 8) = make_uint2(v[u + 1], h[u + 1]);
+                    }
+                } else {
+                    if (both && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+                        *reinterpret_cast<uint2 *>(o) = make_uint2(v[u], v[u + 1]);
+                    } else {
+                        *reinterpret_cast<uint32_t *>(o) = v[u];
+                        if (both) *reinterpret_cast<uint32_t *>(o + 4) = v[u + 1];
+                    }
                 }
             }
-            uint8_t *o = obase + ((int64_t)r * ld + cc) * TS;
-            if constexpr (TS == 8) *reinterpret_cast<uint2 *>(o) = make_uint2(v[0], v[1]);
-            else *reinterpret_cast<uint32_t *>(o) = v[0];
         }
         __syncthreads();                           // stage is read before the next slice's copies
         return true;
