@@ -8,13 +8,12 @@
 // plus Caterva's padded blocked layout (iarray_from_buffer / iarray_to_buffer,
 // src/iarray_constructor.c:218-305).
 //
-// Decode = parse (one thread per block walks its stream headers and queues its LZ4 streams)
-// -> LZ4 (one CTA per LZ4 stream from a job queue that may span several containers; each
-// window of the stream decoded in parallel: token chain by pointer doubling, output resolved
-// in shared memory by pointer jumping) -> unshuffle/scatter (slices of interior blocks staged
-// in shared memory by bulk asynchronous copies, items written to the dense row-major array;
-// a general path for the other blocks).  Raw and run streams are never copied before the
-// scatter.
+// Decode = parse (8 lanes per block read its stream headers and queue its LZ4 streams) -> LZ4 (one
+// CTA per LZ4 stream from a job queue that may span several containers; each window of the
+// stream decoded in parallel: token chain by linked segment tracks, output resolved in shared
+// memory) -> unshuffle/scatter (slices of shuffled blocks staged in shared memory by bulk
+// asynchronous copies, items written to the dense row-major array; a general path for the other
+// blocks).  Raw and run streams are never copied before the scatter.
 //
 // Encode = gather/shuffle (dense -> byte-plane image) -> LZ4 -> layout (per chunk: stream
 // kinds, offsets, memcpy fallback; exclusive scan of chunk sizes) -> emit (copy payloads
@@ -1793,9 +1792,8 @@ __global__ void __launch_bounds__(32, XCTAS) k_lz4_encode(const uint8_t *__restr
 //     at one distance, and candidates inside runs from the lengths of the two runs.
 //  B. the greedy parse (from the parse position, take the first position with a match of
 //     at least 4 bytes, continue after it) is a chain over match positions: J[q] = the first
-//     match position at or after q + L(q).  The chain is located by pointer doubling (J,
-//     J^2, J^4, ... in two ping-pong tables, the chain doubled alongside), the sequences'
-//     output sizes are prefix-summed across the CTA, and every thread writes its own
+//     match position at or after q + L(q).  The chain is located by segment walks (below), the
+//     sequences' output sizes are prefix-summed across the CTA, and every thread writes its own
 //     sequences.  A chain ends at the window end, after the window's last match, or at a
 //     match of PCAP bytes or more, which is extended exactly before it is written.
 // The bytes of the next window are loaded before B and stored after it; literal runs of more than
