@@ -653,7 +653,9 @@ __global__ void __launch_bounds__(dcta::THREADS, 6) k_lz4_decode_cta(const Lz4Jo
                 p = pnext;
                 continue;
             }
-            // the sequence at p does not fit in a window: decode it alone, header from global
+            // the sequence at p does not fit in a window: decode it alone, header from global.
+            // Every thread has to be here before scal is written: it branched on scal[1] and scal[3].
+            __syncthreads();
             if (tid == 0) {
                 int r = p, f = 0, lit = 0, mo = 0, ml = 0, fin = 0;
                 const int tok = __ldg(in + r++);
