@@ -1826,12 +1826,16 @@ INA_API(ina_rc_t) iarray_b200_opt_gemm_cframes(iarray_context_t *ctx, const uint
         } else {
             iab::gemm_f32_native(mk, N, K, (const float *)a_k, lda, dB.as<float>(), ldb, (float *)c_k, ldc, st);
         }
+        // a launch that failed leaves the band unwritten: looked at before the query below replaces
+        // the pending error
+        if (!err && cudaGetLastError() != cudaSuccess) err = -101;
         if (err) break;
         cudaEventRecord(evP.ev[(size_t)k], st);
         cudaStreamWaitEvent(se, evP.ev[(size_t)k], 0);
         w.exact_lz4 = exact_lz4;
         w.memcpy_only = cc->clevel == 0;
         err = iab::encode_launch(gk, c_k, ldc, cc->shuffle, cc->splitmode, &cbuf[(size_t)k], &w, se);
+        if (!err && cudaGetLastError() != cudaSuccess) err = -101;
         if (err) break;
         // the chunk table goes to the host on its own stream: a device-to-host copy queued on
         // the encode stream would wait behind the previous band's download and hold up the
