@@ -1170,6 +1170,8 @@ static ina_rc_t dense_product(iarray_context_t *ctx, int dtype, int64_t M, int64
                                          ctx->split_products_f32, ctx->stream);
         if (r == -100) return rc_err(IARRAY_ERR_GPU_OUT_OF_MEMORY);
         if (r != 0) return rc_err(IARRAY_ERR_NOT_SUPPORTED);
+    } else if (M > INT32_MAX - 256) {
+        return rc_err(IARRAY_ERR_GPU_FAILED);          // the kernels count rows in 32 bits, up to a tile past the last
     } else if (dtype == IARRAY_DATA_TYPE_DOUBLE) {
         iab::gemm_f64_native(M, N, K, (const double *)A, lda, (const double *)B, ldb, (double *)C, ldc, ctx->stream, zs);
     } else {
