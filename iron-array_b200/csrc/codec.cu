@@ -1732,6 +1732,31 @@ __device__ __forceinline__ int64_t stream_at(int64_t k, int64_t total, int per)
     return b * per + (per - 1 - j);
 }
 
+// This thread's share of whether the bytes [b, b + 64 T) of a stream of n bytes all equal `first` (T
+// threads): four 16-byte words, the bytes before the stream's first whole word and after its last one
+// by themselves.  Bound by the loads' requests: byte by byte the streams of a plane, which lie a block
+// apart, took half as long again as those of a block (zeros of 4000 x 3000 float64 in blocks of
+// 100 x 200: 0.223 and 0.263 ms in either order by bytes, 0.033 now).
+template <int T>
+__device__ __forceinline__ bool run_piece(const uint8_t *__restrict__ src, int n, uint8_t first, int b)
+{
+    const int t = threadIdx.x % T, head = min((int)(-reinterpret_cast<uintptr_t>(src) & 15), n), nv = (n - head) / 16;
+    const uint4 *v = reinterpret_cast<const uint4 *>(src + head);
+    const uint32_t all = first * 0x01010101u;
+    uint4 x[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int i = b / 16 + k * T + t;
+        x[k] = i < nv ? __ldg(v + i) : make_uint4(all, all, all, all);
+    }
+    uint32_t d = 0;
+    if (b == 0 && t < head) d |= __ldg(src + t) ^ first;
+    if (b == 0 && head + nv * 16 + t < n) d |= __ldg(src + head + nv * 16 + t) ^ first;
+#pragma unroll
+    for (int k = 0; k < 4; k++) d |= (x[k].x ^ all) | (x[k].y ^ all) | (x[k].z ^ all) | (x[k].w ^ all);
+    return d == 0;
+}
+
 // E2: one warp per stream: run check, then LZ4 into the stream's slot (capacity =
 // stream length; a stream that does not shrink is stored raw).
 // Streams are handed out dynamically (one atomic per stream): compressible streams cost
@@ -1755,14 +1780,7 @@ __global__ void __launch_bounds__(32, XCTAS) k_lz4_encode(const uint8_t *__restr
         const uint8_t *src = img + sid * neblock;
         const uint8_t first = __ldg(src);
         bool run = true;
-        for (int base = 0; base < neblock && run; base += 32 * 16) {
-            bool mine = true;
-            for (int k = 0; k < 16; k++) {
-                const int x = base + k * 32 + lane;
-                if (x < neblock && __ldg(src + x) != first) mine = false;
-            }
-            run = __all_sync(FULLMASK, mine);
-        }
+        for (int b = 0; b < neblock && run; b += 32 * 64) run = __all_sync(FULLMASK, run_piece<32>(src, neblock, first, b));
         EncStream e;
         e.out = -1;
         if (run) {
@@ -2346,14 +2364,7 @@ __global__ void __launch_bounds__(PT, 8) k_lz4_encode_par(const uint8_t *__restr
         const uint8_t *src = img + sid * neblock;
         const uint8_t first = __ldg(src);
         bool run = true;
-        for (int b = 0; b < neblock && run; b += PT * 16) {
-            bool mine = true;
-            for (int k = 0; k < 16; k++) {
-                const int x = b + k * PT + tid;
-                if (x < neblock && __ldg(src + x) != first) mine = false;
-            }
-            run = __syncthreads_and(mine);
-        }
+        for (int b = 0; b < neblock && run; b += PT * 64) run = __syncthreads_and(run_piece<PT>(src, neblock, first, b));
         EncStream e;
         e.out = -1;
         if (run) {
