@@ -761,7 +761,7 @@ __device__ __forceinline__ bool item_pos(const Geom &g, int64_t c, int64_t b, in
 // Partitions with items of 4 or 8 bytes take the fast paths below, edge blocks included:
 // where block rows hold whole groups of 4 items, 4 items and a word of each plane at a time,
 // else item by item.
-__device__ __forceinline__ bool geom_quads(const Geom &g) { return !(g.block[1] & 3); }
+__host__ __device__ __forceinline__ bool geom_quads(const Geom &g) { return !(g.block[1] & 3); }
 
 // D2 fast path: shuffled, split blocks of 4- and 8-byte items, in slices of SC_ITEMS items
 // (one CTA per slice at a time).  One thread stages the slice's bytes of every byte plane (read
@@ -1115,19 +1115,20 @@ __global__ void __launch_bounds__(256) k_scatter(Geom g, int fast_streams, const
 // row and writes one 4-byte word into each byte plane of the image.  Other blocks, whose planes
 // may start at any byte: one item per thread, a byte into each plane, the bytes of a warp
 // next to each other (5000 x 6000 float32 in blocks of 125 x 150: 0.13 ms, 0.29 by the
-// general path).  In slices of GA_ITEMS items, so that a few large blocks spread over the SMs.
-template <int TS>
+// general path).  A few large blocks go in slices, which spread over the SMs (three results of
+// 1000 x 1001 float64 of a batch, each one block: 1.10 ms by a CTA a block, now 0.03).
+template <int TS, bool QUADS>
 __device__ __forceinline__ void gather_fast_block(const Geom &g, const uint8_t *__restrict__ in, int64_t ld,
-                                                  uint8_t *__restrict__ img, int64_t t, int i0s, int cnt)
+                                                  uint8_t *__restrict__ img, int64_t t, int i0s, int cnt, int tid, int nt)
 {
     int64_t c, b;
     divmod(t, g.nblocks, c, b);
     const BlockSpan sp = block_span(g, c, b);
     uint8_t *blk = img + t * g.blocksize;
-    if (!geom_quads(g)) {
-        const int rowlen = (int)g.block[1], step = (int)blockDim.x, step_r = step / rowlen, step_c = step - step_r * rowlen;
-        int r = (i0s + (int)threadIdx.x) / rowlen, cc = i0s + (int)threadIdx.x - r * rowlen;
-        for (int i = i0s + threadIdx.x; i < i0s + cnt; i += step, r += step_r, cc += step_c) {
+    if constexpr (!QUADS) {
+        const int rowlen = (int)g.block[1], step = nt, step_r = step / rowlen, step_c = step - step_r * rowlen;
+        int r = (i0s + tid) / rowlen, cc = i0s + tid - r * rowlen;
+        for (int i = i0s + tid; i < i0s + cnt; i += step, r += step_r, cc += step_c) {
             if (cc >= rowlen) { cc -= rowlen; r++; }
             uint64_t x = 0;
             if (r < sp.nr && cc < sp.nc) {
@@ -1141,9 +1142,9 @@ __device__ __forceinline__ void gather_fast_block(const Geom &g, const uint8_t *
     }
     const int qpr = (int)(g.block[1] / 4), q0 = i0s / 4, nq = cnt / 4;
     // (row, quad column) of each thread's quad, advanced by a fixed step per iteration
-    const int step_r = (int)blockDim.x / qpr, step_q = (int)blockDim.x - step_r * qpr;
-    int r = (q0 + (int)threadIdx.x) / qpr, q = q0 + (int)threadIdx.x - r * qpr;
-    for (int qd = q0 + threadIdx.x; qd < q0 + nq; qd += blockDim.x, r += step_r, q += step_q) {
+    const int step_r = nt / qpr, step_q = nt - step_r * qpr;
+    int r = (q0 + tid) / qpr, q = q0 + tid - r * qpr;
+    for (int qd = q0 + tid; qd < q0 + nq; qd += nt, r += step_r, q += step_q) {
         if (q >= qpr) { q -= qpr; r++; }
         const int i0 = qd * 4, cc = q * 4;
         const uint8_t *src = in + ((sp.row0 + r) * ld + sp.col0 + cc) * TS;
@@ -1174,15 +1175,34 @@ __device__ __forceinline__ void gather_fast_block(const Geom &g, const uint8_t *
     }
 }
 
-template <int TS>
-__global__ void __launch_bounds__(256) k_gather_fast(Geom g, const uint8_t *__restrict__ in, int64_t ld,
-                                                     uint8_t *__restrict__ img)
+// Items of a gather slice: a block's slices are of one size, about GA_ITEMS each unless `nbl` blocks in
+// fewer fill the `slots` of one wave (600 blocks of 100 x 200 float32: 0.030 ms whole, 0.036 in halves).
+static int gather_slice(const Geom &g, int64_t nbl, int64_t slots)
 {
-    const int64_t nsl = (g.blockn + GA_ITEMS - 1) / GA_ITEMS, nu = g.nchunks * g.nblocks * nsl;
-    for (int64_t u = blockIdx.x; u < nu; u += gridDim.x) {
-        int64_t t, sl;
-        divmod(u, nsl, t, sl);
-        gather_fast_block<TS>(g, in, ld, img, t, (int)sl * GA_ITEMS, (int)min((int64_t)GA_ITEMS, g.blockn - sl * GA_ITEMS));
+    const int64_t nsl = std::min(ceil_div(g.blockn, GA_ITEMS), std::max<int64_t>(slots / std::max<int64_t>(nbl, 1), 1));
+    return (int)round_up(ceil_div(g.blockn, nsl), 4);
+}
+// Threads that take a block: a power of two, a warp at least, a CTA at most.  Blocks of few items share
+// a CTA, which else would be all latency.
+static int gather_threads(const Geom &g)
+{
+    const int64_t n = geom_quads(g) ? g.blockn / 4 : g.blockn;
+    int nt = 32;
+    while (nt < 256 && nt < n) nt *= 2;
+    return nt;
+}
+// (A kernel for each of the two kinds of blocks, as both in one cost registers.  250,000 blocks of 8 x 8
+// float32: 0.73 ms with a CTA a block and one kernel for both, now 0.10; float64 0.80 and 0.11.)
+template <int TS, bool QUADS>
+__global__ void __launch_bounds__(256, !QUADS ? 4 : TS == 8 ? 6 : 8) k_gather_fast(Geom g, const uint8_t *__restrict__ in, int64_t ld,
+                                                                               uint8_t *__restrict__ img, int slice, int nt)
+{
+    const int64_t nsl = (g.blockn + slice - 1) / slice, nu = g.nchunks * g.nblocks * nsl;
+    const int per = 256 / nt, tid = threadIdx.x & (nt - 1);
+    for (int64_t u = (int64_t)blockIdx.x * per + threadIdx.x / nt; u < nu; u += (int64_t)gridDim.x * per) {
+        int64_t t = u, sl = 0;
+        if (nsl > 1) divmod(u, nsl, t, sl);
+        gather_fast_block<TS, QUADS>(g, in, ld, img, t, (int)sl * slice, (int)min((int64_t)slice, g.blockn - sl * slice), tid, nt);
     }
 }
 
@@ -2862,13 +2882,13 @@ int encode_gather(const Geom &g, const void *in, int64_t ld, bool shuffle, int s
     const int64_t blocks = std::min<int64_t>(nbl * tpb, (int64_t)sms * 8);
     const bool fast = shuffle && (ts == 4 || ts == 8);
     if (fast) {
-        const int64_t fb = std::min<int64_t>(nbl * ceil_div(g.blockn, GA_ITEMS), (int64_t)sms * 8);
-        if (ts == 8)
-            IAB_TIMED("k_gather_fast", st, k_gather_fast<8><<<(unsigned)std::max<int64_t>(fb, 1), 256, 0, st>>>(
-                g, (const uint8_t *)in, ld, img));
-        else
-            IAB_TIMED("k_gather_fast", st, k_gather_fast<4><<<(unsigned)std::max<int64_t>(fb, 1), 256, 0, st>>>(
-                g, (const uint8_t *)in, ld, img));
+        const int nt = gather_threads(g), slice = gather_slice(g, nbl, (int64_t)sms * 8);
+        const int64_t fb = std::min<int64_t>(ceil_div(nbl * ceil_div(g.blockn, slice), 256 / nt), (int64_t)sms * 8);
+        auto launch = [&](auto kernel) {
+            IAB_TIMED("k_gather_fast", st, kernel<<<(unsigned)std::max<int64_t>(fb, 1), 256, 0, st>>>(g, (const uint8_t *)in, ld, img, slice, nt));
+        };
+        if (ts == 8) launch(geom_quads(g) ? k_gather_fast<8, true> : k_gather_fast<8, false>);
+        else launch(geom_quads(g) ? k_gather_fast<4, true> : k_gather_fast<4, false>);
     } else {
         IAB_TIMED("k_gather", st, k_gather<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
             g, (const uint8_t *)in, ld, shuffle, img));
@@ -3364,14 +3384,21 @@ __global__ void __launch_bounds__(256) k_scatter_g(const CodecItem *__restrict__
     }
 }
 
+// (The group's blocks are of one size: `nsl` slices of `slice` items a block, `nt` threads a slice.)
 template <int TS>
 __global__ void __launch_bounds__(256) k_gather_fast_g(const CodecItem *__restrict__ items,
-                                                       const int64_t *__restrict__ bstart, int n, int64_t nbl)
+                                                       const int64_t *__restrict__ bstart, int n, int64_t nu, int nsl,
+                                                       int slice, int nt)
 {
-    for (int64_t u = blockIdx.x; u < nbl; u += gridDim.x) {
-        const int k = group_find(bstart, n, u);
+    const int per = 256 / nt, tid = threadIdx.x & (nt - 1);
+    for (int64_t u = (int64_t)blockIdx.x * per + threadIdx.x / nt; u < nu; u += (int64_t)gridDim.x * per) {
+        int64_t gb, sl;
+        divmod(u, nsl, gb, sl);
+        const int k = group_find(bstart, n, gb);
         const CodecItem &it = items[k];
-        gather_fast_block<TS>(it.g, it.dense, it.ld, it.img, u - bstart[k], 0, (int)it.g.blockn);
+        const int i0 = (int)sl * slice, cnt = (int)min((int64_t)slice, it.g.blockn - i0);
+        if (geom_quads(it.g)) gather_fast_block<TS, true>(it.g, it.dense, it.ld, it.img, gb - bstart[k], i0, cnt, tid, nt);
+        else gather_fast_block<TS, false>(it.g, it.dense, it.ld, it.img, gb - bstart[k], i0, cnt, tid, nt);
     }
 }
 
@@ -3585,12 +3612,16 @@ int encode_group_launch(CodecGroup *grp, bool exact_lz4, bool memcpy_only, cudaS
     if (grp->nbl == 0) return 0;
     cudaMemsetAsync(grp->counters.p, 0, 128, st);
     const bool fast = grp->shuffle && (ts == 4 || ts == 8);
-    const int64_t gb = std::max<int64_t>(std::min<int64_t>(grp->nbl, (int64_t)sms * 8), 1);
     if (fast && !grp->img_ready) {
+        const int slice = gather_slice(grp->h[0].g, grp->nbl, (int64_t)sms * 8);
+        const int64_t nsl = ceil_div(grp->h[0].g.blockn, slice), nu = grp->nbl * nsl;
+        int nt = 32;                              // as many as the group's widest need (rows of whole quads or not)
+        for (const CodecItem &it : grp->h) nt = std::max(nt, gather_threads(it.g));
+        const unsigned gb = (unsigned)std::min<int64_t>(ceil_div(nu, 256 / nt), (int64_t)sms * 8);
         if (ts == 8)
-            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<8><<<(unsigned)gb, 256, 0, st>>>(items, bstart, n, grp->nbl));
+            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<8><<<gb, 256, 0, st>>>(items, bstart, n, nu, (int)nsl, slice, nt));
         else
-            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<4><<<(unsigned)gb, 256, 0, st>>>(items, bstart, n, grp->nbl));
+            IAB_TIMED("k_gather_fast", st, k_gather_fast_g<4><<<gb, 256, 0, st>>>(items, bstart, n, nu, (int)nsl, slice, nt));
     }
     if (!fast && !grp->img_ready) {
         const int64_t tb = std::max<int64_t>(std::min<int64_t>(grp->nbl * grp->max_tpb, (int64_t)sms * 8), 1);
