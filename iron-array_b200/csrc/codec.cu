@@ -2567,17 +2567,17 @@ __global__ void __launch_bounds__(LAYOUT_T) k_layout(Geom g, int nstreams, int n
     chunk_offsets(g.nchunks, ec, tot, off, len, wsum);
 }
 
-// Copies len bytes with the whole CTA: 16-byte aligned stores to dst, each fed by five
+// Copies len bytes with nt threads (tid: this one's number): 16-byte aligned stores to dst, each fed by five
 // aligned 32-bit loads of src funnel-shifted into place.  Source words are only read
 // inside [lo, hi); pieces whose words would leave it are copied bytewise.
-__device__ __forceinline__ void cta_copy(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src, int len,
-                                         const uint8_t *lo, const uint8_t *hi)
+__device__ __forceinline__ void group_copy(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src, int len,
+                                           const uint8_t *lo, const uint8_t *hi, int tid, int nt)
 {
     int head = (int)((16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15);
     if (head > len) head = len;
-    for (int x = threadIdx.x; x < head; x += blockDim.x) dst[x] = __ldg(src + x);
+    for (int x = tid; x < head; x += nt) dst[x] = __ldg(src + x);
     const int nvec = (len - head) >> 4;
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
+    for (int v = tid; v < nvec; v += nt) {
         const int s = head + (v << 4);
         const uint8_t *sp = src + s;
         const uint8_t *sa = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(sp) & ~uintptr_t(3));
@@ -2599,16 +2599,27 @@ __device__ __forceinline__ void cta_copy(uint8_t *__restrict__ dst, const uint8_
         }
         *reinterpret_cast<uint4 *>(dst + s) = o;
     }
-    for (int x = head + (nvec << 4) + threadIdx.x; x < len; x += blockDim.x) dst[x] = __ldg(src + x);
+    for (int x = head + (nvec << 4) + tid; x < len; x += nt) dst[x] = __ldg(src + x);
 }
 
 // E5: write headers, bstarts, csize words and payloads.  One CTA per stream: where there are few
 // blocks the copies of their streams are under way together, where there are many the last ones
-// are shorter (300 x 200 float64 9 us, by one CTA per block 15; 8192 x 8192 0.19 ms, 0.26).
+// are shorter (300 x 200 float64 9 us, by one CTA per block 15; 8192 x 8192 0.19 ms, 0.26).  Streams
+// below EMIT_WARP bytes, where there are more of them than CTAs at once, take a warp each: a CTA spends
+// most of its time on the loads before the copy (4000 x 4000 float64 in blocks of 8 x 8, 2 million
+// streams: 3.6 ms by a CTA a stream, 0.57 by a CTA a block, 0.74 by warps; of 32 x 32 0.34, 0.36 and
+// 0.08; of 90 x 90 0.068, 0.072 and 0.058; of 128 x 128 0.052 by CTAs, 0.064 by warps).
+constexpr int EMIT_WARP = 8192;
+static int emit_threads(int64_t streams, int neblock, int sms) { return neblock < EMIT_WARP && streams > (int64_t)sms * 8 ? 32 : 256; }
+static unsigned emit_grid(int64_t streams, int nt, int sms)
+{
+    return (unsigned)std::max<int64_t>(std::min<int64_t>(ceil_div(streams, 256 / nt), (int64_t)sms * 8), 1);
+}
 __device__ __forceinline__ void emit_block(const Geom &g, int nstreams, int neblock, bool shuffle, int splitflag,
                                            const uint8_t *__restrict__ img, const uint8_t *__restrict__ slots,
                                            int64_t img_bytes, const EncStream *__restrict__ es,
-                                           const EncChunk *__restrict__ ec, uint8_t *__restrict__ outbuf, int64_t t, int j)
+                                           const EncChunk *__restrict__ ec, uint8_t *__restrict__ outbuf, int64_t t, int j,
+                                           int tid, int nt)
 {
     const int ts = g.itemsize;
     do {
@@ -2617,10 +2628,10 @@ __device__ __forceinline__ void emit_block(const Geom &g, int nstreams, int nebl
         const EncStream e = es[t * nstreams + j];      // (loaded beside the chunk's entry; unused when memcpyed)
         const EncChunk cc = ec[c];
         uint8_t *chunk = outbuf + cc.offset;
-        if (b == 0 && j == 0 && threadIdx.x < 32) {
+        if (b == 0 && j == 0 && tid < 32) {
             const int flags = 0x05 | (1 << 5) | (splitflag ? 0 : 0x10) | (cc.memcpyed ? 0x02 : 0);
             uint8_t hb = 0;
-            const int x = threadIdx.x;
+            const int x = tid;
             if (x == 0) hb = 5;
             else if (x == 1) hb = 1;
             else if (x == 2) hb = (uint8_t)flags;
@@ -2635,7 +2646,7 @@ __device__ __forceinline__ void emit_block(const Geom &g, int nstreams, int nebl
         const uint8_t *blk_img = img + t * g.blocksize;
         if (cc.memcpyed) {
             uint8_t *dst = chunk + 32 + b * g.blocksize;
-            for (int64_t x = (int64_t)j * neblock + threadIdx.x; x < (int64_t)(j + 1) * neblock; x += blockDim.x) {
+            for (int64_t x = (int64_t)j * neblock + tid; x < (int64_t)(j + 1) * neblock; x += nt) {
                 uint8_t v;
                 if (shuffle) { const int64_t i = x / ts, k = x - i * ts; v = blk_img[k * g.blockn + i]; }
                 else v = blk_img[x];
@@ -2643,7 +2654,7 @@ __device__ __forceinline__ void emit_block(const Geom &g, int nstreams, int nebl
             }
             continue;
         }
-        if (j == 0 && threadIdx.x < 4) chunk[32 + 4 * b + threadIdx.x] = (uint8_t)((uint32_t)e.out >> (8 * threadIdx.x));
+        if (j == 0 && tid < 4) chunk[32 + 4 * b + tid] = (uint8_t)((uint32_t)e.out >> (8 * tid));
         uint8_t *w = chunk + e.out;
         int32_t word;
         const uint8_t *payload = nullptr;
@@ -2651,25 +2662,27 @@ __device__ __forceinline__ void emit_block(const Geom &g, int nstreams, int nebl
         if (e.kind == SK_RUN) { word = -e.csize; }
         else if (e.kind == SK_LZ4) { word = e.csize; payload = slots + (t * nstreams + j) * (int64_t)neblock; plen = e.csize; }
         else { word = neblock; payload = blk_img + (int64_t)j * neblock; plen = neblock; }
-        if (threadIdx.x < 4) w[threadIdx.x] = (uint8_t)((uint32_t)word >> (8 * threadIdx.x));
-        if (e.kind == SK_RUN && e.csize != 0 && threadIdx.x == 4) w[4] = 1;
+        if (tid < 4) w[tid] = (uint8_t)((uint32_t)word >> (8 * tid));
+        if (e.kind == SK_RUN && e.csize != 0 && tid == 4) w[4] = 1;
         if (plen > 0) {
             const uint8_t *base = e.kind == SK_LZ4 ? slots : img;
-            cta_copy(w + 4, payload, plen, base, base + img_bytes);
+            group_copy(w + 4, payload, plen, base, base + img_bytes, tid, nt);
         }
     } while (false);
 }
 
+template <int NT>
 __global__ void __launch_bounds__(256) k_emit(Geom g, int nstreams, int neblock, bool shuffle, int splitflag,
                                               const uint8_t *__restrict__ img, const uint8_t *__restrict__ slots,
                                               int64_t img_bytes,
                                               const EncStream *__restrict__ es, const EncChunk *__restrict__ ec,
                                               uint8_t *__restrict__ outbuf)
 {
-    for (int64_t u = blockIdx.x; u < g.nchunks * g.nblocks * nstreams; u += gridDim.x) {
+    constexpr int per = 256 / NT;
+    for (int64_t u = (int64_t)blockIdx.x * per + threadIdx.x / NT; u < g.nchunks * g.nblocks * nstreams; u += (int64_t)gridDim.x * per) {
         int64_t t, j;
         divmod(u, nstreams, t, j);
-        emit_block(g, nstreams, neblock, shuffle, splitflag, img, slots, img_bytes, es, ec, outbuf, t, (int)j);
+        emit_block(g, nstreams, neblock, shuffle, splitflag, img, slots, img_bytes, es, ec, outbuf, t, (int)j, threadIdx.x % NT, NT);
     }
 }
 
@@ -2944,8 +2957,9 @@ int encode_emit(const Geom &g, bool shuffle, int splitmode, DevBuf *d_out, Encod
     IAB_TIMED("k_layout", st, k_layout<<<(unsigned)std::max<int64_t>(g.nchunks, 1), LAYOUT_T, 0, st>>>(
         g, nstreams, neblock, es, ec, w->memcpy_only ? 1 : 0, w->tot.as<int64_t>(), w->d_off.as<int64_t>(),
         w->d_len.as<int32_t>()));
-    const int64_t blocks = std::min<int64_t>(nbl * nstreams, (int64_t)sm_count() * 8);
-    IAB_TIMED("k_emit", st, k_emit<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
+    const int nt = emit_threads(nbl * nstreams, neblock, sm_count());
+    auto *emit = nt == 32 ? k_emit<32> : k_emit<256>;
+    IAB_TIMED("k_emit", st, emit<<<emit_grid(nbl * nstreams, nt, sm_count()), 256, 0, st>>>(
         g, nstreams, neblock, shuffle, encode_split(g, shuffle, splitmode) ? 1 : 0, img, slots, img_bytes, es, ec,
         d_out->as<uint8_t>()));
     return 0;
@@ -3435,17 +3449,19 @@ __global__ void __launch_bounds__(1024) k_chunk_offsets_g(CodecItem *items)
     chunk_offsets(it.g.nchunks, it.ec, &it.out_bytes, nullptr, nullptr, wsum);
 }
 
+template <int NT>
 __global__ void __launch_bounds__(256) k_emit_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart,
                                                 int n, int64_t nbl, int nstreams, int neblock, bool shuffle, int splitflag)
 {
-    for (int64_t u = blockIdx.x; u < nbl * nstreams; u += gridDim.x) {
+    constexpr int per = 256 / NT;
+    for (int64_t u = (int64_t)blockIdx.x * per + threadIdx.x / NT; u < nbl * nstreams; u += (int64_t)gridDim.x * per) {
         int64_t t, j;
         divmod(u, nstreams, t, j);
         const int k = group_find(bstart, n, t);
         const CodecItem &it = items[k];
         const int64_t img_bytes = it.g.nchunks * it.g.nblocks * it.g.blocksize;
         emit_block(it.g, nstreams, neblock, shuffle, splitflag, it.img, it.slots, img_bytes, it.es, it.ec, it.outbuf,
-                   t - bstart[k], (int)j);
+                   t - bstart[k], (int)j, threadIdx.x % NT, NT);
     }
 }
 
@@ -3634,8 +3650,10 @@ int encode_group_launch(CodecGroup *grp, bool exact_lz4, bool memcpy_only, cudaS
     IAB_TIMED("k_layout", st, k_layout_g<<<(unsigned)std::max<int64_t>(grp->nch, 1), LAYOUT_T, 0, st>>>(
         items, cstart, n, grp->nstreams, grp->neblock, memcpy_only ? 1 : 0));
     IAB_TIMED("k_chunk_offsets", st, k_chunk_offsets_g<<<(unsigned)n, 1024, 0, st>>>(items));
-    IAB_TIMED("k_emit", st, k_emit_g<<<(unsigned)std::min<int64_t>(grp->nbl * grp->nstreams, (int64_t)sms * 8), 256, 0, st>>>(items, bstart, n, grp->nbl, grp->nstreams, grp->neblock,
-                                                                   grp->shuffle, grp->split ? 1 : 0));
+    const int nt = emit_threads(grp->nbl * grp->nstreams, grp->neblock, sms);
+    auto *emit = nt == 32 ? k_emit_g<32> : k_emit_g<256>;
+    IAB_TIMED("k_emit", st, emit<<<emit_grid(grp->nbl * grp->nstreams, nt, sms), 256, 0, st>>>(
+        items, bstart, n, grp->nbl, grp->nstreams, grp->neblock, grp->shuffle, grp->split ? 1 : 0));
     return 0;
 }
 
