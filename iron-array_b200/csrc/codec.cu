@@ -97,6 +97,7 @@ __device__ __forceinline__ BlockSpan block_span(const Geom &g, int64_t c, int64_
 // blocks of 150 x 100, whose rule needs the dense matrix, 0.487 -> 0.35).
 struct ParsedStream {
     bool lz4;                  // an LZ4 stream
+    bool general;              // lane 0 of a block that the fast scatter does not take
     int32_t q, cs, neblock;    // its payload's place in the chunk, its size, its output's
     const uint8_t *chunk;
 };
@@ -220,6 +221,7 @@ __device__ __forceinline__ void parse_block(const Geom &g, const uint8_t *__rest
         sd[t * 8 + j] = d;
     }
     ps.lz4 = valid && kind == SK_LZ4;
+    ps.general = valid && j == 0 && !(mode == BM_SHUFFLED && nstreams == g.itemsize);
     ps.q = at; ps.cs = slen; ps.neblock = neblock; ps.chunk = p;
 }
 
@@ -252,8 +254,8 @@ __device__ __forceinline__ void queue_streams(const ParsedStream &ps, uint8_t *b
 constexpr int PARSE_T = 128;
 __global__ void __launch_bounds__(PARSE_T) k_parse(Geom g, const uint8_t *__restrict__ ch, const int64_t *__restrict__ off,
                                                    const int32_t *__restrict__ len, BlockDesc *bd, StreamDesc *sd,
-                                                   Lz4Job *jobs, int *njobs, int64_t jcap, int *err, uint8_t *scratch,
-                                                   uint8_t *zf, int *nzero)
+                                                   Lz4Job *jobs, int *njobs, int64_t jcap, int *err, int *ngeneral,
+                                                   uint8_t *scratch, uint8_t *zf, int *nzero)
 {
     const int64_t total = g.nchunks * g.nblocks;
     for (int64_t t0 = (int64_t)blockIdx.x * (PARSE_T / 8); t0 < total; t0 += (int64_t)gridDim.x * (PARSE_T / 8)) {
@@ -261,6 +263,8 @@ __global__ void __launch_bounds__(PARSE_T) k_parse(Geom g, const uint8_t *__rest
         ParsedStream ps;
         parse_block(g, ch, off, len, bd, sd, err, zf, nzero, t, t < total, ps);
         queue_streams(ps, scratch + t * g.blocksize, err, jobs, njobs, jcap);
+        const unsigned m = __ballot_sync(FULLMASK, ps.general);
+        if (m && (threadIdx.x & 31) == 0) atomicAdd(ngeneral, __popc(m));
     }
 }
 static unsigned parse_grid(int64_t nbl, int sms)
@@ -821,6 +825,11 @@ __device__ __forceinline__ void scatter_tile(const Geom &g, const uint8_t *__res
                 for (int x = threadIdx.x; x < cnt; x += blockDim.x) pl[x] = __ldcg(src + x);
             }
         }
+    } else if (d.mode == BM_PLAIN && d.nstreams == 1) {          // (stored as it is, or one stream)
+        const StreamDesc q = s[0];
+        const uint8_t *src = q.kind == SK_RAW ? ch + q.src + i0 * ts : blk_scratch + i0 * ts;
+        for (int x = threadIdx.x; x < cnt * ts; x += blockDim.x)
+            planes[x] = q.kind == SK_RUN ? (uint8_t)q.len : __ldcg(src + x);
     } else if (d.mode == BM_PLAIN) {
         for (int x = threadIdx.x; x < cnt * ts; x += blockDim.x) {
             const int64_t pos = i0 * ts + x;
@@ -1041,12 +1050,51 @@ __device__ __forceinline__ bool scatter_fast_unit(const Geom &g, const uint8_t *
     return true;
 }
 
+// D2 general path over the blocks that the fast one does not take: those that are not shuffled in
+// fast_streams streams, *ngeneral of them as counted by the parse; every block where fast_streams is 0.
+__device__ __forceinline__ void scatter_general(const Geom &g, int fast_streams, const int *ngeneral, const uint8_t *__restrict__ ch,
+                                                const BlockDesc *__restrict__ bd, const StreamDesc *__restrict__ sd,
+                                                const uint8_t *__restrict__ scratch, uint8_t *__restrict__ out, int64_t ld,
+                                                uint8_t *planes)
+{
+    if (fast_streams && !__ldg(ngeneral)) return;
+    const int64_t tpb = (g.blockn + TILE - 1) / TILE;
+    const int64_t nwork = g.nchunks * g.nblocks * tpb;
+    // Up to 32 tiles are looked at together, a lane each, the same in every warp.  The groups are an
+    // even division of a CTA's share, for where the fast path took none.
+    const int64_t share = (nwork + gridDim.x - 1) / gridDim.x, rounds = (share + 31) / 32;
+    const int group = (int)((share + rounds - 1) / rounds);
+    const int lane = threadIdx.x & 31;
+    for (int64_t w0 = (int64_t)blockIdx.x * group; w0 < nwork; w0 += (int64_t)gridDim.x * group) {
+        int64_t t = 0, i0 = 0;
+        bool mine = lane < group && w0 + lane < nwork;
+        if (mine) {
+            divmod(w0 + lane, tpb, t, i0);
+            mine = !(bd[t].mode == BM_SHUFFLED && bd[t].nstreams == fast_streams);
+        }
+        for (unsigned m = __ballot_sync(FULLMASK, mine); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            scatter_tile(g, ch, bd, sd, scratch, out, ld, __shfl_sync(FULLMASK, t, l), __shfl_sync(FULLMASK, i0, l) * TILE,
+                         planes);
+        }
+    }
+}
+// (Not inlined into the fast kernel, whose registers it would make spill.  By tiles rather than the fast
+// kernel's slices: 200 x 200 float64 stored as they are, in blocks of 100 x 200: 0.070 ms inlined and by
+// slices, 0.019 now, 0.027 by two launches.)
+__device__ __noinline__ void scatter_general_call(const Geom &g, int fast_streams, const int *ngeneral, const uint8_t *ch,
+                                                  const BlockDesc *bd, const StreamDesc *sd, const uint8_t *scratch,
+                                                  uint8_t *out, int64_t ld, uint8_t *planes)
+{
+    scatter_general(g, fast_streams, ngeneral, ch, bd, sd, scratch, out, ld, planes);
+}
+
 template <int TS, bool ALL>
-__global__ void __launch_bounds__(256, 6) k_scatter_fast(Geom g, const uint8_t *__restrict__ ch, const uint8_t *ch_end,
-                                                      const BlockDesc *__restrict__ bd,
+__global__ void __launch_bounds__(256, 6) k_scatter_fast(const __grid_constant__ Geom g, const uint8_t *__restrict__ ch,
+                                                      const uint8_t *ch_end, const BlockDesc *__restrict__ bd,
                                                       const StreamDesc *__restrict__ sd,
                                                       const uint8_t *__restrict__ scratch, const uint8_t *scratch_end,
-                                                      uint8_t *__restrict__ out, int64_t ld, int *err)
+                                                      uint8_t *__restrict__ out, int64_t ld, int *err, const int *ngeneral)
 {
     __shared__ __align__(128) uint8_t stage[TS][SC_PLANE];
     __shared__ __align__(8) uint64_t bar;
@@ -1070,43 +1118,17 @@ __global__ void __launch_bounds__(256, 6) k_scatter_fast(Geom g, const uint8_t *
                                    stage, &bar, parity, &abort_all, general))
             return;
     }
-    // the blocks of other kinds among this CTA's slices (no bulk copy follows: the stage is free)
-    for (int64_t u = blockIdx.x; ALL && general && u < nbl * nsl; u += gridDim.x) {
-        int64_t t, sl;
-        divmod(u, nsl, t, sl);
-        if (bd[t].mode == BM_SHUFFLED && bd[t].nstreams == TS) continue;
-        const int64_t end = min(g.blockn, (sl + 1) * SC_ITEMS);
-        for (int64_t i0 = sl * SC_ITEMS; i0 < end; i0 += TILE)
-            scatter_tile(g, ch, bd, sd, scratch, out, ld, t, i0, stage[0]);
-    }
+    // the blocks of other kinds (no bulk copy follows: the stage is free)
+    if (ALL && __ldg(ngeneral)) scatter_general_call(g, TS, ngeneral, ch, bd, sd, scratch, out, ld, stage[0]);
 }
 
-__global__ void __launch_bounds__(256) k_scatter(Geom g, int fast_streams, const uint8_t *__restrict__ ch,
+__global__ void __launch_bounds__(256, 8) k_scatter(const __grid_constant__ Geom g, int fast_streams, const uint8_t *__restrict__ ch,
                                                  const BlockDesc *__restrict__ bd, const StreamDesc *__restrict__ sd,
-                                                 const uint8_t *__restrict__ scratch, uint8_t *__restrict__ out, int64_t ld)
+                                                 const uint8_t *__restrict__ scratch, uint8_t *__restrict__ out, int64_t ld,
+                                                 const int *ngeneral)
 {
     __shared__ __align__(16) uint8_t planes[8 * TILE];
-    const int64_t tpb = (g.blockn + TILE - 1) / TILE;
-    const int64_t nwork = g.nchunks * g.nblocks * tpb;
-    // Up to 32 tiles are looked at together, a lane each, the same in every warp: where k_scatter_fast
-    // took them all, that look is the whole kernel.  The groups are an even division of a CTA's
-    // share, for where it took none.
-    const int64_t share = (nwork + gridDim.x - 1) / gridDim.x, rounds = (share + 31) / 32;
-    const int group = (int)((share + rounds - 1) / rounds);
-    const int lane = threadIdx.x & 31;
-    for (int64_t w0 = (int64_t)blockIdx.x * group; w0 < nwork; w0 += (int64_t)gridDim.x * group) {
-        int64_t t = 0, i0 = 0;
-        bool mine = lane < group && w0 + lane < nwork;
-        if (mine) {
-            divmod(w0 + lane, tpb, t, i0);
-            mine = !(bd[t].mode == BM_SHUFFLED && bd[t].nstreams == fast_streams);
-        }
-        for (unsigned m = __ballot_sync(FULLMASK, mine); m; m &= m - 1) {
-            const int l = __ffs(m) - 1;
-            scatter_tile(g, ch, bd, sd, scratch, out, ld, __shfl_sync(FULLMASK, t, l), __shfl_sync(FULLMASK, i0, l) * TILE,
-                         planes);
-        }
-    }
+    scatter_general(g, fast_streams, ngeneral, ch, bd, sd, scratch, out, ld, planes);
 }
 
 // ============================================================================ encode
@@ -2759,9 +2781,10 @@ int decode_finish(DecodeWork *w, cudaStream_t st)
     return h[1];
 }
 
-// Grid of the fast scatter: the CTAs resident at once (one wave), at most one per slice.
+// Grid of the fast scatter: the CTAs resident at once (one wave), at most one per slice, or per tile
+// where it also takes the general path.
 template <int TS>
-static int64_t scatter_fast_grid(const Geom &g, int64_t nbl)
+static int64_t scatter_fast_grid(const Geom &g, int64_t nbl, bool all)
 {
     static int per_sm = 0;
     if (!per_sm) {
@@ -2772,7 +2795,7 @@ static int64_t scatter_fast_grid(const Geom &g, int64_t nbl)
         }
         per_sm = n;
     }
-    const int64_t units = nbl * ((g.blockn + SC_ITEMS - 1) / SC_ITEMS);
+    const int64_t units = nbl * ceil_div(g.blockn, all ? TILE : SC_ITEMS);
     return std::max<int64_t>(std::min<int64_t>(units, (int64_t)sm_count() * per_sm), 1);
 }
 
@@ -2811,7 +2834,7 @@ int decode_parse(const DecodeArgs &a, DecodeQueue *q, DecodeWork *w, cudaStream_
     if (!w->zf.allocate((size_t)std::max<int64_t>(nbl, 1), dev)) return -100;
     IAB_TIMED("k_parse", st, k_parse<<<parse_grid(nbl, sm_count()), PARSE_T, 0, st>>>(
         g, a.chunks, a.off, a.len, w->bd.as<BlockDesc>(), w->sd.as<StreamDesc>(), q->jobs.as<Lz4Job>(),
-        q->counters.as<int>(), q->cap, cnt + 1, w->scratch.as<uint8_t>(), w->zf.as<uint8_t>(), cnt + 4));
+        q->counters.as<int>(), q->cap, cnt + 1, cnt + 2, w->scratch.as<uint8_t>(), w->zf.as<uint8_t>(), cnt + 4));
     return 0;
 }
 
@@ -2830,36 +2853,36 @@ int decode_lz4(DecodeQueue *q, cudaStream_t st)
 }
 
 // The decoded streams to the dense array.  Small containers by one launch, the blocks the fast
-// path does not take included; from SC_SPLIT bytes on those have a launch of their own, because
-// the registers of the kernel that holds both paths spill: 0.81 against 0.86 ms for three 512 MiB
-// float64 arrays, where the launch that mostly finds nothing costs 6 us.  Items of 1 and 2 bytes
-// go by the general path.
-constexpr int64_t SC_SPLIT = int64_t(64) << 20;
+// path does not take included; from SC_SPLIT bytes on those have a launch of their own, which finds
+// nothing in 5 us in most containers (4000 x 4000 float32 66 -> 70 us), but writes them with the
+// registers and CTAs that they need (the same array stored as it is 0.31 -> 0.21 ms).
+// Items of 1 and 2 bytes go by the general path.
+constexpr int64_t SC_SPLIT = int64_t(32) << 20;
 template <int TS>
 static void scatter_launch(const Geom &g, bool all, const uint8_t *chunks, const uint8_t *cend, const BlockDesc *bd,
                            const StreamDesc *sd, const uint8_t *scratch, const uint8_t *send, void *out, int64_t ld, int *err,
-                           cudaStream_t st)
+                           const int *ngeneral, cudaStream_t st)
 {
-    const unsigned grid = (unsigned)scatter_fast_grid<TS>(g, g.nchunks * g.nblocks);
+    const unsigned grid = (unsigned)scatter_fast_grid<TS>(g, g.nchunks * g.nblocks, all);
     if (all)
         IAB_TIMED("k_scatter_fast", st, k_scatter_fast<TS, true><<<grid, 256, 0, st>>>(
-            g, chunks, cend, bd, sd, scratch, send, (uint8_t *)out, ld, err));
+            g, chunks, cend, bd, sd, scratch, send, (uint8_t *)out, ld, err, ngeneral));
     else
         IAB_TIMED("k_scatter_fast", st, k_scatter_fast<TS, false><<<grid, 256, 0, st>>>(
-            g, chunks, cend, bd, sd, scratch, send, (uint8_t *)out, ld, err));
+            g, chunks, cend, bd, sd, scratch, send, (uint8_t *)out, ld, err, ngeneral));
 }
 static void scatter_launch(const Geom &g, const uint8_t *chunks, int64_t chunks_bytes, const BlockDesc *bd, const StreamDesc *sd,
-                           const uint8_t *scratch, void *out, int64_t ld, int *err, cudaStream_t st)
+                           const uint8_t *scratch, void *out, int64_t ld, int *err, const int *ngeneral, cudaStream_t st)
 {
     const int64_t nbl = g.nchunks * g.nblocks;
     const uint8_t *cend = chunks + chunks_bytes, *send = scratch + nbl * g.blocksize;
     const bool fast = g.itemsize == 8 || g.itemsize == 4, all = fast && nbl * g.blocksize < SC_SPLIT;
-    if (g.itemsize == 8) scatter_launch<8>(g, all, chunks, cend, bd, sd, scratch, send, out, ld, err, st);
-    else if (g.itemsize == 4) scatter_launch<4>(g, all, chunks, cend, bd, sd, scratch, send, out, ld, err, st);
+    if (g.itemsize == 8) scatter_launch<8>(g, all, chunks, cend, bd, sd, scratch, send, out, ld, err, ngeneral, st);
+    else if (g.itemsize == 4) scatter_launch<4>(g, all, chunks, cend, bd, sd, scratch, send, out, ld, err, ngeneral, st);
     if (!all) {
         const int64_t blocks = std::min<int64_t>(nbl * ceil_div(g.blockn, TILE), (int64_t)sm_count() * 8);
         IAB_TIMED("k_scatter", st, k_scatter<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
-            g, fast ? g.itemsize : 0, chunks, bd, sd, scratch, (uint8_t *)out, ld));
+            g, fast ? g.itemsize : 0, chunks, bd, sd, scratch, (uint8_t *)out, ld, ngeneral));
     }
 }
 
@@ -2867,7 +2890,7 @@ int decode_scatter(const DecodeArgs &a, DecodeWork *w, cudaStream_t st)
 {
     int *cnt = w->ext_counters ? w->ext_counters : w->counters.as<int>();
     scatter_launch(a.g, a.chunks, a.chunks_bytes, w->bd.as<BlockDesc>(), w->sd.as<StreamDesc>(), w->scratch.as<uint8_t>(),
-                   a.out, a.ld, cnt + 1, st);
+                   a.out, a.ld, cnt + 1, cnt + 2, st);
     return 0;
 }
 
@@ -3762,19 +3785,19 @@ int decode_noalloc(const Geom &g, const uint8_t *d_chunks, int64_t chunks_bytes,
     StreamDesc *sd = reinterpret_cast<StreamDesc *>(base + NA_SD);
     Lz4Job *jobs = reinterpret_cast<Lz4Job *>(base + NA_JOBS);
     uint8_t *img = base + NA_IMG;
-    int *njobs = counters, *err = counters + 9;
+    int *njobs = counters, *err = counters + 9, *ngeneral = counters + 10;
     // the job count, the status word and the job cursor must start at zero; descriptors,
     // the chunk index and the image are fully rewritten before they are read
     if (cudaMemsetAsync(counters, 0, 64, st) != cudaSuccess) return -101;
     const int sms = sm_count();
     IAB_TIMED("k_chunk_walk", st, k_chunk_walk<<<1, 32, 0, st>>>(d_chunks, chunks_bytes, g.nchunks, off, len));
     IAB_TIMED("k_parse", st, k_parse<<<parse_grid(nbl, sms), PARSE_T, 0, st>>>(g, d_chunks, off, len, bd, sd, jobs, njobs,
-                                                                              8 * NA_MAX_BLOCKS, err, img, nullptr, nullptr));
+                                                                              8 * NA_MAX_BLOCKS, err, ngeneral, img, nullptr, nullptr));
     {
         IAB_TIMED("k_lz4_decode_cta", st, k_lz4_decode_cta<<<sms * 6, dcta::THREADS, (int)sizeof(dcta::Smem), st>>>(
             jobs, njobs, 8 * NA_MAX_BLOCKS, reinterpret_cast<unsigned *>(counters + 8)));
     }
-    scatter_launch(g, d_chunks, chunks_bytes, bd, sd, img, out, ld, err, st);
+    scatter_launch(g, d_chunks, chunks_bytes, bd, sd, img, out, ld, err, ngeneral, st);
     // a launch that failed (a bad configuration, or an error left by earlier work) never
     // wrote the status word: report it instead of the zero it still holds
     if (cudaPeekAtLastError() != cudaSuccess) return -101;
