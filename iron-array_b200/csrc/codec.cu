@@ -1298,9 +1298,6 @@ __device__ __forceinline__ uint32_t probe_offset(uint32_t t)
 // 32 bytes never wrap.  The window follows the parse position; reads outside it (far search
 // probes, old match candidates) go to global memory.  Without it the candidate reads of
 // low-entropy streams, spread over the last few KiB, mostly miss L1.
-#ifndef XRING_
-#define XRING_ 4096
-#endif
 // The liblz4-identical encoder's warps (one per CTA) hold 16 KiB of table each; with a 2 KiB
 // window eleven of them fit an SM (f32 blocks of 125 x 150, 5000 x 6000 product: 0.98 ms; ten
 // with 4 KiB windows 1.26 ms, twelve with 1 KiB 0.91 ms there but 1.02x the time on 64 KiB
@@ -1860,7 +1857,7 @@ __global__ void __launch_bounds__(32, XCTAS) k_lz4_encode(const uint8_t *__restr
 //     match of PCAP bytes or more, which is extended exactly before it is written.
 // The bytes of the next window are loaded before B and stored after it; literal runs of more than
 // 16 bytes are copied by a warp.
-// What bounds it: the latency of a window's steps (seven streams an SM, each a chain of some
+// What bounds it: the latency of a window's steps (eight streams an SM, each a chain of some
 // 25,000 cycles per window; 45% of the issue slots), and where zero padding makes every match long,
 // the measuring of lengths, once 46,000 of a window's 68,000 cycles and now 16,000 of 40,000.  A batch
 // of 40 float64 products with extents of 64 to 2048: 14.7 -> 13.2 ms; the 16384 x 16384 float32
@@ -3435,20 +3432,6 @@ __global__ void __launch_bounds__(256, 4) k_scatter_fast_g(const CodecItem *__re
     }
 }
 
-// General scatter over every block.
-__global__ void __launch_bounds__(256) k_scatter_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart,
-                                                   int n, int64_t nbl, int64_t tpb)
-{
-    __shared__ __align__(16) uint8_t planes[8 * TILE];
-    for (int64_t w = blockIdx.x; w < nbl * tpb; w += gridDim.x) {
-        const int64_t gb = w / tpb, i0 = (w - gb * tpb) * TILE;
-        const int k = group_find(bstart, n, gb);
-        const CodecItem &it = items[k];
-        if (i0 >= it.g.blockn) continue;
-        scatter_tile(it.g, it.ch, it.bd, it.sd, it.scratch, it.dense, it.ld, gb - bstart[k], i0, planes);
-    }
-}
-
 // (The group's blocks are of one size: `nsl` slices of `slice` items a block, `nt` threads a slice.)
 template <int TS>
 __global__ void __launch_bounds__(256) k_gather_fast_g(const CodecItem *__restrict__ items,
@@ -3464,19 +3447,6 @@ __global__ void __launch_bounds__(256) k_gather_fast_g(const CodecItem *__restri
         const int i0 = (int)sl * slice, cnt = (int)min((int64_t)slice, it.g.blockn - i0);
         if (geom_quads(it.g)) gather_fast_block<TS, true>(it.g, it.dense, it.ld, it.img, gb - bstart[k], i0, cnt, tid, nt);
         else gather_fast_block<TS, false>(it.g, it.dense, it.ld, it.img, gb - bstart[k], i0, cnt, tid, nt);
-    }
-}
-
-__global__ void __launch_bounds__(256) k_gather_g(const CodecItem *__restrict__ items, const int64_t *__restrict__ bstart,
-                                                  int n, int64_t nbl, int64_t tpb, bool shuffle)
-{
-    __shared__ __align__(16) uint8_t planes[8 * TILE];
-    for (int64_t w = blockIdx.x; w < nbl * tpb; w += gridDim.x) {
-        const int64_t gb = w / tpb, i0 = (w - gb * tpb) * TILE;
-        const int k = group_find(bstart, n, gb);
-        const CodecItem &it = items[k];
-        if (i0 >= it.g.blockn) continue;
-        gather_tile(it.g, it.dense, it.ld, shuffle, it.img, gb - bstart[k], i0, planes);
     }
 }
 
@@ -3550,14 +3520,13 @@ int decode_group_setup(const std::vector<DecodeArgs> &a, const std::vector<int *
     if (n <= 0 || cnt.size() != a.size()) return -102;
     grp->n = n;
     grp->ts = a[0].g.itemsize;
+    if (grp->ts != 4 && grp->ts != 8) return -102;
     int64_t nbl = 0, img = 0, jobs = 0;
-    grp->max_tpb = 1;
     for (const DecodeArgs &x : a) {
         if (x.g.itemsize != grp->ts) return 1;
         nbl += x.g.nchunks * x.g.nblocks;
         img += x.g.nchunks * x.g.nblocks * x.g.blocksize;
         jobs += decode_max_jobs(x.g);
-        grp->max_tpb = std::max<int64_t>(grp->max_tpb, (x.g.blockn + TILE - 1) / TILE);
     }
     if (!grp->bd.allocate(sizeof(BlockDesc) * (size_t)std::max<int64_t>(nbl, 1), dev) ||
         !grp->sd.allocate(sizeof(StreamDesc) * 8 * (size_t)std::max<int64_t>(nbl, 1), dev) ||
@@ -3596,30 +3565,22 @@ int decode_group_launch(CodecGroup *grp, cudaStream_t st)
                                                                      grp->q.counters.as<int>(), grp->q.cap));
     int r = decode_lz4(&grp->q, st);
     if (r) return r;
-    const bool fast = grp->ts == 4 || grp->ts == 8;
-    if (fast) {
-        static int per_sm[2] = {0, 0};
-        const int slot = grp->ts == 8;
-        if (!per_sm[slot]) {
-            int m = 0;
-            const cudaError_t e = slot ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_scatter_fast_g<8>, 256, 0)
-                                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_scatter_fast_g<4>, 256, 0);
-            if (e != cudaSuccess || m < 1) { cudaGetLastError(); m = 4; }
-            per_sm[slot] = m;
-        }
-        const int64_t grid = std::max<int64_t>(std::min<int64_t>(grp->nsf, (int64_t)sms * per_sm[slot]), 1);
-        if (slot)
-            IAB_TIMED("k_scatter_fast", st, k_scatter_fast_g<8><<<(unsigned)grid, 256, 0, st>>>(
-                items, sstart, n, grp->nsf));
-        else
-            IAB_TIMED("k_scatter_fast", st, k_scatter_fast_g<4><<<(unsigned)grid, 256, 0, st>>>(
-                items, sstart, n, grp->nsf));
+    static int per_sm[2] = {0, 0};
+    const int slot = grp->ts == 8;
+    if (!per_sm[slot]) {
+        int m = 0;
+        const cudaError_t e = slot ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_scatter_fast_g<8>, 256, 0)
+                                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_scatter_fast_g<4>, 256, 0);
+        if (e != cudaSuccess || m < 1) { cudaGetLastError(); m = 4; }
+        per_sm[slot] = m;
     }
-    if (!fast) {
-        const int64_t sb = std::min<int64_t>(grp->nbl * grp->max_tpb, (int64_t)sms * 8);
-        IAB_TIMED("k_scatter", st, k_scatter_g<<<(unsigned)std::max<int64_t>(sb, 1), 256, 0, st>>>(
-            items, bstart, n, grp->nbl, grp->max_tpb));
-    }
+    const int64_t grid = std::max<int64_t>(std::min<int64_t>(grp->nsf, (int64_t)sms * per_sm[slot]), 1);
+    if (slot)
+        IAB_TIMED("k_scatter_fast", st, k_scatter_fast_g<8><<<(unsigned)grid, 256, 0, st>>>(
+            items, sstart, n, grp->nsf));
+    else
+        IAB_TIMED("k_scatter_fast", st, k_scatter_fast_g<4><<<(unsigned)grid, 256, 0, st>>>(
+            items, sstart, n, grp->nsf));
     return 0;
 }
 
@@ -3633,11 +3594,11 @@ int encode_group_setup(const std::vector<Geom> &g, const std::vector<const void 
         return -102;
     grp->n = n;
     grp->ts = g[0].itemsize;
+    if (grp->ts != 4 && grp->ts != 8) return -102;
     grp->shuffle = true;
     grp->nstreams = encode_nstreams(g[0], true, 3 /* automatic split */);
     grp->split = encode_split(g[0], true, 3);
     grp->neblock = (int)(g[0].blocksize / grp->nstreams);
-    grp->max_tpb = 1;
     int64_t img = 0, ns = 0;
     for (const Geom &x : g) {
         const int nsx = encode_nstreams(x, true, 3);
@@ -3646,7 +3607,6 @@ int encode_group_setup(const std::vector<Geom> &g, const std::vector<const void 
             return 1;
         img += x.nchunks * x.nblocks * x.blocksize;
         ns += x.nchunks * x.nblocks * nsx;
-        grp->max_tpb = std::max<int64_t>(grp->max_tpb, (x.blockn + TILE - 1) / TILE);
     }
     if (!grp->img.allocate((size_t)std::max<int64_t>(img, 16), dev) || !grp->slots.allocate((size_t)std::max<int64_t>(img, 16), dev) ||
         !grp->es.allocate(sizeof(EncStream) * (size_t)std::max<int64_t>(ns, 1), dev) || !grp->counters.allocate(128, dev))
@@ -3678,8 +3638,7 @@ int encode_group_launch(CodecGroup *grp, bool exact_lz4, bool memcpy_only, cudaS
     const int64_t *bstart = grp->starts.as<int64_t>(), *cstart = bstart + 2 * (n + 1);
     if (grp->nbl == 0) return 0;
     cudaMemsetAsync(grp->counters.p, 0, 128, st);
-    const bool fast = grp->shuffle && (ts == 4 || ts == 8);
-    if (fast && !grp->img_ready) {
+    if (!grp->img_ready) {
         const int slice = gather_slice(grp->h[0].g, grp->nbl, (int64_t)sms * 8);
         const int64_t nsl = ceil_div(grp->h[0].g.blockn, slice), nu = grp->nbl * nsl;
         int nt = 32;                              // as many as the group's widest need (rows of whole quads or not)
@@ -3689,10 +3648,6 @@ int encode_group_launch(CodecGroup *grp, bool exact_lz4, bool memcpy_only, cudaS
             IAB_TIMED("k_gather_fast", st, k_gather_fast_g<8><<<gb, 256, 0, st>>>(items, bstart, n, nu, (int)nsl, slice, nt));
         else
             IAB_TIMED("k_gather_fast", st, k_gather_fast_g<4><<<gb, 256, 0, st>>>(items, bstart, n, nu, (int)nsl, slice, nt));
-    }
-    if (!fast && !grp->img_ready) {
-        const int64_t tb = std::max<int64_t>(std::min<int64_t>(grp->nbl * grp->max_tpb, (int64_t)sms * 8), 1);
-        IAB_TIMED("k_gather", st, k_gather_g<<<(unsigned)tb, 256, 0, st>>>(items, bstart, n, grp->nbl, grp->max_tpb, grp->shuffle));
     }
     if (!memcpy_only)
         encode_streams(grp->img.as<uint8_t>(), grp->nbl * grp->nstreams, grp->nstreams, grp->neblock, grp->slots.as<uint8_t>(),

@@ -292,7 +292,6 @@ struct CodecGroup {
     int n = 0, ts = 0;
     int nstreams = 0, neblock = 0;         // encode: the shared stream shape
     int64_t nbl = 0, nch = 0, nsf = 0;     // blocks, chunks, fast-scatter slices of all containers
-    int64_t max_tpb = 0;                   // general-path tiles per block (largest over containers)
     bool shuffle = true, split = true;     // encode: byte shuffle, one stream per item byte
     std::vector<CodecItem> h;              // host copy of the table
     DevBuf items, starts;                  // device table; starts: blocks, slices, chunks ([n + 1] each)
