@@ -19,8 +19,8 @@
 // kinds, offsets, memcpy fallback; exclusive scan of chunk sizes) -> emit (copy payloads
 // into the final contiguous chunk buffer).  Two LZ4 encoders: one warp per stream
 // reproducing liblz4 1.9.4 LZ4_compress_fast(acceleration 1) output byte for byte (the codec
-// c-blosc2 calls for BLOSC_LZ4: 16 KiB hash table in shared memory, 32 match probes
-// evaluated per step), and a parallel-parse encoder (one CTA per stream, valid LZ4 with
+// c-blosc2 calls for BLOSC_LZ4: 16 KiB hash table in shared memory, 32 positions at a time),
+// and a parallel-parse encoder (one CTA per stream, valid LZ4 with
 // different bytes).  Stream-kind selection (zero/run, raw when LZ4 does not fit, memcpyed
 // chunk when the output would exceed nbytes + 32) follows c-blosc2's blosc_c rules.
 #include <cuda_runtime.h>
@@ -273,19 +273,19 @@ static unsigned parse_grid(int64_t nbl, int sms)
 }
 
 // D1: LZ4 stream decode, one CTA (256 threads) per stream, streams handed out
-// dynamically (a CTA's first is that of its own number, see stream_at) from a job queue (which may hold the streams of several containers: each job
-// carries its source, destination and status word).  The stream is consumed in windows of up
-// to DW compressed bytes staged in shared memory (the next window's loads are issued as soon
-// as its start is known).  With many streams in flight the SM's issue rate bounds the kernel,
-// so each step is chosen for few instructions per byte:
+// dynamically (a CTA's first is that of its own number, see stream_at) from a job queue, which may
+// hold the streams of several containers: each job carries its source, destination and status
+// word.  The stream is consumed in windows of up to DW compressed bytes staged in shared memory
+// (the next window's loads are issued as soon as its start is known).  With many streams in flight
+// the SM's issue rate bounds the kernel (1,024 of 64 KiB: 72% of the slots), so each step is chosen
+// for few instructions per byte:
 //  1. the chain of token positions from the window start: every thread walks the tokens of one
 //     32-byte segment from one of its first four bytes, four tracks per segment.  A walk from
 //     a wrong byte need not meet the true chain soon (sequences of 3 bytes keep their phase),
 //     but the true chain soon runs on one of the four tracks: so a track's exit is linked to
 //     the track it enters (after a few more tokens, where it is on none), and the tracks on
 //     the path from the window start are marked by pointer doubling over the 256 tracks.  The
-//     result is a bit per window byte.  (Doubling over every byte of the window took 24,000 of
-//     a window's 51,000 cycles, with the SM full; this takes 8,700 of 27,000);
+//     result is a bit per window byte;
 //  2. each thread reads the lengths of the tokens of its 8 bytes, and an exclusive scan over
 //     token counts and output lengths numbers the sequences and places their output;
 //  3. the output is resolved in groups of at most DCAP bytes in shared memory: a literal
@@ -1406,10 +1406,15 @@ __device__ __forceinline__ uint32_t lz_hash_v(uint32_t v4, uint32_t b4)
 // long backward extensions are walked too, with warp-wide loops.  Inserted lanes enter the table
 // at the window's end.  Searches past their 64th probe, whose step grows, take 32 probes per step
 // at the probes' own positions.
-// Measured against one scalar step per sequence (650 cycles each; a window of 32 positions now
-// takes about 2,100): 64 KiB sign/exponent planes 5.1 -> 2.2 ms a stream; k_lz4_encode on the
-// 5000 x 6000 float32 product 4.75 -> 0.98 ms, on the 4056 x 3712 float64 one 2.30 -> 0.93 ms
-// (of which 0.4 ms from handing out the compressible planes first).
+// Measured against one scalar step per sequence: sign/exponent planes of gaussian float64 values, a
+// stream by itself, 64 KiB 4.57 -> 3.19 ms (3,060 cycles for 32 positions; five-byte hashes, of 256
+// KiB, 2,070); k_lz4_encode on the 5000 x 6000 float32 product 4.75 -> 0.98 ms, on the 4056 x 3712
+// float64 one 2.30 -> 0.88 ms.  Where every match is long and follows another, a window holds one
+// step, and the scalar step was the faster: (i + j) / 50 rounded down as float64, 4000 x 3000 in
+// blocks of 500 x 500, 4.8 -> 7.0 ms, counting 5.4 -> 6.9.  A form of the function for such streams,
+// chosen after 2 KiB by what they had compressed to, lost more on streams of a few KiB (1.7 -> 4.3
+// ms) than it gave there, and leaving out the chain where the first lane has a long match cost the
+// other streams 3 to 5%.
 template <bool SMALL>
 __device__ __forceinline__ int warp_lz4_compress(const uint8_t *__restrict__ src, int n, uint8_t *__restrict__ dst,
                                                  int cap, uint32_t *tab, uint32_t *bm, uint8_t *ring, int rcap,
@@ -1861,11 +1866,10 @@ __global__ void __launch_bounds__(32, XCTAS) k_lz4_encode(const uint8_t *__restr
 //     match of PCAP bytes or more, which is extended exactly before it is written.
 // The bytes of the next window are loaded before B and stored after it; literal runs of more than
 // 16 bytes are copied by a warp.
-// What bounds it: the latency of a window's steps (eight streams an SM, each a chain of some
-// 25,000 cycles per window; 45% of the issue slots), and where zero padding makes every match long,
-// the measuring of lengths, once 46,000 of a window's 68,000 cycles and now 16,000 of 40,000.  A batch
-// of 40 float64 products with extents of 64 to 2048: 14.7 -> 13.2 ms; the 16384 x 16384 float32
-// result of a split product 3.83 -> 3.6 ms.
+// What bounds it: the latency of a window's steps (1,024 streams of 64 KiB, seven an SM: 26,000
+// cycles a window, 60% of the issue slots; a stream by itself 13,000), and where zero padding makes
+// every match long, the measuring of lengths.  A batch of 40 float64 products with extents of 64 to
+// 2048: 14.7 -> 13.2 ms; the 16384 x 16384 float32 result of a split product 3.83 -> 3.45 ms.
 // Format rules kept: offsets 1..65535, matches start at least 12 bytes before the end and
 // end at least 5 bytes before it, so the block ends with >= 5 literals.
 constexpr int PW = 1024;
