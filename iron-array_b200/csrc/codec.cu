@@ -2858,11 +2858,11 @@ int decode_lz4(DecodeQueue *q, cudaStream_t st)
 }
 
 // The decoded streams to the dense array.  Small containers by one launch, the blocks the fast
-// path does not take included; from SC_SPLIT bytes on those have a launch of their own, which finds
-// nothing in 5 us in most containers (4000 x 4000 float32 66 -> 70 us), but writes them with the
-// registers and CTAs that they need (the same array stored as it is 0.31 -> 0.21 ms).
-// Items of 1 and 2 bytes go by the general path.
-constexpr int64_t SC_SPLIT = int64_t(32) << 20;
+// path does not take included; from SC_SPLIT bytes on those have a launch of their own, which costs
+// 5 us where it finds nothing, but writes them with the registers and CTAs that they need (4000 x 4000
+// float32, 61 MiB: 66 us by one launch, 70 by two; stored as it is 0.29 and 0.21 ms, 0.41 by two launches
+// with a list of the blocks between them).  Items of 1 and 2 bytes go by the general path.
+constexpr int64_t SC_SPLIT = int64_t(64) << 20;
 template <int TS>
 static void scatter_launch(const Geom &g, bool all, const uint8_t *chunks, const uint8_t *cend, const BlockDesc *bd,
                            const StreamDesc *sd, const uint8_t *scratch, const uint8_t *send, void *out, int64_t ld, int *err,
